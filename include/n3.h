@@ -56,9 +56,12 @@ int n3_init_device(void);
  * (a) Population scoring.
  * ------------------------------------------------------------------------- */
 
-/* Exact collinear-triple count of B states given as P/Q, one warp per state,
- * int32 cross-product determinants.  Replaces the reference kernel
- * score_population (src/no_three_75/gpu.py:13-42, launched at gpu.py:76) and,
+/* Exact collinear-triple count of B states given as P/Q.  Counted by cross
+ * products on small grids and by gcd-reduced directions on larger ones (a state
+ * with a column off the 75 x 75 grid or two equal points in a row, which has no
+ * direction count, by cross products at every size): the same integers.
+ * Replaces the reference kernel score_population (src/no_three_75/gpu.py:13-42,
+ * launched at gpu.py:76) and,
  * with badness != NULL, score_population_badness
  * (src/no_three_75/gpu_device_search.py:118-161): badness[b][s] is the number
  * of collinear triples containing slot s.
@@ -80,10 +83,9 @@ int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* 
 
 /* Fused, cross-checked scoring: determinant count and slope count per state,
  * plus the column-range / duplicate-point checks.  scores = determinant E,
- * badness = slope badness, or NULL: then the slope side counts E alone, each
- * collinear triple once from its first slot (about 2/3 of the slope side's
- * time).  *mismatch (device int32, accumulated, caller zeroes it) counts
- * states whose two counts differ or whose badness does not sum to 3E;
+ * badness = slope badness, or NULL: then the slope side counts E alone.
+ * *mismatch (device int32, accumulated, caller zeroes it) counts states whose
+ * two counts differ;
  * *error_word (device uint32, OR-ed, caller zeroes it, may be NULL) collects
  * the device error bits (1: column range, 2: duplicate point, 4: mismatch).  The reference runs this audit on the host
  * (src/no_three_75/gpu.py:131 exact_match, src/no_three_75/tempering.py:193-204). */

@@ -1,10 +1,10 @@
-// (a) Population scoring: exact collinear-triple counts, one warp per state.
+// (a) Population scoring: exact collinear-triple counts of populations of states.
 //
-// Two independent kernels and a fused, cross-checked one:
+// Two independent kernels and a cross-checked pair of launches:
 //
 // * Determinant count (replaces src/no_three_75/gpu.py:13-42 and
 //   src/no_three_75/gpu_device_search.py:118-161).  Every triple i<j<k is
-//   tested once with an exact int32 cross product, at its middle slot j.  The
+//   tested once with an exact cross product, at its middle slot j.  The
 //   two slots of j's row are pivots together; the triple's other two points
 //   lie in rows above and below that row.  The larger side sits in lane
 //   registers, the smaller side is broadcast from shared memory one row (two
@@ -13,21 +13,33 @@
 //   in another row are never collinear.
 //
 // * Normalised-slope line count (the counting form of
-//   src/no_three_75/verifier_b.py:8-33).  For every anchor a, the other points
-//   are binned by gcd-reduced undirected direction in an 8-bit shared-memory
-//   histogram; sum over bins of C(c,2) is the anchor's badness and
-//   E = sum(badness) / 3 (a line of k points gives each member C(k-1,2) pairs,
-//   src/no_three_75/conflicts.py:373-378).  The gcd reduction is tabulated once
-//   per device by build_dir_lut_kernel.
+//   src/no_three_75/verifier_b.py:8-33).  From every slot, the later slots are
+//   told apart by gcd-reduced undirected direction; C(c,2) pairs of a
+//   direction's c slots make collinear triples with it.  The gcd reduction is
+//   tabulated once per device by build_dir_lut_kernel.
 //
-// * Checked scoring runs both per state and flags disagreement on device.
+// The plain scores (n3_score_population, n3_score_columns) take the faster of
+// the two for the grid size; n3_score_slope is the second, n3_score_checked
+// runs both and flags disagreement on the device.
+//
+// What bounds them, at 4096 n = 75 states:
+//   det_kernel<.., 1, false>   278 us (304 us on 32-bit integers).  Four tests are
+//       four packed multiply-add-pipe instructions, two compares and two adds
+//       that read 22 registers; at two register reads a cycle and scheduler that
+//       is 11 cycles (11.5 measured for the loop alone), the loop runs 4850 times
+//       per state on 592 schedulers: 194 us.  The rest is the loop's overhead
+//       over 19 rows on average and the pivots' set-up.
+//   tag_kernel, E alone         74 us, with badness 88 us (86 and 122 us with
+//       4-bit counters; the determinant count with badness took 464 us).  Shared
+//       memory is busy 87 % of the cycles: a direction load (3.5 cycles for 32
+//       random 2-byte words), a tag store and a tag load (2.9 each) per 32 slots.
 #include <cstdio>
 
 #include "score_impl.cuh"
 
 namespace n3 {
 
-__device__ uint16_t g_dir_lut[kLutSize];
+__device__ __align__(16) uint16_t g_dir_lut[kTagLutBytes / 2];
 __device__ __align__(16) uint16_t g_dir_lut_full[kFullLutBytes / 2];
 __device__ int g_dir_count;
 
@@ -108,134 +120,169 @@ struct ColSource {
 
 constexpr int kDetWarps = 4;  // small CTAs: 4096 states spread evenly over 148 SMs
 
-template <class Src, bool BAD>
-__global__ void __launch_bounds__(kDetWarps * 32) det_kernel(Src src, int B, int n, int32_t* __restrict__ scores,
-                                                               int32_t* __restrict__ badness) {
-  __shared__ __align__(16) int cs_all[kDetWarps][kMaxM];
-  __shared__ int bad_all[BAD ? kDetWarps : 1][BAD ? kMaxM : 1];
+// E by determinants: on packed floats when every column lies on the grid, else
+// on 32-bit integers (det_state), as the count has always taken any columns.
+// PARTS = 1: a warp per state, kDetWarps states per CTA.  PARTS > 1, for fewer
+// states than warps that the GPU can hold: a CTA of PARTS warps per state,
+// which share its pivot rows.
+template <class Src, int PARTS, bool BAD>
+__global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
+    det_kernel(Src src, int B, int n, int32_t* __restrict__ scores, int32_t* __restrict__ badness) {
+  __shared__ float4 rows_all[PARTS > 1 ? 1 : kDetWarps][kMaxN];
+  __shared__ int bad_all[PARTS > 1 || !BAD ? 1 : kDetWarps][BAD ? kMaxM : 1];
+  __shared__ int total;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * kDetWarps + warp;
+  const int b = PARTS > 1 ? blockIdx.x : blockIdx.x * kDetWarps + warp;
   if (b >= B) return;
-  const int m = 2 * n;
-  int* cs = cs_all[warp];
-  int* bad = BAD ? bad_all[warp] : nullptr;
-  for (int s = lane; s < m; s += 32) {
-    cs[s] = src.col(b, n, s);
-    if (BAD) bad[s] = 0;
+  float4* rows4 = rows_all[PARTS > 1 ? 0 : warp];
+  int* bad = BAD ? bad_all[PARTS > 1 ? 0 : warp] : nullptr;
+  const int first = PARTS > 1 ? threadIdx.x : lane, stride = PARTS > 1 ? PARTS * 32 : 32;
+  bool on_grid = true;
+  for (int r = first; r < n; r += stride) {
+    const int c0 = src.col(b, n, 2 * r), c1 = src.col(b, n, 2 * r + 1);
+    on_grid = on_grid && (unsigned)c0 < (unsigned)kMaxN && (unsigned)c1 < (unsigned)kMaxN;
+    rows4[r] = make_float4((float)c0, (float)c0, (float)c1, (float)c1);
+    if (BAD) bad[2 * r] = bad[2 * r + 1] = 0;
   }
-  __syncwarp();
-  const int cnt = warp_sum(det_state<BAD>(cs, n, lane, bad));
-  if (lane == 0) scores[b] = cnt;
-  if (BAD) {
+  if (PARTS > 1) {
+    if (threadIdx.x == 0) total = 0;
+    on_grid = __syncthreads_and(on_grid);
+  } else {
+    on_grid = __all_sync(0xffffffffu, on_grid);
     __syncwarp();
-    for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = bad[s];
   }
-}
-
-// Loads one state, validating columns (range, row duplicates).  Returns the
-// device error bits for this state (warp-uniform).
-template <class Src>
-__device__ __forceinline__ uint32_t load_checked(const Src& src, int b, int n, int* cs, int lane) {
-  const int m = 2 * n;
-  uint32_t err = 0;
-  for (int s = lane; s < m; s += 32) {
-    const int c = src.col(b, n, s);
-    if (c < 0 || c >= n) err |= kErrColumnRange;
-    cs[s] = min(max(c, 0), n - 1);
+  int cnt = 0;
+  if (on_grid) {  // uniform
+    cnt = det_state_f<BAD>(rows4, n, lane, PARTS > 1 ? warp : 0, PARTS, bad);
+  } else if (PARTS == 1 || warp == 0) {
+    int* cs = reinterpret_cast<int*>(rows4);
+    for (int s = lane; s < 2 * n; s += 32) cs[s] = src.col(b, n, s);
+    __syncwarp();
+    cnt = det_state<BAD>(cs, n, lane, bad);
   }
-  __syncwarp();
-  for (int r = lane; r < n; r += 32)
-    if (cs[2 * r] == cs[2 * r + 1]) err |= kErrDuplicate;
-  err = __reduce_or_sync(0xffffffffu, err);
-  return err;
+  cnt = warp_sum(cnt);
+  if (PARTS > 1) {
+    if (lane == 0 && cnt) atomicAdd(&total, cnt);
+    __syncthreads();
+    cnt = total;
+  } else {
+    __syncwarp();
+  }
+  if (first == 0) scores[b] = cnt;
+  if (BAD)
+    for (int s = first; s < 2 * n; s += stride) badness[(size_t)b * 2 * n + s] = bad[s];
 }
 
-// The slope count of every state with 4-bit histograms: W = blockDim.x / 32
-// <= 32 warps share one direction table, a warp per state, each state loaded
-// and validated (column range, row duplicates).  MODE 0: slope count only
-// (scores, badness).  MODE 2: slope count and badness, checked against the
-// determinant counts already in `scores` (written by det_kernel on the same
-// stream).  MODE 3: the forward slope count of E only (slope_forward_state4),
-// checked the same way (and, if `badness` is given, that badness checked to
-// sum to 3E).  A state that may have overflowed a 4-bit counter is recounted
-// by slope_state_halves in the same shared memory.
-constexpr int kSlope4MaxWarps = 32;
-__host__ __device__ constexpr size_t slope4_smem(int warps) {
-  return kFullLutBytes + (size_t)warps * (sizeof(uint32_t) * kHist4Words + sizeof(int) * kMaxM * 2);
-}
+// The slope count (tag_state): up to kTagWarps warps share one compact direction
+// table, `parts` warps (a power of two) a state, which share its centres, so that
+// few states fill the SMs too (64 n = 75 states: 8.4 us; 51 us with a warp each);
+// with enough states for every warp, parts is 1.
+//   kCount   E and, if wanted, badness of any states: one with a column off the
+//            grid or two equal points in a row, which has no line count, is
+//            counted by determinants (det_state), so the results are the
+//            determinant count's for every input.
+//   kSlope   the same, but such a state gets -1 (and the error bits, if wanted).
+//   kChecked compared with the determinant counts already in `scores` (written
+//            by det_kernel on the same stream).
+enum TagMode { kCount, kSlope, kChecked };
+constexpr int kTagWarps = 28;  // 28 x 148 = 4144 states at once; 32 would need 6.4 KB each beside the table
+constexpr int kTagMaxParts = 16;     // warps that share a state
+constexpr int kTagMinThreads = 256;  // threads that copy the table when few states are scored
+__host__ __device__ constexpr size_t tag_smem(int warps) { return kTagLutBytes + (size_t)warps * kTagWarpBytes; }
+static_assert(tag_smem(kTagWarps) <= 227 * 1024, "tag_kernel shared memory");
+static_assert(kDirCount >= (int)sizeof(int) * kMaxM, "a state's columns fit in a warp's tags");
 
-template <int MODE>
-__global__ void __launch_bounds__(kSlope4MaxWarps * 32, 1) slope4_kernel(ColSource src, int B, int n,
-                                                                          int32_t* __restrict__ scores,
-                                                                          int32_t* __restrict__ badness,
-                                                                          int32_t* __restrict__ mismatch,
-                                                                          uint32_t* __restrict__ error_word) {
-  static_assert(MODE == 0 || MODE == 2 || MODE == 3, "slope count only, or checked against determinant counts");
+template <class Src, int MODE, bool BAD, bool SPLIT>
+__global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, int n, int W, int parts,
+                                                                 const uint16_t* __restrict__ g_lut,
+                                                                 int32_t* __restrict__ scores,
+                                                                 int32_t* __restrict__ badness,
+                                                                 int32_t* __restrict__ mismatch,
+                                                                 uint32_t* __restrict__ error_word) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int W = blockDim.x >> 5;
+  __shared__ int total_all[kTagWarps];
   uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
-  uint32_t* hist_all = reinterpret_cast<uint32_t*>(smem + kFullLutBytes);
-  int* cs_all = reinterpret_cast<int*>(hist_all + kHist4Words * W);
-  int* bad_all = cs_all + kMaxM * W;
-  full_lut_copy(lut, g_dir_lut_full);
-  for (int i = threadIdx.x; i < kHist4Words * W; i += blockDim.x) hist_all[i] = 0u;
-  __syncthreads();
-  if (threadIdx.x == 0) lut[kFullLutCentre] = (uint16_t)kDirCount;  // (0, 0): the centre's own counter
+  tag_lut_copy(lut, g_lut);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= W) return;  // it only helped to copy the table
   const int m = 2 * n;
-  int* cs = cs_all + warp * kMaxM;
-  int* bad = bad_all + warp * kMaxM;
-  uint32_t* hist = hist_all + warp * kHist4Words;
-  for (int b = blockIdx.x * W + warp; b < B; b += gridDim.x * W) {
-    const uint32_t err = load_checked(src, b, n, cs, lane);
-    if (err) {  // invalid state: no count is meaningful
-      if (lane == 0) {
-        scores[b] = -1;
-        if (error_word) atomicOr(error_word, err);
-        if (MODE != 0) atomicAdd(mismatch, 1);
-      }
-      if (badness)
-        for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = -1;
+  if (!SPLIT) parts = 1;
+  const int group = warp / parts, part = warp % parts;
+  uint8_t* tag = smem + kTagLutBytes + (size_t)warp * kTagWarpBytes;
+  // the group's badness and count live with its first warp
+  uint32_t* word = reinterpret_cast<uint32_t*>(tag + kDirCount);
+  uint32_t* bad = reinterpret_cast<uint32_t*>(smem + kTagLutBytes + (size_t)group * parts * kTagWarpBytes + kDirCount);
+  int* total = total_all + group;
+  auto group_sync = [&]() {  // at most 14 groups of more than one warp: barrier ids 1 .. 14
+    if (!SPLIT)
       __syncwarp();
+    else
+      asm volatile("barrier.sync %0, %1;" ::"r"(1 + group), "r"(32 * parts) : "memory");
+  };
+  for (int b = blockIdx.x * (W / parts) + group; b < B; b += gridDim.x * (W / parts)) {
+    int key[kSlotsPerLane];
+    uint32_t err = 0;
+#pragma unroll
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      const int s = lane + 32 * t;
+      const bool in = s < m;
+      const int c = in ? src.col(b, n, s) : 0;
+      // the two points of a row are neighbouring lanes
+      const int c2 = __shfl_xor_sync(0xffffffffu, c, 1);
+      if (in && (c < 0 || c >= (MODE == kCount ? kMaxN : n))) err |= kErrColumnRange;
+      if (in && c == c2) err |= kErrDuplicate;
+      key[t] = in ? (s >> 1) * kLutW + c : -1;
+      if (in) word[s] = 0u;
+    }
+    if (part == 0 && lane == 0) *total = 0;
+    err = __reduce_or_sync(0xffffffffu, err);  // the same in every warp of the group
+    group_sync();
+    if (err) {  // no line count exists
+      if (part == 0) {
+        if (MODE == kCount) {
+          int* cs = reinterpret_cast<int*>(tag);
+          for (int s = lane; s < m; s += 32) cs[s] = src.col(b, n, s);
+          __syncwarp();
+          const int e = warp_sum(det_state<BAD>(cs, n, lane, reinterpret_cast<int*>(bad)));
+          if (lane == 0) scores[b] = e;
+          __syncwarp();
+          if (BAD)
+            for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = (int)bad[s];
+        } else {
+          if (lane == 0) {
+            scores[b] = -1;
+            if (error_word) atomicOr(error_word, err);
+            if (MODE == kChecked) atomicAdd(mismatch, 1);
+          }
+          if (BAD)
+            for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = -1;
+        }
+      }
+      group_sync();
       continue;
     }
-    bool overflow;
-    if (MODE == 3) {  // forward count of E, compared with the determinant count (and badness, if given)
-      int e_slope = slope_forward_state4(cs, n, lut, hist, lane, &overflow);
-      if (overflow) {  // uniform
-        __syncwarp();
-        e_slope = slope_state_halves(cs, n, lut, hist, lane, nullptr) / 3;
-      }
-      int bad_sum = 0;
-      if (badness)
-        for (int s = lane; s < m; s += 32) bad_sum += badness[(size_t)b * m + s];
-      bad_sum = warp_sum(bad_sum);
-      const int e_det = scores[b];
-      if (lane == 0 && (e_slope != e_det || (badness && bad_sum != 3 * e_det))) {
-        atomicAdd(mismatch, 1);
-        if (error_word) atomicOr(error_word, kErrMismatch);
-      }
+    int e = tag_state<BAD, SPLIT>(key, m, lut, tag, lane, word, bad, part, parts);
+    if (SPLIT) {
+      if (lane == 0) atomicAdd(total, e);
+      group_sync();
+      e = *total;
+    } else {
       __syncwarp();
-      continue;
     }
-    int total = slope_state4(cs, n, lut, hist, lane, bad, &overflow);
-    if (overflow) {  // uniform
-      __syncwarp();
-      total = slope_state_halves(cs, n, lut, hist, lane, bad);
-    }
-    __syncwarp();
-    if (MODE == 0) {
-      if (lane == 0) scores[b] = total / 3;
-    } else {  // scores[b] holds the determinant count of this state
-      if (lane == 0 && total != 3 * scores[b]) {
-        atomicAdd(mismatch, 1);
-        if (error_word) atomicOr(error_word, kErrMismatch);
+    if (part == 0) {
+      if (MODE == kChecked) {  // scores[b] holds the determinant count of this state
+        if (lane == 0 && e != scores[b]) {
+          atomicAdd(mismatch, 1);
+          if (error_word) atomicOr(error_word, kErrMismatch);
+        }
+      } else if (lane == 0) {
+        scores[b] = e;
       }
+      if (BAD)
+        for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = (int)bad[s];
     }
-    if (badness)
-      for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = bad[s];
-    __syncwarp();
+    group_sync();
   }
 }
 
@@ -276,39 +323,80 @@ static int check_common(int B, int n, const void* a, const void* out) {
   return N3_OK;
 }
 
-int prepare_score() {
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(n3::slope4_kernel<0>), n3::slope4_smem(n3::kSlope4MaxWarps)));
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(n3::slope4_kernel<2>), n3::slope4_smem(n3::kSlope4MaxWarps)));
-  return allow_smem(reinterpret_cast<const void*>(n3::slope4_kernel<3>), n3::slope4_smem(n3::kSlope4MaxWarps));
+template <class Src, int MODE, bool BAD>
+static int launch_tag(Src src, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+                      uint32_t* error_word, cudaStream_t st) {
+  using namespace n3;
+  N3_TRY(ensure_device_tables());
+  const int sms = sm_count();
+  const int per = (B + sms - 1) / sms;  // states per SM
+  int parts = 1;
+  while (parts < kTagMaxParts && 2 * parts * per <= kTagWarps) parts *= 2;
+  const auto kernel = parts > 1 ? tag_kernel<Src, MODE, BAD, true> : tag_kernel<Src, MODE, BAD, false>;
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(kernel), tag_smem(kTagWarps)));
+  const int groups = per * parts < kTagWarps ? per : kTagWarps / parts, W = groups * parts;
+  const int want = (B + groups - 1) / groups;
+  const int threads = W * 32 > kTagMinThreads ? W * 32 : kTagMinThreads;
+  kernel<<<want < sms ? want : sms, threads, tag_smem(W), st>>>(src, B, n, W, parts, dir_lut_device_ptr(), scores,
+                                                                badness, mismatch, error_word);
+  return check_launch("tag_kernel");
 }
 
-template <class Src>
-static int launch_det(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
+template <int MODE>
+static int launch_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+                        uint32_t* error_word, cudaStream_t st) {
   if (B == 0) return N3_OK;
-  const int grid = (B + n3::kDetWarps - 1) / n3::kDetWarps;
-  if (badness)
-    n3::det_kernel<Src, true><<<grid, n3::kDetWarps * 32, 0, st>>>(src, B, n, scores, badness);
+  const n3::ColSource src{cols};
+  return badness ? launch_tag<n3::ColSource, MODE, true>(src, B, n, scores, badness, mismatch, error_word, st)
+                 : launch_tag<n3::ColSource, MODE, false>(src, B, n, scores, nullptr, mismatch, error_word, st);
+}
+
+template <class Src, bool BAD>
+static int launch_det(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
+  using namespace n3;
+  const int sms = sm_count();
+  // warps per state: 16 while two such CTAs fit every SM, 4 while eight do (64
+  // n = 75 states: 14 us against 79 us with one warp a state; 1024: 76 and 105)
+  if (B <= 2 * sms)
+    det_kernel<Src, 16, BAD><<<B, 16 * 32, 0, st>>>(src, B, n, scores, badness);
+  else if (B <= 8 * sms)
+    det_kernel<Src, 4, BAD><<<B, 4 * 32, 0, st>>>(src, B, n, scores, badness);
   else
-    n3::det_kernel<Src, false><<<grid, n3::kDetWarps * 32, 0, st>>>(src, B, n, scores, nullptr);
+    det_kernel<Src, 1, BAD><<<(B + kDetWarps - 1) / kDetWarps, kDetWarps * 32, 0, st>>>(src, B, n, scores, badness);
   return check_launch("det_kernel");
 }
 
-// The 4-bit slope kernel: one CTA per SM of W warps, W = ceil(B / SMs) up to
-// 32, so that 4096 states are one state per warp on 147 SMs.
-template <int MODE>
-static int launch_slope4(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
-                         uint32_t* error_word, cudaStream_t st) {
+// Up to these sizes the determinants are the faster count (us for 20,011
+// states, determinants against tags: E alone n = 24: 86 / 99, n = 28: 121 / 115;
+// with badness n = 20: 82 / 100, n = 24: 125 / 119): they grow with n^3, the
+// tags with n^2, but every centre costs the tags two round trips to shared
+// memory.  At 64 states the determinants stay ahead up to n = 60 by 1-2 us.
+constexpr int kDetMaxN = 26, kDetMaxNBad = 22;
+
+template <class Src>
+static int launch_count(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
   if (B == 0) return N3_OK;
-  N3_TRY(ensure_device_tables());
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(n3::slope4_kernel<MODE>), n3::slope4_smem(n3::kSlope4MaxWarps)));
-  const int sms = sm_count();
-  int W = (B + sms - 1) / sms;
-  W = W < 1 ? 1 : (W > n3::kSlope4MaxWarps ? n3::kSlope4MaxWarps : W);
-  const int blocks_needed = (B + W - 1) / W;
-  const int grid = blocks_needed < sms ? blocks_needed : sms;
-  n3::slope4_kernel<MODE><<<grid, W * 32, n3::slope4_smem(W), st>>>(n3::ColSource{cols}, B, n, scores, badness,
-                                                                    mismatch, error_word);
-  return check_launch("slope4_kernel");
+  if (badness)
+    return n <= kDetMaxNBad ? launch_det<Src, true>(src, B, n, scores, badness, st)
+                         : launch_tag<Src, n3::kCount, true>(src, B, n, scores, badness, nullptr, nullptr, st);
+  return n <= kDetMaxN ? launch_det<Src, false>(src, B, n, scores, nullptr, st)
+                       : launch_tag<Src, n3::kCount, false>(src, B, n, scores, nullptr, nullptr, nullptr, st);
+}
+
+template <class Src, int MODE>
+static int prepare_tag() {
+  using namespace n3;
+  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, true, true>), tag_smem(kTagWarps))));
+  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, true, false>), tag_smem(kTagWarps))));
+  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, true>), tag_smem(kTagWarps))));
+  return allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, false>), tag_smem(kTagWarps));
+}
+
+int prepare_score() {
+  N3_TRY((prepare_tag<n3::PQSource, n3::kCount>()));
+  N3_TRY((prepare_tag<n3::ColSource, n3::kCount>()));
+  N3_TRY((prepare_tag<n3::ColSource, n3::kSlope>()));
+  return prepare_tag<n3::ColSource, n3::kChecked>();
 }
 
 }  // namespace n3host
@@ -319,32 +407,30 @@ int n3_score_population(const int32_t* p, const int32_t* q, int B, int n, int32_
                         void* stream) {
   N3_TRY(n3host::check_common(B, n, p, scores));
   if (B > 0 && q == nullptr) return n3host::set_error(N3_ERR_ARG, "null Q pointer");
-  return n3host::launch_det(n3::PQSource{p, q}, B, n, scores, badness, (cudaStream_t)stream);
+  return n3host::launch_count(n3::PQSource{p, q}, B, n, scores, badness, (cudaStream_t)stream);
 }
 
 int n3_score_columns(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
   N3_TRY(n3host::check_common(B, n, cols, scores));
-  return n3host::launch_det(n3::ColSource{cols}, B, n, scores, badness, (cudaStream_t)stream);
+  return n3host::launch_count(n3::ColSource{cols}, B, n, scores, badness, (cudaStream_t)stream);
 }
 
 int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
   N3_TRY(n3host::check_common(B, n, cols, scores));
-  return n3host::launch_slope4<0>(cols, B, n, scores, badness, nullptr, nullptr, (cudaStream_t)stream);
+  return n3host::launch_slope<n3::kSlope>(cols, B, n, scores, badness, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
                      uint32_t* error_word, void* stream) {
   N3_TRY(n3host::check_common(B, n, cols, scores));
   if (B > 0 && mismatch == nullptr) return n3host::set_error(N3_ERR_ARG, "null mismatch counter");
+  if (B == 0) return N3_OK;
   // Two launches on one stream: the determinant count at full occupancy, then
-  // the independent slope count, which validates each state and compares.  With
-  // badness wanted, the full slope count provides it (the determinant kernel's
-  // own badness output costs it 70 % more time than the whole slope pass);
-  // without, the forward slope count checks E at 3/4 of the cost.
-  N3_TRY(n3host::launch_det(n3::ColSource{cols}, B, n, scores, nullptr, (cudaStream_t)stream));
-  if (badness)
-    return n3host::launch_slope4<2>(cols, B, n, scores, badness, mismatch, error_word, (cudaStream_t)stream);
-  return n3host::launch_slope4<3>(cols, B, n, scores, nullptr, mismatch, error_word, (cudaStream_t)stream);
+  // the independent slope count, which validates each state, compares, and
+  // gives the badness if it is wanted.
+  N3_TRY((n3host::launch_det<n3::ColSource, false>(n3::ColSource{cols}, B, n, scores, nullptr,
+                                                   (cudaStream_t)stream)));
+  return n3host::launch_slope<n3::kChecked>(cols, B, n, scores, badness, mismatch, error_word, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -78,6 +78,126 @@ __device__ __forceinline__ int det_pivot_row(const int* __restrict__ cs, int n, 
   return cnt;
 }
 
+// The same tests on packed float pairs, for columns in [0, kMaxN) (every value
+// below stays under 2^14 in magnitude, so float arithmetic is exact; a product
+// of two non-zero differences is at least 1, so it is zero iff one of them is).
+// Per register slot and row y: the targets of the two pivots advance by one
+// packed add, two packed multiply-adds give the four differences
+// a_x c_y - T (pivot 0 in the low half, pivot 1 in the high half), and one
+// packed multiply joins the row's two points, which hit at most one of them
+// (see above), so two compares and two adds count four tests: eight
+// instructions, four on the multiply-add pipe (two results each) and four on
+// the ALU pipe, against 12 with 32-bit integer multiplies and compares
+// (integer multiply-adds run at half the float rate).
+// rows4[row] = (c, c, c', c') of the row's two points.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// One compare and one predicated add (from the plain expression the compiler
+// makes a select as well).
+__device__ __forceinline__ void count_zero(int& cnt, float x) {
+  asm("{\n\t.reg .pred p;\n\tsetp.eq.f32 p, %1, 0f00000000;\n\t@p add.s32 %0, %0, 1;\n\t}" : "+r"(cnt) : "f"(x));
+}
+
+template <int R, bool BAD>
+__device__ __forceinline__ int det_pivot_row_f(const float4* __restrict__ rows4, int n, int rho, int lane,
+                                               int* __restrict__ bad) {
+  const float cj0 = rows4[rho].x, cj1 = rows4[rho].z;
+  const int above = rho, below = n - 1 - rho;
+  const bool lanes_above = above >= below;
+  const int L = 2 * (lanes_above ? above : below);
+  const int lbase = lanes_above ? 0 : 2 * rho + 2;
+  const int rb0 = lanes_above ? rho + 1 : 0;
+  const int rb1 = lanes_above ? n : rho;
+  uint64_t ax[R], nb[R], nt[R];  // (a, a), (-b0, -b1), (-T0, -T1) of the current row
+  const float ay0 = (float)(rb0 - rho);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int x = lane + 32 * r;
+    if (x < L) {
+      const int s = lbase + x;
+      const float4 v = rows4[s >> 1];
+      const float c = (s & 1) ? v.z : v.x, a = (float)((s >> 1) - rho);
+      const float b0 = c - cj0, b1 = c - cj1;
+      ax[r] = pack2(a, a);
+      nb[r] = pack2(-b0, -b1);
+      nt[r] = pack2(-(ay0 * b0 + a * cj0), -(ay0 * b1 + a * cj1));
+    } else {  // idle slot: every difference is 1, never a hit
+      ax[r] = 0ull;
+      nb[r] = 0ull;
+      nt[r] = pack2(1.f, 1.f);
+    }
+  }
+  int cnt = 0, cnt1 = 0;
+  const ulonglong2* rows2 = reinterpret_cast<const ulonglong2*>(rows4);
+#pragma unroll 4
+  for (int row = rb0; row < rb1; ++row) {
+    const ulonglong2 cy = rows2[row];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint64_t d0 = fma2(ax[r], cy.x, nt[r]), p = mul2(d0, fma2(ax[r], cy.y, nt[r]));
+      float p0, p1;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
+      if (BAD && (p0 == 0.f || p1 == 0.f)) {  // x, the pivot, and slot 2 row or 2 row + 1
+        float e0, e1;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(d0));
+        if (p0 == 0.f) {
+          atomicAdd(bad + lbase + lane + 32 * r, 1);
+          atomicAdd(bad + 2 * rho, 1);
+          atomicAdd(bad + 2 * row + (e0 == 0.f ? 0 : 1), 1);
+        }
+        if (p1 == 0.f) {
+          atomicAdd(bad + lbase + lane + 32 * r, 1);
+          atomicAdd(bad + 2 * rho + 1, 1);
+          atomicAdd(bad + 2 * row + (e1 == 0.f ? 0 : 1), 1);
+        }
+      }
+      count_zero(cnt, p0);
+      count_zero(cnt1, p1);
+      nt[r] = add2(nt[r], nb[r]);
+    }
+  }
+  return cnt + cnt1;
+}
+
+// E's share of this lane from the pivot rows 1 + part, 1 + part + parts, ...;
+// rows4 in shared memory, columns in [0, kMaxN).  BAD: bad[s] (shared memory,
+// zeroed) receives the number of triples holding slot s.
+template <bool BAD>
+__device__ __forceinline__ int det_state_f(const float4* __restrict__ rows4, int n, int lane, int part, int parts,
+                                           int* __restrict__ bad) {
+  int cnt = 0;
+  for (int rho = 1 + part; rho < n - 1; rho += parts) {
+    const int L = 2 * max(rho, n - 1 - rho);
+    switch ((L + 31) >> 5) {
+      case 1: cnt += det_pivot_row_f<1, BAD>(rows4, n, rho, lane, bad); break;
+      case 2: cnt += det_pivot_row_f<2, BAD>(rows4, n, rho, lane, bad); break;
+      case 3: cnt += det_pivot_row_f<3, BAD>(rows4, n, rho, lane, bad); break;
+      case 4: cnt += det_pivot_row_f<4, BAD>(rows4, n, rho, lane, bad); break;
+      default: cnt += det_pivot_row_f<5, BAD>(rows4, n, rho, lane, bad); break;
+    }
+  }
+  return cnt;
+}
+
 template <bool BAD>
 __device__ __forceinline__ int det_state(const int* __restrict__ cs, int n, int lane, int* bad) {
   int cnt = 0;
@@ -94,187 +214,131 @@ __device__ __forceinline__ int det_state(const int* __restrict__ cs, int n, int 
   return cnt;
 }
 
-// Slope line count of one state.  Returns sum over anchors of badness (3E).
-// lutf: the full direction table in shared memory (dirs.cuh).  hist: this
-// warp's zeroed direction histogram (kDirWords words); it is left zeroed on
-// return.  bad_out (per slot) may be null.
-__device__ __forceinline__ int slope_state(const int* __restrict__ cs, int n, const uint16_t* __restrict__ lutf,
-                                           uint32_t* __restrict__ hist, int lane, int* __restrict__ bad_out) {
-  constexpr int kT = (kMaxM + 31) / 32;
-  const int m = 2 * n;
-  // this lane's slots b = lane + 32 t: their keys (row * kLutW + column) and rows
-  int key[kT], row[kT];
-#pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    const int b = lane + 32 * t;
-    row[t] = b < m ? b >> 1 : -1;
-    key[t] = b < m ? (b >> 1) * kLutW + cs[b] : 0;
-  }
-  int total = 0;
-  for (int a = 0; a < m; ++a) {
-    const int ra = a >> 1;
-    const uint16_t* base = lutf + kFullLutCentre - (ra * kLutW + cs[a]);
-    int pairs = 0;
-    int ids[kT];
-#pragma unroll
-    for (int t = 0; t < kT; ++t) {
-      ids[t] = -1;
-      if (row[t] >= 0 && row[t] != ra) {  // the row partner has the lone direction (0,1)
-        const int id = base[key[t]];
-        ids[t] = id;
-        pairs += hist_add(hist, id);  // earlier points on this direction
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kT; ++t)
-      if (ids[t] >= 0) hist_clear(hist, ids[t]);
-    __syncwarp();
-    pairs = warp_sum(pairs);
-    if (bad_out != nullptr && lane == (a & 31)) bad_out[a] = pairs;
-    total += pairs;
-  }
-  return total;
+// Normalised-slope line count of one state by tags: E for the whole warp.
+//
+// From each centre a, in slot order, the later slots k of other rows are told
+// apart by the gcd-reduced direction of k - a, so every collinear triple is
+// found once, from its first slot.  Each k writes its slot number into the tag
+// byte of its direction and reads it back: the last writer of a direction (the
+// winner) reads itself, every other slot of the direction (a loser) reads the
+// winner.  A few of the 148 slots lose, so most centres cost a load of the
+// direction, a store and a load per slot; nothing is counted or cleared for a
+// slot alone in its direction, and a slot only reads bytes that its own
+// direction wrote at this centre.  The losers then count themselves in the top
+// byte of their winner's word: a direction of c slots has c - 1 losers, which
+// find 0, 1, ... there and add 1 + 2 + ... = C(c, 2) triples.
+//
+// key: this lane's slots' table keys row * kLutW + column, negative beyond m.
+// lut: the compact direction table in shared memory, whose entry of the
+// difference d = key(k) - key(a) > 0 is lut[d + kMaxN - 1].  tag: this warp's
+// kDirCount bytes, any contents.  word[s] (shared memory, zeroed): with BAD, the
+// number of triples holding slot s on return (at most C(149, 2), below 2^24).
+constexpr size_t kTagLutBytes = ((sizeof(uint16_t) * kLutSize + 15) / 16) * 16;
+constexpr size_t kTagWarpBytes = kDirCount + sizeof(uint32_t) * kMaxM;  // the tags, then word[]
+
+// Copies the compact table (n3host::dir_lut_device_ptr) into shared memory; all
+// threads of the block call it.
+__device__ __forceinline__ void tag_lut_copy(uint16_t* __restrict__ dst, const uint16_t* __restrict__ g_lut) {
+  const uint4* s = reinterpret_cast<const uint4*>(g_lut);
+  uint4* d = reinterpret_cast<uint4*>(dst);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < (int)(kTagLutBytes / 16); i += blockDim.x) d[i] = s[i];
 }
 
-// The slope count with 4-bit counters (8 per word, kHist4Words words per
-// warp): the same pair sums as slope_state in half the shared memory, so twice
-// the warps fit beside one direction table.  lutf is the caller's copy of the
-// full table with the entry of (0, 0) set to kDirCount, a counter of its own
-// (the last word): every slot of the state is inserted, the centre itself into
-// that counter (adding 0, once) and its row partner into the (0, 1) class,
-// where it is alone (adding 0), so no insertion tests its row.  A counter that
-// reaches 16 wraps; by then its direction has added 0 + 1 + ... + 15 = 120
-// pairs to the centre's sum, so *overflow is set for every centre whose sum
-// reaches 120, and the caller recounts the state with slope_state_halves.
-// Every touched word is cleared, so the histogram is zero on return.
-constexpr int kDirWords4 = kDirCount / 8;     // 848
-constexpr int kHist4Words = kDirWords4 + 1;   // + the word of the centre's own counter
-__device__ __forceinline__ int slope_state4(const int* __restrict__ cs, int n, const uint16_t* __restrict__ lutf,
-                                            uint32_t* __restrict__ hist, int lane, int* __restrict__ bad_out,
-                                            bool* overflow) {
-  constexpr int kT = (kMaxM + 31) / 32;
-  const int m = 2 * n;
-  int key[kT];
-#pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    const int b = lane + 32 * t;
-    key[t] = b < m ? (b >> 1) * kLutW + cs[b] : -1;
+template <bool BAD>
+static __device__ __noinline__ int tag_centre_hist(int a, int ka, const int (&key)[kSlotsPerLane],
+                                                   const uint16_t* __restrict__ lut, uint8_t* __restrict__ tag,
+                                                   int lane, int* __restrict__ bad) {
+  uint32_t* hist = reinterpret_cast<uint32_t*>(tag);
+  __syncwarp();
+  for (int i = lane; i < kDirWords; i += 32) hist[i] = 0u;
+  __syncwarp();
+  int pairs = 0;
+  for (int t = 0; t < kSlotsPerLane; ++t)
+    if (lane + 32 * t > (a | 1) && key[t] >= 0) pairs += hist_add(hist, lut[key[t] - ka + kMaxN - 1]);
+  __syncwarp();
+  if (BAD) {
+    for (int t = 0; t < kSlotsPerLane; ++t)
+      if (lane + 32 * t > (a | 1) && key[t] >= 0)
+        atomicAdd(bad + lane + 32 * t, hist_get(hist, lut[key[t] - ka + kMaxN - 1]) - 1);
+    if (pairs) atomicAdd(bad + a, pairs);
   }
-  int total = 0;
-  bool ovf = false;
-  for (int a = 0; a < m; ++a) {
-    const uint16_t* base = lutf + kFullLutCentre - ((a >> 1) * kLutW + cs[a]);
-    int pairs = 0;
-    int ids[kT];
-#pragma unroll
-    for (int t = 0; t < kT; ++t) {
-      ids[t] = -1;
-      if (key[t] >= 0) {
-        const int id = base[key[t]];
-        ids[t] = id;
-        const int sh = (id & 7) << 2;
-        pairs += (int)((atomicAdd(hist + (id >> 3), 1u << sh) >> sh) & 0xFu);
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kT; ++t)
-      if (ids[t] >= 0) hist[ids[t] >> 3] = 0u;
-    __syncwarp();
-    pairs = warp_sum(pairs);
-    ovf |= pairs >= 120;
-    if (bad_out != nullptr && lane == (a & 31)) bad_out[a] = pairs;
-    total += pairs;
-  }
-  *overflow = ovf;  // uniform: from warp sums
-  return total;
+  __syncwarp();
+  return pairs;
 }
 
-// The forward slope count (from each centre a only the slots b > a, so every
-// collinear triple is counted once, from its first slot) with 4-bit counters,
-// as slope_state4; returns E for the whole warp.  A centre whose forward pair
-// sum reaches 120 sets *overflow (see slope_state4).
-__device__ __forceinline__ int slope_forward_state4(const int* __restrict__ cs, int n,
-                                                    const uint16_t* __restrict__ lutf, uint32_t* __restrict__ hist,
-                                                    int lane, bool* overflow) {
-  constexpr int kT = (kMaxM + 31) / 32;
-  const int m = 2 * n;
-  int key[kT];
+// SPLIT: only the centres part, part + parts, ... are counted (parts a power of
+// two up to 32), so that `parts` warps can share a state.  Each then counts its
+// losers in words of its own, and the badness of all goes to `bad`, the first
+// warp's (only that warp touches a top byte there).
+template <bool BAD, bool SPLIT = false>
+__device__ __forceinline__ int tag_state(const int (&key)[kSlotsPerLane], int m, const uint16_t* __restrict__ lut,
+                                         uint8_t* __restrict__ tag, int lane, uint32_t* word, uint32_t* bad,
+                                         int part = 0, int parts = 1) {
+  constexpr int kT = kSlotsPerLane;
+  constexpr uint32_t kOne = 1u << 24;
+  volatile uint8_t* vtag = tag;
+  int total = 0;  // this lane's triples
 #pragma unroll
-  for (int t = 0; t < kT; ++t) {
-    const int b = lane + 32 * t;
-    key[t] = b < m ? (b >> 1) * kLutW + cs[b] : -1;
-  }
-  int total = 0;
-  bool ovf = false;
-  for (int a = 0; a < m - 2; ++a) {
-    const uint16_t* base = lutf + kFullLutCentre - ((a >> 1) * kLutW + cs[a]);
-    int pairs = 0;
-    int ids[kT];
+  for (int ta = 0; ta < kT; ++ta) {
+    const int la_end = min(32, m - 32 * ta);  // centres 32 ta + la
+    for (int la = SPLIT ? part : 0; la < la_end; la += SPLIT ? parts : 1) {
+      const int ka = __shfl_sync(0xffffffffu, key[ta], la);
+      const uint16_t* base = lut + (kMaxN - 1) - ka;
+      int id[kT];
+      unsigned lose = 0u;
 #pragma unroll
-    for (int t = 0; t < kT; ++t) {
-      ids[t] = -1;
-      if (key[t] >= 0 && lane + 32 * t > a) {  // the row partner is alone in its direction
-        const int id = base[key[t]];
-        ids[t] = id;
-        const int sh = (id & 7) << 2;
-        pairs += (int)((atomicAdd(hist + (id >> 3), 1u << sh) >> sh) & 0xFu);
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kT; ++t)
-      if (ids[t] >= 0) hist[ids[t] >> 3] = 0u;
-    __syncwarp();
-    pairs = warp_sum(pairs);
-    ovf |= pairs >= 120;
-    total += pairs;
-  }
-  *overflow = ovf;
-  return total;
-}
-
-// The exact slope count in the 4-bit histogram's space (kDirWords4 words):
-// 8-bit counters for the direction ids of each half, [0, kDirCount / 2) then
-// [kDirCount / 2, kDirCount), one pass per half.  Same results as slope_state.
-static __device__ __noinline__ int slope_state_halves(const int* __restrict__ cs, int n, const uint16_t* __restrict__ lutf,
-                                               uint32_t* __restrict__ hist, int lane, int* __restrict__ bad_out) {
-  constexpr int kT = (kMaxM + 31) / 32;
-  constexpr int kHalf = kDirCount / 2;
-  static_assert(kHalf == 4 * kDirWords4, "one half of the ids fills the 4-bit histogram as 8-bit counters");
-  const int m = 2 * n;
-  int total = 0;
-  for (int a = 0; a < m; ++a) {
-    const int ra = a >> 1;
-    const uint16_t* base = lutf + kFullLutCentre - (ra * kLutW + cs[a]);
-    int ids[kT];
-#pragma unroll
-    for (int t = 0; t < kT; ++t) {
-      const int b = lane + 32 * t;
-      ids[t] = (b < m && (b >> 1) != ra) ? (int)base[(b >> 1) * kLutW + cs[b]] : -1;
-    }
-    int pairs = 0;
-    for (int h = 0; h < 2; ++h) {
-#pragma unroll
-      for (int t = 0; t < kT; ++t) {
-        const int local = ids[t] - h * kHalf;
-        if (ids[t] >= 0 && local >= 0 && local < kHalf) pairs += hist_add(hist, local);
+      for (int t = ta; t < kT; ++t) {
+        const bool in = key[t] >= 0 && (t > ta || lane > (la | 1));
+        id[t] = in ? (int)base[key[t]] : -1;
+        if (in) vtag[id[t]] = (uint8_t)(lane + 32 * t);
       }
       __syncwarp();
+      int win[kT];
 #pragma unroll
-      for (int t = 0; t < kT; ++t) {
-        const int local = ids[t] - h * kHalf;
-        if (ids[t] >= 0 && local >= 0 && local < kHalf) hist_clear(hist, local);
+      for (int t = ta; t < kT; ++t) {
+        win[t] = lane + 32 * t;
+        if (id[t] >= 0) win[t] = vtag[id[t]];
+        lose |= (unsigned)(win[t] != lane + 32 * t) << t;
       }
-      __syncwarp();
+      if (__any_sync(0xffffffffu, lose != 0u)) {
+        uint32_t before[kT];
+#pragma unroll
+        for (int t = ta; t < kT; ++t)
+          if ((lose >> t) & 1u) {
+            before[t] = atomicAdd(word + win[t], kOne) >> 24;
+            total += (int)before[t] + 1;
+          }
+        __syncwarp();
+        if (BAD) {
+          uint32_t others[kT];  // the other slots of the direction
+#pragma unroll
+          for (int t = ta; t < kT; ++t)
+            if ((lose >> t) & 1u) others[t] = *(volatile uint32_t*)(word + win[t]) >> 24;
+          __syncwarp();
+#pragma unroll
+          for (int t = ta; t < kT; ++t)
+            if ((lose >> t) & 1u) {
+              if (before[t] == 0u) {  // the first loser speaks for the winner
+                if (SPLIT && word != bad) {  // uniform
+                  word[win[t]] = 0u;
+                  atomicAdd(bad + win[t], others[t]);
+                } else {
+                  atomicAdd(word + win[t], others[t] - others[t] * kOne);
+                }
+              }
+              atomicAdd(bad + lane + 32 * t, others[t]);
+              atomicAdd(bad + 32 * ta + la, before[t] + 1u);
+            }
+        } else {
+#pragma unroll
+          for (int t = ta; t < kT; ++t)
+            if ((lose >> t) & 1u) word[win[t]] = 0u;
+        }
+      }
     }
-    pairs = warp_sum(pairs);
-    if (bad_out != nullptr && lane == (a & 31)) bad_out[a] = pairs;
-    total += pairs;
   }
-  return total;
+  return warp_sum(total);
 }
-
 
 }  // namespace n3

@@ -268,33 +268,43 @@ __global__ void __launch_bounds__(512, 1) temper_kernel(const TemperArgs A) {
 // Full recompute of every chain's energy (determinant count) and badness
 // (slope count) compared with the maintained values.  One warp per chain.
 constexpr int kAuditWarps = 4;
-constexpr size_t kAuditSmem = kFullLutBytes + kAuditWarps * (sizeof(uint32_t) * kDirWords + 2 * sizeof(int) * kMaxM);
+constexpr size_t kAuditSmem = kTagLutBytes + kAuditWarps * (kTagWarpBytes + sizeof(int) * kMaxM);
 
 __global__ void __launch_bounds__(kAuditWarps * 32) audit_kernel(const n3_chains ch, const uint16_t* __restrict__ g_lut,
                                                                    int32_t* mismatch) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
-  uint32_t* hist_all = reinterpret_cast<uint32_t*>(smem + kFullLutBytes);
-  int* cs_all = reinterpret_cast<int*>(hist_all + kAuditWarps * kDirWords);
-  int* bs_all = cs_all + kAuditWarps * kMaxM;
-  full_lut_copy(lut, g_lut);
-  for (int i = threadIdx.x; i < kAuditWarps * kDirWords; i += blockDim.x) hist_all[i] = 0u;
+  tag_lut_copy(lut, g_lut);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int* cs = cs_all + warp * kMaxM;
-  int* bs = bs_all + warp * kMaxM;
-  uint32_t* hist = hist_all + warp * kDirWords;
+  uint8_t* tag = smem + kTagLutBytes + warp * (kTagWarpBytes + sizeof(int) * kMaxM);
+  uint32_t* bs = reinterpret_cast<uint32_t*>(tag + kDirCount);
+  int* cs = reinterpret_cast<int*>(bs + kMaxM);
   for (int c = blockIdx.x * kAuditWarps + warp; c < ch.n_chains; c += gridDim.x * kAuditWarps) {
     const int n = ch.ladder_n[c / ch.ladder_size], m = 2 * n;
-    for (int s = lane; s < m; s += 32) cs[s] = ch.cols[(size_t)c * kMaxM + s];
+    int key[kSlotsPerLane];
+    int ok = 1;
+#pragma unroll
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      const int s = lane + 32 * t;
+      const int col = s < m ? (int)ch.cols[(size_t)c * kMaxM + s] : 0;
+      if (s < m) {
+        ok &= col >= 0 && col < kMaxN;
+        cs[s] = col;
+        bs[s] = 0u;
+      }
+      key[t] = s < m ? (s >> 1) * kLutW + col : -1;
+    }
+    ok = __all_sync(0xffffffffu, ok);
     __syncwarp();
-    const int e = warp_sum(det_state<false>(cs, n, lane, nullptr));
-    slope_state(cs, n, lut, hist, lane, bs);
-    __syncwarp();
-    int bad_ok = 1;
-    for (int s = lane; s < m; s += 32) bad_ok &= bs[s] == ch.badness[(size_t)c * kMaxM + s];
-    bad_ok = __all_sync(0xffffffffu, bad_ok);
-    if (lane == 0 && (e != ch.energy[c] || !bad_ok)) {
+    if (ok) {  // uniform: every column is on the grid
+      const int e = warp_sum(det_state<false>(cs, n, lane, nullptr));
+      tag_state<true>(key, m, lut, tag, lane, bs, bs);
+      __syncwarp();
+      for (int s = lane; s < m; s += 32) ok &= (int)bs[s] == ch.badness[(size_t)c * kMaxM + s];
+      ok = __all_sync(0xffffffffu, ok) && e == ch.energy[c];
+    }
+    if (lane == 0 && !ok) {
       atomicAdd(mismatch, 1);
       if (ch.error_word) atomicOr(ch.error_word, kErrAudit);
     }
@@ -422,7 +432,7 @@ int n3_temper_audit(const n3_chains* chains, int32_t* mismatch, void* stream) {
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::audit_kernel), smem));
   const int want = (ch.n_chains + n3::kAuditWarps - 1) / n3::kAuditWarps;
   const int grid = want < n3host::sm_count() * 4 ? want : n3host::sm_count() * 4;
-  n3::audit_kernel<<<grid, n3::kAuditWarps * 32, smem, (cudaStream_t)stream>>>(ch, n3host::dir_lut_full_device_ptr(),
+  n3::audit_kernel<<<grid, n3::kAuditWarps * 32, smem, (cudaStream_t)stream>>>(ch, n3host::dir_lut_device_ptr(),
                                                                                  mismatch);
   return n3host::check_launch("audit_kernel");
 }
