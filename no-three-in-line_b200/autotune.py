@@ -8,13 +8,9 @@ src/no_three_75/hardware.py:48-80).  Here the choices are measured:
 * threads per chain (32, 64, 128 or 256) and chains per CTA (`cpb`), searched
   together: every pair the ladder admits (at most 16 warps per CTA; cpb a
   divisor of L with at most 8 CTAs per cluster, or a multiple of L) is timed on
-  a copy of the chains and the fastest kept.  A team of 2, 4 or 8 warps shares
-  one chain's direction histogram (one 8-bit counter per gcd-reduced
-  direction, 6.8 KB of shared memory per chain) and splits its 2n slots, so a
-  proposal takes fewer dependent steps at the price of barriers and fewer
-  chains per SM: wider teams win when there are too few chains to fill the
-  GPU's warps (the reference's default of 128 replicas), one warp per chain
-  when there are thousands.
+  a copy of the chains and the fastest kept.  One warp works on a chain at
+  every width, so the width only bounds cpb; fewer chains per CTA leave each
+  warp more of its SM when there are too few chains to fill the GPU.
 * per-size sweeps per launch: in one mixed-size launch every CTA runs its own
   ladders' rounds, and the launch ends with its slowest CTA.  The tuner times
   each size alone, then gives each size a number of sweeps proportional to its

@@ -64,6 +64,15 @@ __device__ __forceinline__ void full_lut_copy(uint16_t* __restrict__ dst, const 
   for (int i = threadIdx.x; i < (int)(kFullLutBytes / 16); i += blockDim.x) d[i] = s[i];
 }
 
+// The compact tables' bytes, padded to 16, and their copy into shared memory.
+constexpr size_t kCompactLutBytes = ((sizeof(uint16_t) * kLutSize + 15) / 16) * 16;
+__device__ __forceinline__ void compact_lut_copy(uint16_t* __restrict__ dst, const uint16_t* __restrict__ lut) {
+  const uint4* s = reinterpret_cast<const uint4*>(lut);
+  uint4* d = reinterpret_cast<uint4*>(dst);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < (int)(kCompactLutBytes / 16); i += blockDim.x) d[i] = s[i];
+}
+
 __device__ __forceinline__ int dir_id_full(const uint16_t* __restrict__ lutf, int dx, int dy) {
   return lutf[dx * kLutW + dy + kFullLutCentre];
 }
@@ -86,6 +95,12 @@ namespace n3host {
 // Device address of the direction table on the current device (set-up on
 // first use by ensure_device_tables).
 const uint16_t* dir_lut_device_ptr();
+// Device address of the table of primitive steps: entry |d| + kMaxN - 1 of a key
+// difference d holds four times the key a * kLutW + b of its gcd-reduced step
+// (compact-table size, padded to 16 bytes).
+const uint16_t* prim4_lut_device_ptr();
+// The same for four times the compact id, kDirCount at d = 0.
+const uint16_t* dir4_lut_device_ptr();
 // Device address of the full signed table built from it (kFullLutBytes).
 const uint16_t* dir_lut_full_device_ptr();
 }  // namespace n3host

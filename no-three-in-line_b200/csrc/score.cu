@@ -39,8 +39,10 @@
 
 namespace n3 {
 
-__device__ __align__(16) uint16_t g_dir_lut[kTagLutBytes / 2];
+__device__ __align__(16) uint16_t g_dir_lut[kCompactLutBytes / 2];
 __device__ __align__(16) uint16_t g_dir_lut_full[kFullLutBytes / 2];
+__device__ __align__(16) uint16_t g_prim4_lut[kCompactLutBytes / 2];
+__device__ __align__(16) uint16_t g_dir4_lut[kCompactLutBytes / 2];
 __device__ int g_dir_count;
 
 __device__ __forceinline__ int gcd_dev(int a, int b) {
@@ -62,7 +64,8 @@ __device__ __forceinline__ bool is_primitive(int e) {
 }
 
 // One block: numbers the primitive directions in (p, q) order, then maps every
-// difference vector to the id of its gcd-reduced direction.
+// difference vector to the id of its gcd-reduced direction, to four times that
+// (kDirCount for (0, 0)) and to four times the key p * kLutW + q of the direction.
 __global__ void __launch_bounds__(1024) build_dir_lut_kernel() {
   __shared__ uint16_t prim[kLutSize];
   __shared__ int scan[1024];
@@ -86,13 +89,16 @@ __global__ void __launch_bounds__(1024) build_dir_lut_kernel() {
   for (int e = tid; e < kLutSize; e += 1024) {
     const int dx = e / kLutW, dy = e % kLutW - (kMaxN - 1);
     const int g = gcd_dev(dx, dy);
-    uint16_t v = 0xFFFFu;  // (0, 0) has no direction
+    uint16_t v = 0xFFFFu, step = 0;  // (0, 0) has no direction
     if (g) {
       const int p = dx / g;
       const int q = p == 0 ? 1 : dy / g;  // (0, -1) ~ (0, 1)
       v = prim[p * kLutW + q + (kMaxN - 1)];
+      step = (uint16_t)(4 * (p * kLutW + q));
     }
     g_dir_lut[e] = v;
+    g_prim4_lut[e] = step;
+    g_dir4_lut[e] = (uint16_t)(4 * (g ? v : kDirCount));
   }
 }
 
@@ -188,7 +194,7 @@ enum TagMode { kCount, kSlope, kChecked };
 constexpr int kTagWarps = 28;  // 28 x 148 = 4144 states at once; 32 would need 6.4 KB each beside the table
 constexpr int kTagMaxParts = 16;     // warps that share a state
 constexpr int kTagMinThreads = 256;  // threads that copy the table when few states are scored
-__host__ __device__ constexpr size_t tag_smem(int warps) { return kTagLutBytes + (size_t)warps * kTagWarpBytes; }
+__host__ __device__ constexpr size_t tag_smem(int warps) { return kCompactLutBytes + (size_t)warps * kTagWarpBytes; }
 static_assert(tag_smem(kTagWarps) <= 227 * 1024, "tag_kernel shared memory");
 static_assert(kDirCount >= (int)sizeof(int) * kMaxM, "a state's columns fit in a warp's tags");
 
@@ -202,17 +208,17 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int total_all[kTagWarps];
   uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
-  tag_lut_copy(lut, g_lut);
+  compact_lut_copy(lut, g_lut);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp >= W) return;  // it only helped to copy the table
   const int m = 2 * n;
   if (!SPLIT) parts = 1;
   const int group = warp / parts, part = warp % parts;
-  uint8_t* tag = smem + kTagLutBytes + (size_t)warp * kTagWarpBytes;
+  uint8_t* tag = smem + kCompactLutBytes + (size_t)warp * kTagWarpBytes;
   // the group's badness and count live with its first warp
   uint32_t* word = reinterpret_cast<uint32_t*>(tag + kDirCount);
-  uint32_t* bad = reinterpret_cast<uint32_t*>(smem + kTagLutBytes + (size_t)group * parts * kTagWarpBytes + kDirCount);
+  uint32_t* bad = reinterpret_cast<uint32_t*>(smem + kCompactLutBytes + (size_t)group * parts * kTagWarpBytes + kDirCount);
   int* total = total_all + group;
   auto group_sync = [&]() {  // at most 14 groups of more than one warp: barrier ids 1 .. 14
     if (!SPLIT)
@@ -307,6 +313,18 @@ int build_dir_lut(cudaStream_t st) {
 const uint16_t* dir_lut_device_ptr() {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, n3::g_dir_lut) != cudaSuccess) return nullptr;
+  return static_cast<const uint16_t*>(p);
+}
+
+const uint16_t* prim4_lut_device_ptr() {
+  void* p = nullptr;
+  if (cudaGetSymbolAddress(&p, n3::g_prim4_lut) != cudaSuccess) return nullptr;
+  return static_cast<const uint16_t*>(p);
+}
+
+const uint16_t* dir4_lut_device_ptr() {
+  void* p = nullptr;
+  if (cudaGetSymbolAddress(&p, n3::g_dir4_lut) != cudaSuccess) return nullptr;
   return static_cast<const uint16_t*>(p);
 }
 

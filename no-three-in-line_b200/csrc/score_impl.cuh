@@ -233,39 +233,7 @@ __device__ __forceinline__ int det_state(const int* __restrict__ cs, int n, int 
 // difference d = key(k) - key(a) > 0 is lut[d + kMaxN - 1].  tag: this warp's
 // kDirCount bytes, any contents.  word[s] (shared memory, zeroed): with BAD, the
 // number of triples holding slot s on return (at most C(149, 2), below 2^24).
-constexpr size_t kTagLutBytes = ((sizeof(uint16_t) * kLutSize + 15) / 16) * 16;
 constexpr size_t kTagWarpBytes = kDirCount + sizeof(uint32_t) * kMaxM;  // the tags, then word[]
-
-// Copies the compact table (n3host::dir_lut_device_ptr) into shared memory; all
-// threads of the block call it.
-__device__ __forceinline__ void tag_lut_copy(uint16_t* __restrict__ dst, const uint16_t* __restrict__ g_lut) {
-  const uint4* s = reinterpret_cast<const uint4*>(g_lut);
-  uint4* d = reinterpret_cast<uint4*>(dst);
-#pragma unroll 4
-  for (int i = threadIdx.x; i < (int)(kTagLutBytes / 16); i += blockDim.x) d[i] = s[i];
-}
-
-template <bool BAD>
-static __device__ __noinline__ int tag_centre_hist(int a, int ka, const int (&key)[kSlotsPerLane],
-                                                   const uint16_t* __restrict__ lut, uint8_t* __restrict__ tag,
-                                                   int lane, int* __restrict__ bad) {
-  uint32_t* hist = reinterpret_cast<uint32_t*>(tag);
-  __syncwarp();
-  for (int i = lane; i < kDirWords; i += 32) hist[i] = 0u;
-  __syncwarp();
-  int pairs = 0;
-  for (int t = 0; t < kSlotsPerLane; ++t)
-    if (lane + 32 * t > (a | 1) && key[t] >= 0) pairs += hist_add(hist, lut[key[t] - ka + kMaxN - 1]);
-  __syncwarp();
-  if (BAD) {
-    for (int t = 0; t < kSlotsPerLane; ++t)
-      if (lane + 32 * t > (a | 1) && key[t] >= 0)
-        atomicAdd(bad + lane + 32 * t, hist_get(hist, lut[key[t] - ka + kMaxN - 1]) - 1);
-    if (pairs) atomicAdd(bad + a, pairs);
-  }
-  __syncwarp();
-  return pairs;
-}
 
 // SPLIT: only the centres part, part + parts, ... are counted (parts a power of
 // two up to 32), so that `parts` warps can share a state.  Each then counts its

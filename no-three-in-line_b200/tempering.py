@@ -166,8 +166,8 @@ class TemperingChains:
         self.ladder_n_host = np.asarray(ladder_n, np.int32)
         self.n = int(self.ladder_n_host.max())
         self.seed = int(seed) & 0xFFFFFFFFFFFFFFFF
-        # launch shape (threads that evaluate one chain's moves: 32, 64, 128
-        # or 256; chains per CTA, None for the default), e.g. the autotuner's
+        # launch shape (threads per chain: 32, 64, 128 or 256, which bounds the
+        # chains per CTA; those, None for the default), e.g. the autotuner's
         # choice; results do not depend on it
         self.threads_per_chain = 32
         self.chains_per_block = None
