@@ -23,8 +23,8 @@
 
 #include <climits>
 
-#include "chain_move.cuh"
 #include "dirs.cuh"
+#include "pair_move.cuh"
 #include "pyrandom.cuh"
 #include "n3_common.cuh"
 
@@ -208,12 +208,13 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
 // --------------------------------------------------------------------------
 // Children's scores by exact deltas: warp per child, the parent's columns and
 // badness in shared memory, then each recorded swap applied with its exact dE
-// and the exact update of every badness (team_move<1, true>: the tempering
-// move by one warp, without the Metropolis test).  E and badness equal a full
-// recount.
+// and the exact update of every badness (pair_move, accepting every move).  E
+// and badness equal a full recount.
 // --------------------------------------------------------------------------
-constexpr int kDeltaWarps = 22;
-constexpr size_t kDeltaSmem = kFullLutBytes + kDeltaWarps * (sizeof(uint32_t) * kDirWords + 2 * sizeof(int) * kMaxM);
+constexpr int kDeltaWarps = 26;
+constexpr size_t kDeltaWarpBytes = 2 * sizeof(uint32_t) * DenseNumbering::kWords + sizeof(int) * kMaxM + 152;
+constexpr size_t kDeltaSmem = kCompactLutBytes + kDeltaWarps * kDeltaWarpBytes;
+static_assert(kDeltaSmem <= 227 * 1024 && kDeltaWarpBytes % 8 == 0, "child_delta_kernel shared memory");
 
 struct DeltaArgs {
   const int32_t* ep;
@@ -225,7 +226,7 @@ struct DeltaArgs {
   const int32_t* nmoves;
   int moves_cap, n, population;
   const int64_t* status;
-  const uint16_t* lutf;
+  const uint16_t* lut4;
   int32_t* scores;
   int32_t* badness;
   uint32_t* error_word;
@@ -234,39 +235,43 @@ struct DeltaArgs {
 __global__ void __launch_bounds__(kDeltaWarps * 32, 1) child_delta_kernel(const DeltaArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (A.status[1] == 0) return;  // uniform: the search has reached E = 0
-  uint16_t* lutf = reinterpret_cast<uint16_t*>(smem);
-  uint32_t* hist_all = reinterpret_cast<uint32_t*>(smem + kFullLutBytes);
-  int* cs_all = reinterpret_cast<int*>(hist_all + kDeltaWarps * kDirWords);
-  int* bs_all = cs_all + kDeltaWarps * kMaxM;
-  full_lut_copy(lutf, A.lutf);
-  for (int i = threadIdx.x; i < kDeltaWarps * kDirWords / 4; i += blockDim.x)
-    reinterpret_cast<uint4*>(hist_all)[i] = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();
+  uint16_t* lut4 = reinterpret_cast<uint16_t*>(smem);
+  compact_lut_copy(lut4, A.lut4);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = A.n, m = 2 * n;
-  int* cs = cs_all + warp * kMaxM;
-  int* bs = bs_all + warp * kMaxM;
-  uint32_t* hist = hist_all + warp * kDirWords;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + kCompactLutBytes + (size_t)warp * kDeltaWarpBytes);
+  for (int i = lane; i < 2 * DenseNumbering::kWords; i += 32) hist[i] = 0u;
+  __syncthreads();
+  const int n = A.n, m = 2 * n, nt = (m + 31) >> 5;
+  WarpState W;
+  W.m = m;
+  W.lane = lane;
+  W.bs = reinterpret_cast<int*>(hist + 2 * DenseNumbering::kWords);
+  W.cs = reinterpret_cast<uint8_t*>(W.bs + kMaxM);
   uint32_t err = 0;
   for (int c = blockIdx.x * kDeltaWarps + warp; c < A.population; c += gridDim.x * kDeltaWarps) {
     const int par = A.parent[c];
-    for (int s = lane; s < m; s += 32) {
-      cs[s] = (s & 1) ? A.eq[(size_t)par * n + (s >> 1)] : A.ep[(size_t)par * n + (s >> 1)];
-      bs[s] = A.ebad[(size_t)par * m + s];
+#pragma unroll
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      const int s = W.slot(t);
+      W.key2[t] = 0;
+      if (s < m) {
+        const int col = (s & 1) ? A.eq[(size_t)par * n + (s >> 1)] : A.ep[(size_t)par * n + (s >> 1)];
+        W.cs[s] = (uint8_t)col;
+        W.key2[t] = 2 * ((s >> 1) * kLutW + col);
+        W.bs[s] = A.ebad[(size_t)par * m + s];
+      }
     }
     __syncwarp();
-    Team<1> tm{lane, 0, nullptr, 0, {}};
-    team_load_keys(tm, cs, m);  // the slots' table keys, kept in registers across the moves
     int E = A.es[par];
     const int k_end = min(A.nmoves[c], A.moves_cap);
     for (int k = 0; k < k_end; ++k) {
       const int mv = A.moves[(size_t)c * A.moves_cap + k];
       int dE;
-      team_move<1, true, false, false, true>(tm, cs, bs, m, lutf, hist, mv & 0xFF, (mv >> 8) & 0xFF, 0u, nullptr, 0,
-                                             E, err, &dE);
+      pair_move_any<DenseNumbering>(W, lut4, hist, nt, prepare_move(W, mv & 0xFF, (mv >> 8) & 0xFF),
+                                    [](int) { return true; }, E, err, &dE);
     }
     if (lane == 0) A.scores[c] = E;
-    for (int s = lane; s < m; s += 32) A.badness[(size_t)c * m + s] = bs[s];
+    for (int s = lane; s < m; s += 32) A.badness[(size_t)c * m + s] = W.bs[s];
     __syncwarp();
   }
   if (lane == 0 && err && A.error_word) atomicOr(A.error_word, err);
@@ -1200,7 +1205,7 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   D.n = b->n;
   D.population = b->population;
   D.status = b->status;
-  D.lutf = n3host::dir_lut_full_device_ptr();
+  D.lut4 = n3host::dir4_lut_device_ptr();
   D.scores = b->child_scores;
   D.badness = b->child_badness;
   D.error_word = b->error_word;
