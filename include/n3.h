@@ -188,12 +188,12 @@ typedef struct n3_temper_config {
   int exchange;                 /* 1: neighbour exchange after every round */
   int target_energy;            /* >= 0: record the first chain reaching E <= target (and raise *stop) */
   int bad_bias;                 /* percent of proposals whose slot u is drawn by badness (tempering.py:51-55) */
-  int threads_per_chain;        /* 32 (or 0), 64, 128 or 256: warps that evaluate one chain's moves together;
-                                   chains_per_block x threads_per_chain / 32 <= 16 warps per CTA */
+  int threads_per_chain;        /* 32 (or 0), 64, 128 or 256; bounds the launch (chains_per_block x
+                                   threads_per_chain / 32 <= 16).  Each chain is worked on by one warp. */
 } n3_temper_config;
 
 /* Runs cfg->rounds rounds (proposals, then an exchange) on every ladder in one
- * persistent launch: grid C/cpb CTAs of cpb x threads_per_chain threads,
+ * persistent launch: grid C/cpb CTAs of cpb warps,
  * clusters of L/cpb CTAs when a ladder spans several CTAs.  Results do not
  * depend on cpb or threads_per_chain (the same proposals, dE and acceptances).  Capturable in a CUDA graph (fixed
  * arguments; the per-device tables must have been set up by an earlier call).
@@ -266,11 +266,10 @@ int n3_mlp_infer(const n3_mlp* mlp, int tiles, void* stream);
  * advances the step counter.  temps: the ladder's L temperatures (device). */
 int n3_mlp_step(const n3_chains* chains, const n3_mlp* mlp, const float* temps, uint64_t seed, int moves,
                 void* stream);
-/* The same step with the width of the team that works on one chain chosen by
- * the caller: threads_per_chain 32 (one warp) or 64 (two warps sharing the
- * chain's histogram); 0 takes the default (64 for several moves per step, 32
- * for one).  No counterpart in the reference.  Results do not depend on the
- * width.  A ring buffer capacity below 1 is rejected with N3_ERR_ARG. */
+/* The same step; threads_per_chain 0, 32 or 64 is accepted and changes nothing
+ * (one warp works on a chain; pairs of warps were an earlier choice).  No
+ * counterpart in the reference.  A ring buffer capacity below 1 is rejected with
+ * N3_ERR_ARG. */
 int n3_mlp_step_team(const n3_chains* chains, const n3_mlp* mlp, const float* temps, uint64_t seed, int moves,
                      int threads_per_chain, void* stream);
 /* One Adam step on a batch drawn from the ring slots recorded so far (all

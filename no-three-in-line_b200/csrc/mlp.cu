@@ -30,9 +30,9 @@
 #include <mutex>
 #include <math.h>
 
-#include "chain_move.cuh"
 #include "dirs.cuh"
 #include "n3_common.cuh"
+#include "pair_move.cuh"
 #include "philox.cuh"
 #include "umma.cuh"
 
@@ -487,14 +487,12 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(const InferArgs
 // Learned step: sample one candidate per chain from softmax(-pred / T), score
 // it exactly, Metropolis-accept with the chain's threshold row, update the
 // state and badness, and push the (features, exact dE) tuple to the ring.
-// One team of WPC warps per chain (1 or 2), state in shared memory (as in the
-// tempering kernel).  Every warp of a team runs the same draw on the same
-// registers, so the team needs no broadcast; the exact move splits its slots
-// over the team.
+// One warp per chain, state in shared memory, the exact move from two
+// histograms at a time (pair_move.cuh).
 // ---------------------------------------------------------------------------
 struct StepArgs {
   n3_chains ch;
-  const uint16_t* lut;
+  const uint16_t* lut4;   // StepNumbering's table
   const float* temps;     // [L] ladder temperatures
   const int32_t* cand;    // [C][128]
   const float* pred;      // [C][128]
@@ -511,37 +509,46 @@ struct StepArgs {
 
 constexpr int kStepChains = 14;  // chains per CTA: 2048 chains -> 147 CTAs, one per SM
 
-template <int WPC>
-__global__ void __launch_bounds__(kStepChains * 32 * WPC, 1) learned_step_kernel(const StepArgs A) {
-  constexpr int TT = Team<WPC>::kThreads;
+constexpr size_t kStepChainBytes = 2 * sizeof(uint32_t) * StepNumbering::kWords + sizeof(int) * kMaxM +
+                                   kCand * (sizeof(int) + sizeof(float)) + 152;
+constexpr size_t kStepSmem = kCompactLutBytes + kStepChains * kStepChainBytes;
+static_assert(kStepSmem <= 227 * 1024 && kStepChainBytes % 16 == 0, "learned_step_kernel shared memory");
+
+__global__ void __launch_bounds__(kStepChains * 32, 1) learned_step_kernel(const StepArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const n3_chains& ch = A.ch;
-  uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
-  uint32_t* hist_all = reinterpret_cast<uint32_t*>(smem + kFullLutBytes);
-  int* cs_all = reinterpret_cast<int*>(hist_all + kStepChains * kDirWords);
-  int* bs_all = cs_all + kStepChains * kMaxM;
-  int* team_red = bs_all + kStepChains * kMaxM;  // 2 WPC ints per chain (WPC > 1)
-  int* cand_all = team_red + kStepChains * 4;    // this step's candidate codes and predictions
-  float* pred_all = reinterpret_cast<float*>(cand_all + kStepChains * kCand);
-  full_lut_copy(lut, A.lut);
-  for (int i = threadIdx.x; i < kStepChains * kDirWords / 4; i += blockDim.x)
-    reinterpret_cast<uint4*>(hist_all)[i] = make_uint4(0u, 0u, 0u, 0u);
+  uint16_t* lut4 = reinterpret_cast<uint16_t*>(smem);
+  compact_lut_copy(lut4, A.lut4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char* mine = smem + kCompactLutBytes + (size_t)warp * kStepChainBytes;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(mine);
+  int* cand_c = reinterpret_cast<int*>(hist + 2 * StepNumbering::kWords);  // this step's candidate codes and
+  float* pred_c = reinterpret_cast<float*>(cand_c + kCand);               // predictions
+  int* bs = reinterpret_cast<int*>(pred_c + kCand);
+  uint8_t* cs = reinterpret_cast<uint8_t*>(bs + kMaxM);
+  for (int i = lane; i < 2 * StepNumbering::kWords / 4; i += 32)
+    reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  const int team = threadIdx.x / TT;  // this chain's index in the CTA
-  Team<WPC> tm{(int)threadIdx.x % TT, 1 + team, team_red + 2 * WPC * team, 0, {}};
-  const int lane = tm.t & 31;
-  const int c = blockIdx.x * kStepChains + team;
-  if (c >= ch.n_chains) return;  // the whole team leaves; no block-level barrier follows
+  const int c = blockIdx.x * kStepChains + warp;
+  if (c >= ch.n_chains) return;  // no block-level barrier follows
   const int L = ch.ladder_size;
-  const int n = ch.ladder_n[c / L], m = 2 * n;
-  int* cs = cs_all + team * kMaxM;
-  int* bs = bs_all + team * kMaxM;
-  uint32_t* hist = hist_all + team * kDirWords;
-  for (int s = tm.t; s < m; s += TT) {
-    cs[s] = ch.cols[(size_t)c * kMaxM + s];
-    bs[s] = ch.badness[(size_t)c * kMaxM + s];
+  const int n = ch.ladder_n[c / L], m = 2 * n, nt = (m + 31) >> 5;
+  WarpState W;
+  W.m = m;
+  W.lane = lane;
+  W.cs = cs;
+  W.bs = bs;
+#pragma unroll
+  for (int t = 0; t < kSlotsPerLane; ++t) {
+    const int s = W.slot(t);
+    W.key2[t] = 0;
+    if (s < m) {
+      const int col = ch.cols[(size_t)c * kMaxM + s];
+      cs[s] = (uint8_t)col;
+      bs[s] = ch.badness[(size_t)c * kMaxM + s];
+      W.key2[t] = 2 * ((s >> 1) * kLutW + col);
+    }
   }
-  team_load_keys(tm, cs, m);  // the thread's own slots' table keys, kept in registers across the moves
   const int temp = ch.temp_of[c];
   const float T = A.temps[temp];
   // softmax(-pred / T) over the legal candidates, sampled by inverse CDF;
@@ -553,17 +560,13 @@ __global__ void __launch_bounds__(kStepChains * 32 * WPC, 1) learned_step_kernel
   static_assert(kPer == 4, "four candidates per lane");
   // The codes and predictions also go to shared memory, where a draw reads the
   // picked one (registers hold only the weights).
-  int* cand_c = cand_all + team * kCand;
-  float* pred_c = pred_all + team * kCand;
   float w[kPer];
   float mx = -INFINITY;
   {
     const int4 cw4 = reinterpret_cast<const int4*>(A.cand + (size_t)c * kCand)[lane];
     const float4 pr4 = reinterpret_cast<const float4*>(A.pred + (size_t)c * kCand)[lane];
-    if (tm.t < 32) {
-      reinterpret_cast<int4*>(cand_c)[lane] = cw4;
-      reinterpret_cast<float4*>(pred_c)[lane] = pr4;
-    }
+    reinterpret_cast<int4*>(cand_c)[lane] = cw4;
+    reinterpret_cast<float4*>(pred_c)[lane] = pr4;
     const int cwv[kPer] = {cw4.x, cw4.y, cw4.z, cw4.w};
     const float prv[kPer] = {pr4.x, pr4.y, pr4.z, pr4.w};
 #pragma unroll
@@ -572,7 +575,7 @@ __global__ void __launch_bounds__(kStepChains * 32 * WPC, 1) learned_step_kernel
       mx = fmaxf(mx, w[q]);
     }
   }
-  tm.sync();  // the state and the candidates are read by the whole team from here on
+  __syncwarp();  // the state and the candidates are read by the whole warp from here on
 #pragma unroll
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
 #pragma unroll
@@ -581,7 +584,7 @@ __global__ void __launch_bounds__(kStepChains * 32 * WPC, 1) learned_step_kernel
   int E = ch.energy[c];
   int bestE = ch.best_energy[c];
   uint32_t err = 0, n_acc = 0, n_scored = 0;
-  int sum_dE_acc = 0;  // with n_acc, n_scored and st_abs: this chain's statistics (team-uniform)
+  int sum_dE_acc = 0;  // with n_acc, n_scored and st_abs: this chain's statistics (warp-uniform)
   float st_abs = 0.f;
   // the moves' Philox blocks 32 at a time: lane l makes move k0 + l's, move k takes lane k % 32's
   U4 batch = {0u, 0u, 0u, 0u};
@@ -637,42 +640,46 @@ __global__ void __launch_bounds__(kStepChains * 32 * WPC, 1) learned_step_kernel
     }
     const int u = cw & 0xFF, v = (cw >> 8) & 0xFF;
     if (k > 0 && !legal_swap(cs, u, v)) continue;  // an earlier move of this step made it illegal
-    // tuple: features of the state before the move (thread i writes feature i).
-    // These reads of cs and bs come before the move's first team barrier, and
-    // the move writes the state only after later ones.
+    // tuple: features of the state before the move (lane i writes feature i)
     int64_t slot = slot0 + k;
     if (slot >= A.rb_cap) {
       slot -= A.rb_cap;
       if (slot >= A.rb_cap) slot %= A.rb_cap;
     }
-    if (tm.t < kCandFeat) {
-      const int which = tm.t & 3;
+    if (lane < kCandFeat) {
+      const int which = lane & 3;
       const int sidx = which == 0 ? u : which == 1 ? v : which == 2 ? (u ^ 1) : (v ^ 1);
-      const float f = tm.t < 4 ? (float)bs[sidx] * (1.0f / 16.0f)
-                               : (float)(tm.t < 8 ? (sidx >> 1) : cs[sidx]) * (1.0f / (float)n);
-      A.rb_feat[slot * kCandFeat + tm.t] = bf16_bits(f);
+      const float f = lane < 4 ? (float)bs[sidx] * (1.0f / 16.0f)
+                               : (float)(lane < 8 ? (sidx >> 1) : cs[sidx]) * (1.0f / (float)n);
+      A.rb_feat[slot * kCandFeat + lane] = bf16_bits(f);
     }
-    for (int s = tm.t; s < kChainFeat; s += TT)
-      A.rb_bad[slot * kChainFeat + s] = (uint8_t)(s < m ? min(bs[s], 255) : 0);
+#pragma unroll
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      const int s = W.slot(t);
+      if (s < kChainFeat) A.rb_bad[slot * kChainFeat + s] = (uint8_t)(s < m ? min(bs[s], 255) : 0);
+    }
     int dE = 0;
-    const uint32_t* thr = ch.acc_thresh + (size_t)temp * ch.acc_width;  // formed here: fewer live registers
-    const int acc = team_move<WPC, false, false, false, true>(tm, cs, bs, m, lut, hist, u, v, r.y, thr, ch.acc_width,
-                                                              E, err, &dE);
-    if (tm.t == 0) A.rb_dE[slot] = (int16_t)max(-32768, min(32767, dE));
+    const uint32_t* thr = ch.acc_thresh + (size_t)temp * ch.acc_width;
+    const int width = ch.acc_width;
+    const uint32_t z = r.y;
+    const bool acc = pair_move_any<StepNumbering>(
+        W, lut4, hist, nt, prepare_move(W, u, v),
+        [=](int d) { return d <= 0 || (d < width && z < thr[d]); }, E, err, &dE);
+    if (lane == 0) A.rb_dE[slot] = (int16_t)max(-32768, min(32767, dE));
     n_acc += acc ? 1u : 0u;
     st_abs += fabsf(p - (float)dE);
     n_scored += 1u;
     if (acc) sum_dE_acc += dE;
     if (acc && E < bestE) {
       bestE = E;
-      for (int s = tm.t; s < m; s += TT) ch.best_cols[(size_t)c * kMaxM + s] = (int16_t)cs[s];
+      for (int s = lane; s < m; s += 32) ch.best_cols[(size_t)c * kMaxM + s] = (int16_t)cs[s];
     }
   }
-  for (int s = tm.t; s < m; s += TT) {
+  for (int s = lane; s < m; s += 32) {
     ch.cols[(size_t)c * kMaxM + s] = (int16_t)cs[s];
     ch.badness[(size_t)c * kMaxM + s] = bs[s];
   }
-  if (tm.t == 0) {
+  if (lane == 0) {
     ch.energy[c] = E;
     ch.best_energy[c] = bestE;
     ch.accepted[c] += n_acc;
@@ -970,21 +977,10 @@ static int launch_pack(const n3_mlp* M, cudaStream_t st) {
   return check_launch("mlp pack_kernel");
 }
 
-static size_t step_smem() {  // the team scratch is sized for the widest team (2 warps)
-  return n3::kFullLutBytes + kStepChains * (sizeof(uint32_t) * n3::kDirWords + 2 * sizeof(int) * n3::kMaxM +
-                                            4 * sizeof(int) + kCand * (sizeof(int) + sizeof(float)));
-}
-
-// Threads per chain of the learned step when the caller leaves it open: two
-// warps for several moves per step (2048 chains x 16 moves: 6.50 against
-// 6.68 ms per 50 steps), one for a single move (4.31 against 4.33 ms).
-static int default_step_threads(int moves) { return moves > 1 ? 64 : 32; }
-
 int prepare_mlp() {
   N3_TRY(allow_smem(reinterpret_cast<const void*>(infer_kernel), kInferSmem));
   N3_TRY(allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<3>), kTcSmem));
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(learned_step_kernel<1>), step_smem()));
-  return allow_smem(reinterpret_cast<const void*>(learned_step_kernel<2>), step_smem());
+  return allow_smem(reinterpret_cast<const void*>(learned_step_kernel), kStepSmem);
 }
 
 }  // namespace n3host
@@ -1126,14 +1122,12 @@ int n3_mlp_step_team(const n3_chains* ch, const n3_mlp* M, const float* temps, u
   if (!ch || !M || !temps) return n3host::set_error(N3_ERR_ARG, "null descriptor");
   if (moves < 1 || moves > kCand) return n3host::set_error(N3_ERR_RANGE, "moves per step %d outside [1, 128]", moves);
   if (M->rb_capacity < 1) return n3host::set_error(N3_ERR_ARG, "ring buffer capacity %lld", (long long)M->rb_capacity);
-  if (threads_per_chain == 0) threads_per_chain = n3host::default_step_threads(moves);
-  if (threads_per_chain != 32 && threads_per_chain != 64)
+  if (threads_per_chain != 0 && threads_per_chain != 32 && threads_per_chain != 64)
     return n3host::set_error(N3_ERR_RANGE, "threads per chain %d: the learned step takes 32 or 64", threads_per_chain);
   N3_TRY(n3host::ensure_device_tables());
-  const size_t smem = n3host::step_smem();
   StepArgs A;
   A.ch = *ch;
-  A.lut = n3host::dir_lut_full_device_ptr();
+  A.lut4 = n3host::prim4_lut_device_ptr();
   A.temps = temps;
   A.cand = M->cand;
   A.pred = M->pred;
@@ -1147,13 +1141,8 @@ int n3_mlp_step_team(const n3_chains* ch, const n3_mlp* M, const float* temps, u
   A.stats = M->stats;
   A.moves = moves;
   const int grid = (ch->n_chains + kStepChains - 1) / kStepChains;
-  if (threads_per_chain == 64) {
-    N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(learned_step_kernel<2>), smem));
-    learned_step_kernel<2><<<grid, kStepChains * 64, smem, (cudaStream_t)stream>>>(A);
-  } else {
-    N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(learned_step_kernel<1>), smem));
-    learned_step_kernel<1><<<grid, kStepChains * 32, smem, (cudaStream_t)stream>>>(A);
-  }
+  N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(learned_step_kernel), kStepSmem));
+  learned_step_kernel<<<grid, kStepChains * 32, kStepSmem, (cudaStream_t)stream>>>(A);
   N3_TRY(n3host::check_launch("learned_step_kernel"));
   bump_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(M->counters, 0);
   return n3host::check_launch("bump_kernel");

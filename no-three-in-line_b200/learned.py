@@ -114,7 +114,7 @@ class LearnedProposal:
         if threads_per_chain not in (0, 32, 64):
             raise ValueError("threads_per_chain must be 0 (the default), 32 or 64")
         self.bad_bias = int(bad_bias)
-        # width of the team that makes one chain's exact moves (0: the library's default)
+        # accepted for its callers; one warp makes a chain's exact moves at every width
         self.threads_per_chain = int(threads_per_chain)
         self.ch = chains
         dev = chains.device
