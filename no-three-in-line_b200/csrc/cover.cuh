@@ -87,13 +87,14 @@ __device__ __forceinline__ int cover_get(const uint32_t* __restrict__ T, int cel
   return reinterpret_cast<const uint16_t*>(T)[cell];
 }
 
-// T of the state in cs, into zeroed T.
+// The pairs of slots part, part + parts, ... with the later ones, into T of the
+// state in cs (`parts` warps build zeroed T together).
 static __device__ __noinline__ void cover_build(const uint8_t* __restrict__ cs, uint32_t* __restrict__ T, int n,
                                                 const uint16_t* __restrict__ prim4,
                                                 const uint32_t* __restrict__ recip, uint2* __restrict__ scratch,
-                                                int lane) {
+                                                int lane, int part = 0, int parts = 1) {
   const int m = 2 * n;
-  for (int i = 0; i + 1 < m; ++i) {
+  for (int i = part; i + 1 < m; i += parts) {
     const int ri = i >> 1, ci = cs[i];
     for (int k0 = (i | 1) + 1; k0 < m; k0 += 32) {  // the slots after i's row
       const int k = k0 + lane;
@@ -123,6 +124,24 @@ static __device__ __noinline__ void cover_swap(const uint8_t* __restrict__ cs, u
       cover_line(T, n, rx, cx, in ? k >> 1 : rx, in ? ck : cx, c < 2 ? -1 : 1, in, prim4, recip, scratch, lane);
     }
   }
+}
+
+// Occupancy of the grid: three words a row, bit c & 31 of word c >> 5 for column c.
+constexpr int kOccWords = 3 * kMaxN;
+
+// Points of the state on the line through (r0, c0) and (r1, c1), the cell
+// (r0, c0) left out; 0 if the two share a row or a column.
+__device__ __forceinline__ int points_on_line(const uint32_t* __restrict__ occ, int n,
+                                              const uint16_t* __restrict__ prim4, int r0, int c0, int r1, int c1) {
+  if (r0 == r1 || c0 == c1) return 0;
+  const int key = (int)(dir4(prim4, r1 * kLutW + c1, r0 * kLutW + c0) >> 2);
+  const int a = (key + kMaxN - 1) / kLutW, b = key - a * kLutW;
+  int count = 0;
+  for (int r = r0 + a, c = c0 + b; r < n && (unsigned)c < (unsigned)n; r += a, c += b)
+    count += (occ[3 * r + (c >> 5)] >> (c & 31)) & 1u;
+  for (int r = r0 - a, c = c0 - b; r >= 0 && (unsigned)c < (unsigned)n; r -= a, c -= b)
+    count += (occ[3 * r + (c >> 5)] >> (c & 31)) & 1u;
+  return count;
 }
 
 }  // namespace n3

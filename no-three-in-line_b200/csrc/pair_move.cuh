@@ -210,6 +210,42 @@ __device__ __forceinline__ bool call_slow_move(WarpState& W, const uint16_t* __r
   return true;
 }
 
+// What the histograms around the new centres u' = (r_u, c_v) and v' = (r_v, c_u)
+// tell about the swap of slots u and v in different rows and columns.
+struct PairCount {
+  int ta, tb;    // t(u'), t(v') over A
+  int j_new;     // points of A on the line (u', v')
+  int joint;     // points of A on the line (u, v)
+  bool wide;     // a counter may have wrapped: the rest is not to be used
+};
+
+// Counts them into hist (two zero histograms of Num::kWords words each) and leaves
+// the centres' directions in a and b: the caller clears those words.
+template <class Num, int NT>
+__device__ __forceinline__ PairCount count_pair(const WarpState& W, const uint16_t* __restrict__ lut4,
+                                                uint32_t* __restrict__ hist, int ru, int rv, int cu, int cv,
+                                                Directions& a, Directions& b, uint32_t& line_new) {
+  uint32_t* const h0 = hist;
+  uint32_t* const h1 = hist + Num::kWords;
+  const int kA = 2 * (ru * kLutW + cv), kB = 2 * (rv * kLutW + cu);  // u', v'
+  line_new = dir4_2(lut4, kB, kA);
+  find_centre<Num, NT>(W, lut4, h0, kA, a);
+  find_centre<Num, NT>(W, lut4, h1, kB, b);
+  // pair sums in 12 bits each, the points on the line (u, v), both included, in the top byte
+  const uint32_t part = count_centres<NT>(W, a, b) + ((uint32_t)W.on_line<NT>(ru, cu, rv - ru, cv - cu) << 24);
+  __syncwarp();
+  PairCount p;
+  p.j_new = (int)counter_of(h0, line_new);
+  const int xa = (int)counter_of(h0, Num::kCol), xb = (int)counter_of(h1, Num::kCol);
+  const uint32_t sums = __reduce_add_sync(0xffffffffu, part);
+  const int sa = (int)(sums & 0xFFFu), sb = (int)((sums >> 12) & 0xFFFu);
+  p.ta = sa - xa;
+  p.tb = sb - xb;
+  p.joint = (int)(sums >> 24) - 2;
+  p.wide = sa >= kMoveSum || sb >= kMoveSum;
+  return p;
+}
+
 // One legal move, prepared as `mv` on the current state.  lut4: Num's table; hist:
 // two histograms of Num::kWords words each, zero, left zero.  NT = ceil(m / 32).
 // accept(dE) as in slow_move.
@@ -222,27 +258,18 @@ __device__ __forceinline__ bool pair_move(WarpState& W, const uint16_t* __restri
   uint32_t* const h1 = hist + Num::kWords;
   const int u = (int)(mv.slots & 0xFFu), v = (int)((mv.slots >> 8) & 0xFFu);
   const int cu = (int)((mv.slots >> 16) & 0xFFu), cv = (int)(mv.slots >> 24);
-  const int ru = u >> 1, rv = v >> 1, dr = rv - ru, dc = cv - cu;
-  const int kA = 2 * (ru * kLutW + cv), kB = 2 * (rv * kLutW + cu);  // u', v'
-  const uint32_t line_new = dir4_2(lut4, kB, kA);
+  const int ru = u >> 1, rv = v >> 1, dc = cv - cu;
   Directions a, b;
-  find_centre<Num, NT>(W, lut4, h0, kA, a);
-  find_centre<Num, NT>(W, lut4, h1, kB, b);
-  // pair sums in 12 bits each, the points on the line (u, v), both included, in the top byte
-  const uint32_t part = count_centres<NT>(W, a, b) + ((uint32_t)W.on_line<NT>(ru, cu, dr, dc) << 24);
-  __syncwarp();
-  const int jn = (int)counter_of(h0, line_new), xa = (int)counter_of(h0, e_col), xb = (int)counter_of(h1, e_col);
-  const uint32_t sums = __reduce_add_sync(0xffffffffu, part);
-  const int sa = (int)(sums & 0xFFFu), sb = (int)((sums >> 12) & 0xFFFu), joint = (int)(sums >> 24) - 2;
-  const int dE = sa + sb - xa - xb + jn + joint - mv.bad;
+  uint32_t line_new;
+  const PairCount p = count_pair<Num, NT>(W, lut4, hist, ru, rv, cu, cv, a, b, line_new);
+  const int dE = p.ta + p.tb + p.j_new + p.joint - mv.bad;
   *dE_out = dE;
-  const bool wide = sa >= kMoveSum || sb >= kMoveSum;
-  if (wide || !accept(dE)) {  // uniform
+  if (p.wide || !accept(dE)) {  // uniform
     __syncwarp();
     clear_centre<NT>(a);
     clear_centre<NT>(b);
     __syncwarp();
-    return wide ? call_slow_move<2 * Num::kWords>(W, lut4, hist, u, v, accept, E, err, dE_out) : false;
+    return p.wide ? call_slow_move<2 * Num::kWords>(W, lut4, hist, u, v, accept, E, err, dE_out) : false;
   }
   // every other point's badness change: the points it shares a line through u' and v' with, less
   // those through u and v.  At the new centres u or v is counted too for a point of their row or
@@ -274,7 +301,7 @@ __device__ __forceinline__ bool pair_move(WarpState& W, const uint16_t* __restri
     __syncwarp();
     return call_slow_move<2 * Num::kWords>(W, lut4, hist, u, v, accept, E, err, dE_out);
   }
-  if (mv.bad != tc + td || jo != joint) err |= kErrAudit;
+  if (mv.bad != tc + td || jo != p.joint) err |= kErrAudit;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
     const int k = W.slot(t);
@@ -283,8 +310,8 @@ __device__ __forceinline__ bool pair_move(WarpState& W, const uint16_t* __restri
   W.swap_keys(u, v, dc);
   __syncwarp();
   if (W.lane == 0) {
-    W.bs[u] = sa - xa + jn;
-    W.bs[v] = sb - xb + jn;
+    W.bs[u] = p.ta + p.j_new;
+    W.bs[v] = p.tb + p.j_new;
     W.cs[u] = (uint8_t)cv;
     W.cs[v] = (uint8_t)cu;
   }
