@@ -386,20 +386,22 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
       for (int i = tid; i < kPartnerRegion; i += blockDim.x) S.T[i] = 0u;
       __syncthreads();
     }
-    bool on_grid = true;
+    bool regular = true;  // two points in every column, in cells of their own
     for (int s = tid; s < m; s += blockDim.x) {
       const int c = cols[(size_t)b * m + s];
-      on_grid = c >= 0 && c < n;
+      const bool on_grid = c >= 0 && c < n;
+      regular = regular && on_grid;
       S.cs[s] = (uint8_t)min(max(c, 0), n - 1);
       if (cover && on_grid) {
         atomicAdd(&S.columns[c], 1);
-        atomicOr(&S.occ[3 * (s >> 1) + (c >> 5)], 1u << (c & 31));
+        const uint32_t bit = 1u << (c & 31);
+        if (atomicOr(&S.occ[3 * (s >> 1) + (c >> 5)], bit) & bit) regular = false;
       }
     }
     __syncthreads();
     if (cover) {
-      for (int c = tid; c < n; c += blockDim.x) on_grid = on_grid && S.columns[c] == 2;
-      cover = __syncthreads_and(on_grid);
+      for (int c = tid; c < n; c += blockDim.x) regular = regular && S.columns[c] == 2;
+      cover = __syncthreads_and(regular);
     }
     if (cover) {
       cover_build(S.cs, S.T, n, S.prim4, S.recip, S.scratch[warp], lane, warp, kPartnerWarps);

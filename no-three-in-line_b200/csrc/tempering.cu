@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(512, 1) temper_kernel(const TemperArgs A) {
   W.bs = bs;
   for (int i = lane; i < kRegionWords; i += 32) region[i] = 0u;
   // The state; a column off the grid stops the chain (error bit 1), and columns
-  // that do not hold two points each keep it from the cover table.
+  // that do not hold two points each, or a cell that holds two, keep it from the
+  // cover table.
   bool on_grid = true, factor = true;
 #pragma unroll
   for (int t = 0; t < kSlotsPerLane; ++t) {
@@ -331,6 +332,8 @@ __global__ void __launch_bounds__(512, 1) temper_kernel(const TemperArgs A) {
       cs[s] = (uint8_t)col;
       bs[s] = ch.badness[(size_t)c * kMaxM + s];
     }
+    const int row_other = __shfl_xor_sync(0xffffffffu, W.key2[t], 1);
+    factor = factor && (row_other != W.key2[t] || s >= m);
   }
   on_grid = __all_sync(0xffffffffu, on_grid);
   if (on_grid) {  // points per column

@@ -65,3 +65,21 @@ def test_diagonals_and_uneven_columns(cuda):
     uneven[0, 1::2] = 7 + r % 11
     cols = np.concatenate((diag, uneven, diag))
     check(cols, [(b, u) for b in (0, 1, 2) for u in range(0, 2 * n, 3)] + [(1, 5), (0, 3)], cuda)
+
+
+def test_a_cell_held_twice(cuda):
+    """Two points in every column, but one cell twice: runs of a state's anchors and single ones agree."""
+    import torch
+
+    n = 40
+    r = np.arange(n)
+    cols = state.pq_to_columns(r[None].astype(np.int32), ((r + 1) % n)[None].astype(np.int32))
+    cols[0, 11], cols[0, 9] = 5, 6   # rows 5 and 4 held columns 5, 6 and 4, 5
+    cols = np.repeat(cols, 2, axis=0)
+    E, bad = gpu.score_columns_gpu(cols, badness=True)
+    runs = [(b, u) for b in (0, 1) for u in range(2 * n)]
+    single = [(b, u) for u in range(2 * n) for b in (0, 1)]
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()  # noqa: E731
+    for call in (gpu_delta.two_switch_scores, gpu_delta.transposition_scores):
+        a, b = (call(dev(cols), dev(bad), dev(E), dev(np.asarray(x, np.int32))).cpu().numpy() for x in (runs, single))
+        assert np.array_equal(a.reshape(2, 2 * n, -1), b.reshape(2 * n, 2, -1).transpose(1, 0, 2))
