@@ -7,8 +7,8 @@ through the anchor slot in the reference's enumeration order, the first
 lowest-scoring legal one kept if it improves on the state, the same
 ``evaluated`` / ``legal`` counts.  The reference builds every candidate state
 on the host (3.1 M states at n = 75 for a four-cycle scan) and rescores each in
-full on the GPU; here one kernel scores every candidate exactly from direction
-histograms of the 12 positions a slot set's candidates can take
+full on the GPU; here one kernel scores every candidate exactly from a cover
+table and direction histograms around the positions that three of its slots fix
 (libn3 ``n3_neighborhood_scan``), and the host only decodes the winner and
 checks it with the two independent device counts.  ``batch_size`` is accepted
 for the reference's signature; the scan needs no batching.
@@ -18,13 +18,16 @@ from __future__ import annotations
 import ctypes
 import time
 from dataclasses import dataclass
-from itertools import combinations, permutations
+from itertools import permutations
+from math import comb
 
 import numpy as np
 
 from . import _lib
 from .accelerated import score_and_badness
 from .state import PairPermutations, points_to_permutations
+
+_BASE = 1 << 30  # above any score, so that no candidate's goes below 0
 
 _lib.register("n3_neighborhood_scan", [_lib._P, _lib._P, _lib._I, _lib._I, _lib._I64, _lib._P, _lib._P, _lib._P])
 
@@ -54,7 +57,7 @@ class DoubleSwitchResult:
 def _values_state(values: np.ndarray) -> PairPermutations:
     """gpu_neighborhood.py:34-37."""
     n = values.shape[0]
-    points = [(row, int(values[row, layer])) for row in range(n) for layer in range(2)]
+    points = [(row, column) for row, pair in enumerate(values.tolist()) for column in pair]
     return points_to_permutations(points, n)
 
 
@@ -73,22 +76,32 @@ def _scan(state: PairPermutations, anchor_index: int):
         raise ValueError(f"n={n} outside [5, {_lib.MAX_N}]")
     t = _lib.torch()
     device = _lib.require_device()
-    p = np.asarray(state.P, dtype=np.int32)
-    q = np.asarray(state.Q, dtype=np.int32)
-    base_score = int(score_and_badness(p, q)[0])
-    dp, dq = t.from_numpy(p).to(device), t.from_numpy(q).to(device)
-    out = t.empty(4, dtype=t.int64, device=device)
-    _lib.call("n3_neighborhood_scan", _lib.ptr(dp), _lib.ptr(dq), n, int(anchor_index), base_score, _lib.ptr(out),
-              _lib.ptr(out) + 16, _lib.stream_ptr())
-    best4, best2, legal4, legal2 = (int(x) for x in out.cpu().numpy().view(np.uint64))
-    return n, p, q, base_score, (best4, legal4), (best2, legal2)
+    pq = np.asarray((state.P, state.Q), dtype=np.int32)
+    on_device = t.from_numpy(pq).to(device)
+    dp = _lib.ptr(on_device)
+    dq, stream = dp + 4 * n, _lib.stream_ptr()
+    # The scan runs with _BASE in place of the state's score, so that the score
+    # follows it on the stream and both come back in one copy.
+    out = t.empty(5, dtype=t.int64, device=device)
+    dst = _lib.ptr(out)
+    _lib.call("n3_neighborhood_scan", dp, dq, n, int(anchor_index), _BASE, dst, dst + 16, stream)
+    _lib.call("n3_score_population", dp, dq, 1, n, dst + 32, None, stream)
+    best4, best2, legal4, legal2, score = (int(x) for x in out.cpu().numpy().view(np.uint64))
+    base_score = score & 0xFFFFFFFF
+    rebase = (base_score - _BASE) << 32
+    return n, pq[0], pq[1], base_score, (best4 + rebase, legal4), (best2 + rebase, legal2)
 
 
 def _slot_set(n: int, anchor: int, combo_layers: int):
     """Decode (row triple, layer choice) number k of gpu_neighborhood.py:108-110."""
-    others = [row for row in range(n) if row != anchor // 2]
-    rows = list(combinations(others, 3))[combo_layers // 8]
-    layers = combo_layers % 8
+    rank, layers = divmod(combo_layers, 8)
+    rows, low = [], 0
+    for left in (2, 1, 0):  # rows still to choose after this one
+        while (later := comb(n - 2 - low, left)) <= rank:
+            rank -= later
+            low += 1
+        rows.append(low if low < anchor // 2 else low + 1)
+        low += 1
     return tuple(2 * r + ((layers >> (2 - i)) & 1) for i, r in enumerate(rows))
 
 
@@ -105,7 +118,8 @@ def _verified(values: np.ndarray, score: int, what: str) -> None:
     from .gpu import score_checked_gpu
     from .state import pq_to_columns
 
-    checked = score_checked_gpu(pq_to_columns(values[None, :, 0], values[None, :, 1]), raise_on_mismatch=False)
+    checked = score_checked_gpu(pq_to_columns(values[None, :, 0], values[None, :, 1]), raise_on_mismatch=False,
+                                badness=False)
     exact = int(checked.scores[0])
     if exact != score or checked.mismatches:
         raise AssertionError(f"GPU {what} score {score} != full score {exact}")

@@ -139,29 +139,22 @@ def points_to_permutations(points: list[Point], n: int) -> PairPermutations:
             raise ValueError(f"point {(r, c)} outside grid")
         adjacency[r].append(c)
         column_degree[c] += 1
-    if any(len(a) != 2 for a in adjacency) or any(d != 2 for d in column_degree):
+    if set(map(len, adjacency)) - {2} or column_degree.count(2) != n:
         raise ValueError("points are not a row/column 2-factor")
-    for a in adjacency:
-        a.sort()
+    # Rows and columns form cycles, so an augmenting path never branches: it goes
+    # from column to owner to the owner's other column, and ends at a free one.
+    both = [int(a) + int(b) for a, b in adjacency]
     owner = [-1] * n  # column -> row matched through P
-
-    def augment(row: int, seen: list[bool]) -> bool:
-        for col in adjacency[row]:
-            if seen[col]:
-                continue
-            seen[col] = True
-            if owner[col] == -1 or augment(owner[col], seen):
-                owner[col] = row
-                return True
-        return False
-
-    for r in range(n):
-        if not augment(r, [False] * n):
-            raise ValueError("2-factor unexpectedly has no perfect matching")
+    for r, (a, b) in enumerate(adjacency):
+        row, col = r, min(a, b)
+        while (previous := owner[col]) >= 0:
+            owner[col] = row
+            row, col = previous, both[previous] - col
+        owner[col] = row
     p = [-1] * n
     for col, r in enumerate(owner):
         p[r] = col
-    q = [next(c for c in adjacency[r] if c != p[r]) for r in range(n)]
+    q = [both[r] - p[r] for r in range(n)]
     state = PairPermutations(tuple(p), tuple(q))
     state.validate()
     return state
