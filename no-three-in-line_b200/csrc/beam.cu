@@ -15,10 +15,9 @@
 // every child's score each generation.  Here the selection is one CTA: a
 // one-pass histogram (or radix) select of the elite_size-th smallest score, a
 // bitonic sort of the scores below it, ordered compactions by per-warp counts,
-// the MT19937 state blocks twisted by the whole CTA, the shuffle's draws
-// (exactly CPython's: by the whole CTA for the wide draw widths, by one warp
-// for the last ones), and the first elite_size shuffled positions traced back
-// through the draws.
+// the MT19937 state blocks twisted by the whole CTA, the shuffle's draws (exactly
+// CPython's), and the first elite_size shuffled positions traced back through
+// the draws.
 #include <stdint.h>
 
 #include <climits>
@@ -61,20 +60,39 @@ struct MutArgs {
 };
 
 // One thread per child, the reference's draws in the reference's order.  The
-// CTA's 64 children live in shared memory (slot layout s = 2 * row + layer)
-// from the parent copy to one coalesced write of their rows.  When the parents'
-// badness prefix sums fit in shared memory (prefix_cap parents), the CTA builds
-// them once and the roulette draw becomes a binary search: with no negative
-// badness, the linear scan `t -= bad[u]` stops at the first u whose inclusive
-// prefix exceeds t, which the search finds.  A negative badness anywhere, or
-// one large enough for a sum to overflow (neither is a state's badness), sends
-// the CTA back to the linear scan, so every draw and result stays the
-// reference's for any input.  The parent's total badness is taken once per
-// child instead of once per attempt (it does not change).
-constexpr int kMutThreads = 64;
+// CTA's children live in shared memory in 16 bits (slot layout s = 2 * row +
+// layer) from the parent copy to one coalesced write of their rows.  When the
+// parents' badness prefix sums fit in shared memory (prefix_cap parents), the CTA
+// builds them once, a warp per parent, and the roulette draw becomes a binary
+// search: with no negative badness, the linear scan `t -= bad[u]` stops at the
+// first u whose inclusive prefix exceeds t, which the search finds.  A negative
+// badness anywhere, or one large enough for a sum to overflow (neither is a
+// state's badness), sends the CTA back to the linear scan, so every draw and
+// result stays the reference's for any input.  The parent's total badness is
+// taken once per child instead of once per attempt (it does not change), and its
+// draws' remainders by a reciprocal.
+//
+// A child is one thread's serial chain (about five draws a swap), so what counts
+// besides is the staging, which every CTA repeats: with as many threads as spread
+// the children over the SMs once (64 .. 256), 32,768 children of 64 parents at
+// n = 75 take 31 us, 71 us in CTAs of 64.
+constexpr int kMutThreads = 256;  // at most
 constexpr size_t kMutPrefixMaxBytes = 96 * 1024;
 
-constexpr size_t kMutSmemMax = sizeof(int32_t) * kMutThreads * kMaxM + kMutPrefixMaxBytes;
+constexpr size_t kMutSmemMax = sizeof(int16_t) * kMutThreads * kMaxM + kMutPrefixMaxBytes;
+static_assert(kMutSmemMax <= 227 * 1024 - 2048, "mutate_kernel shared memory");
+
+// x % d by a reciprocal: the quotient's estimate is at most two short.
+struct Remainder {
+  uint64_t d, inverse;
+  __device__ explicit Remainder(uint64_t divisor) : d(divisor), inverse(~0ull / divisor) {}
+  __device__ __forceinline__ uint64_t of(uint64_t x) const {
+    uint64_t r = x - __umul64hi(x, inverse) * d;
+    if (r >= d) r -= d;
+    if (r >= d) r -= d;
+    return r;
+  }
+};
 
 __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -87,10 +105,11 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
     active = min(A.max_strength, 2 + (A.generation - (int)A.status[4]) / 10);
   }
   const int n = A.n, m = 2 * n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int child0 = blockIdx.x * kMutThreads, child = child0 + tid;
-  const int nc = min(kMutThreads, A.population - child0);
-  int32_t* rows = reinterpret_cast<int32_t*>(smem);  // [kMutThreads][m]
-  int32_t* prefix = rows + kMutThreads * m;          // [prefix_cap][m] inclusive prefix sums
+  const int threads = blockDim.x, warps = threads / 32;
+  const int child0 = blockIdx.x * threads, child = child0 + tid;
+  const int nc = min(threads, A.population - child0);
+  int32_t* prefix = reinterpret_cast<int32_t*>(smem);                       // [prefix_cap][m] inclusive prefix sums
+  short2* rows = reinterpret_cast<short2*>(prefix + (size_t)A.prefix_cap * m);  // [threads][n] both layers of a row
   uint64_t rng = A.seed ^ (0x9e3779b97f4a7c15ULL * (uint64_t)(child + 1)) ^
                  (0xbf58476d1ce4e5b9ULL * (uint64_t)(A.generation + 1));
   int parent = child;
@@ -100,44 +119,53 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
     parent = (int)(xs64(rng) % (uint64_t)pool);
   }
   s_parent[tid] = parent;
+  __syncthreads();
+#pragma unroll 4
+  for (int c = warp; c < nc; c += warps) {  // the parents' rows into the children's, a warp per child
+    const int32_t* src_p = A.pp + (size_t)s_parent[c] * n;
+    const int32_t* src_q = A.pq + (size_t)s_parent[c] * n;
+#pragma unroll
+    for (int k = 0; k < (kMaxN + 31) / 32; ++k) {
+      const int r = lane + 32 * k;
+      if (r < n) rows[c * n + r] = make_short2((short)src_p[r], (short)src_q[r]);
+    }
+  }
   bool use_prefix = parent_count <= A.prefix_cap;  // uniform
   if (use_prefix) {
-    const int count = parent_count * m;
-#pragma unroll 8
-    for (int i = tid; i < count; i += kMutThreads) prefix[i] = A.pbad[i];  // coalesced, loads in flight together
-    __syncthreads();
     bool negative = false;
-    for (int p = tid; p < parent_count; p += kMutThreads) {  // in place, a thread per parent
-      int32_t* row = prefix + p * m;
-      int acc = 0;
-#pragma unroll 10
-      for (int e = 0; e < m; ++e) {
-        const int b = row[e];
-        negative |= b < 0 || b > 0x7fffffff / kMaxM;  // keeps every prefix sum below 2^31
-        row[e] = acc += b;
+#pragma unroll 4
+    for (int p = warp; p < parent_count; p += warps) {
+      int acc[kMaxM / 32 + 1];
+#pragma unroll
+      for (int k = 0; k < kMaxM / 32 + 1; ++k) {
+        const int e = 32 * k + lane;
+        acc[k] = e < m ? A.pbad[p * m + e] : 0;
+        negative |= acc[k] < 0 || acc[k] > 0x7fffffff / kMaxM;  // keeps every prefix sum below 2^31
+      }
+      int before = 0;
+#pragma unroll
+      for (int k = 0; k < kMaxM / 32 + 1; ++k) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, acc[k], o);
+          if (lane >= o) acc[k] = (int)((unsigned)acc[k] + (unsigned)y);
+        }
+        const int e = 32 * k + lane;
+        if (e < m) prefix[p * m + e] = (int)((unsigned)acc[k] + (unsigned)before);
+        before = (int)((unsigned)before + (unsigned)__shfl_sync(0xffffffffu, acc[k], 31));
       }
     }
     use_prefix = !__syncthreads_or(negative);
   } else {
     __syncthreads();
   }
-  for (int c = warp; c < nc; c += kMutThreads / 32) {  // the parents' rows into the children's, a warp per child
-    const int32_t* src_p = A.pp + (size_t)s_parent[c] * n;
-    const int32_t* src_q = A.pq + (size_t)s_parent[c] * n;
-    int32_t* dst = rows + c * m;
-    for (int r = lane; r < n; r += 32) {
-      dst[2 * r] = src_p[r];
-      dst[2 * r + 1] = src_q[r];
-    }
-  }
-  __syncthreads();
   const bool record = A.child_moves != nullptr;
   if (child < A.population) {
     if (record) A.child_parent[child] = parent;
     if (child < parent_count) {
       if (record) A.child_nmoves[child] = 0;
     } else {
-      int32_t* cs = rows + tid * m;
+      int16_t* cs = reinterpret_cast<int16_t*>(rows + tid * n);
       const int32_t* bad = A.pbad + (size_t)parent * m;
       const int32_t* pre = prefix + parent * m;
       int total = 0;
@@ -146,6 +174,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
       } else {
         for (int e = 0; e < m; ++e) total += bad[e];
       }
+      const Remainder by_total((uint64_t)(int64_t)(total ? total : 1)), by_slots((uint64_t)m);
       int strength, nmoves = 0;
       if ((xs64(rng) & 31ULL) == 0ULL)
         strength = 1 + (int)(xs64(rng) % (uint64_t)A.max_strength);
@@ -156,7 +185,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
           int u;
           if ((int)(xs64(rng) % 100ULL) < A.bad_bias) {
             if (total) {
-              const int t = (int)(xs64(rng) % (uint64_t)total);
+              const int t = (int)by_total.of(xs64(rng));
               if (use_prefix) {  // first u with prefix[u] > t; prefix[m - 1] = total > t
                 int lo = 0, hi = m - 1;
                 while (lo < hi) {
@@ -173,18 +202,18 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
                 }
               }
             } else {
-              u = (int)(xs64(rng) % (uint64_t)m);
+              u = (int)by_slots.of(xs64(rng));
             }
           } else {
-            u = (int)(xs64(rng) % (uint64_t)m);
+            u = (int)by_slots.of(xs64(rng));
           }
-          const int v = (int)(xs64(rng) % (uint64_t)m);
+          const int v = (int)by_slots.of(xs64(rng));
           if ((u >> 1) == (v >> 1)) continue;
           const int cu = cs[u], cv = cs[v];
           if (cu == cv) continue;
           if (cv == cs[u ^ 1] || cu == cs[v ^ 1]) continue;  // the other point of each row
-          cs[u] = cv;
-          cs[v] = cu;
+          cs[u] = (int16_t)cv;
+          cs[v] = (int16_t)cu;
           if (record && nmoves < A.moves_cap) A.child_moves[(size_t)child * A.moves_cap + nmoves] = u | (v << 8);
           ++nmoves;
           break;
@@ -194,13 +223,13 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
     }
   }
   __syncthreads();
-  for (int c = warp; c < nc; c += kMutThreads / 32) {  // coalesced rows, a warp per child
-    const int32_t* src = rows + c * m;
+  for (int c = warp; c < nc; c += warps) {  // coalesced rows, a warp per child
     int32_t* dst_p = A.cp + (size_t)(child0 + c) * n;
     int32_t* dst_q = A.cq + (size_t)(child0 + c) * n;
     for (int r = lane; r < n; r += 32) {
-      dst_p[r] = src[2 * r];
-      dst_q[r] = src[2 * r + 1];
+      const short2 both = rows[c * n + r];
+      dst_p[r] = both.x;
+      dst_q[r] = both.y;
     }
   }
 }
@@ -278,33 +307,39 @@ __global__ void __launch_bounds__(kDeltaWarps * 32, 1) child_delta_kernel(const 
 }
 
 
-__global__ void py_seed_kernel(uint32_t* state, uint64_t seed) {
-  uint32_t* mt = state;
-  const uint32_t key[2] = {(uint32_t)seed, (uint32_t)(seed >> 32)};
-  const int len = (seed >> 32) ? 2 : 1;
-  mt[0] = 19650218u;
-  for (int i = 1; i < kMT; ++i) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
-  int i = 1, j = 0;
-  for (int k = kMT > len ? kMT : len; k; --k) {
-    mt[i] = (mt[i] ^ ((mt[i - 1] ^ (mt[i - 1] >> 30)) * 1664525u)) + key[j] + (uint32_t)j;
-    ++i;
-    ++j;
-    if (i >= kMT) {
-      mt[0] = mt[kMT - 1];
-      i = 1;
+// One thread seeds (each word follows from the one before) in shared memory.
+__global__ void __launch_bounds__(32) py_seed_kernel(uint32_t* state, uint64_t seed) {
+  __shared__ uint32_t mt[kMT];
+  if (threadIdx.x == 0) {
+    const uint32_t key[2] = {(uint32_t)seed, (uint32_t)(seed >> 32)};
+    const int len = (seed >> 32) ? 2 : 1;
+    uint32_t last = mt[0] = 19650218u;
+    for (int i = 1; i < kMT; ++i) mt[i] = last = 1812433253u * (last ^ (last >> 30)) + (uint32_t)i;
+    int i = 1, j = 0;
+    last = mt[0];
+    for (int k = kMT > len ? kMT : len; k; --k) {
+      mt[i] = last = (mt[i] ^ ((last ^ (last >> 30)) * 1664525u)) + key[j] + (uint32_t)j;
+      ++i;
+      ++j;
+      if (i >= kMT) {
+        mt[0] = last;
+        i = 1;
+      }
+      if (j >= len) j = 0;
     }
-    if (j >= len) j = 0;
-  }
-  for (int k = kMT - 1; k; --k) {
-    mt[i] = (mt[i] ^ ((mt[i - 1] ^ (mt[i - 1] >> 30)) * 1566083941u)) - (uint32_t)i;
-    ++i;
-    if (i >= kMT) {
-      mt[0] = mt[kMT - 1];
-      i = 1;
+    for (int k = kMT - 1; k; --k) {
+      mt[i] = last = (mt[i] ^ ((last ^ (last >> 30)) * 1566083941u)) - (uint32_t)i;
+      ++i;
+      if (i >= kMT) {
+        mt[0] = last;
+        i = 1;
+      }
     }
+    mt[0] = 0x80000000u;
   }
-  mt[0] = 0x80000000u;
-  state[kMT] = kMT;  // position: the first draw twists
+  __syncwarp();
+  for (int i = threadIdx.x; i < kMT; i += 32) state[i] = mt[i];
+  if (threadIdx.x == 0) state[kMT] = kMT;  // position: the first draw twists
 }
 
 __global__ void py_shuffle_kernel(uint32_t* state, int32_t* values, int count) {
@@ -321,67 +356,29 @@ __global__ void py_shuffle_kernel(uint32_t* state, int32_t* values, int count) {
   for (int i = threadIdx.x; i < kMT; i += blockDim.x) state[i] = mt[i];
 }
 
-// The state twist by a whole CTA, out of place: dst = twist(src).  Word k of the
+// The state twist by part of a CTA, out of place: dst = twist(src).  Word k of the
 // sequential in-place update reads the old words k, k + 1 and k + 397 (k < 227)
 // or the new word k - 227 (k >= 227; for k = 623 also the new word 0), so three
-// phases of at most 227 words each reproduce it.  Every thread calls it.
+// phases of at most 227 words each reproduce it.
 __device__ __forceinline__ uint32_t mt_mix(uint32_t hi_word, uint32_t lo_word, uint32_t far) {
   const uint32_t y = (hi_word & 0x80000000u) | (lo_word & 0x7fffffffu);
   return far ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
 }
 
-__device__ void mt_twist_cta(const uint32_t* src, uint32_t* dst) {
-  const int t = threadIdx.x;
+// Eight warps do it, with barriers of their own; the callers' __syncthreads follows.
+constexpr int kTwistThreads = 256;
+__device__ __forceinline__ void twist_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kTwistThreads) : "memory"); }
+__device__ void mt_twist(const uint32_t* src, uint32_t* dst) {
+  const int t = threadIdx.x;  // < kTwistThreads
   if (t < 227) dst[t] = mt_mix(src[t], src[t + 1], src[t + 397]);
-  __syncthreads();
+  twist_barrier();
   if (t < 227) dst[227 + t] = mt_mix(src[227 + t], src[228 + t], dst[t]);
-  __syncthreads();
+  twist_barrier();
   if (t < 170) {
     const int k = 454 + t;
     dst[k] = mt_mix(src[k], k == kMT - 1 ? dst[0] : src[k + 1], dst[k - 227]);
   }
-  __syncthreads();
-}
-
-// The shuffle's draws by one warp from the tempered outputs out[0, avail)
-// (consecutive blocks of the stream; out holds 32 more words, read and
-// ignored), starting at output pos, for steps i, i - 1, ... >= 1: the j of
-// step s goes to jstep[s] and no swap is made.  A round takes the next 32
-// words: word l serves step i - A_l (A_l: accepted words before it), so with
-// bounds A_lo <= A_l <= A_hi it is accepted for sure when r <= i - A_hi and
-// rejected for sure when r > i - A_lo.  Ballots of the decided words give the
-// bounds (A_lo: accepted below the lane; A_hi: the lane less the rejected
-// below it), and the lowest undecided lane always has exact bounds, so a few
-// iterations decide all 32.  The round keeps the words up to the m-th
-// acceptance (m: the steps left in this draw width, at most 32).  Stops when
-// the steps end or the outputs do; i and pos advance.
-__device__ void shuffle_draws_warp(const uint32_t* out, int avail, int& pos, int& i, uint16_t* jstep, int lane) {
-  const unsigned below = (1u << lane) - 1u;
-  while (i >= 1 && pos < avail) {
-    const int shift = __clz((uint32_t)i + 1u);
-    const int lo = max(1, (int)(0x80000000u >> shift) - 1);  // the width's last step
-    const int m = min(32, i - lo + 1);
-    const int draws = min(32, avail - pos);
-    const int r = (int)(out[pos + lane] >> shift);
-    unsigned accm = 0u, rejm = draws < 32 ? ~0u << draws : 0u;  // lanes past the outputs: decided, unused
-    for (;;) {
-      const bool und = !(((accm | rejm) >> lane) & 1u);
-      const int a_lo = __popc(accm & below), a_hi = lane - __popc(rejm & below);
-      accm |= __ballot_sync(0xffffffffu, und && r <= i - a_hi);
-      rejm |= __ballot_sync(0xffffffffu, und && r > i - a_lo);
-      if ((accm | rejm) == 0xffffffffu) break;  // uniform
-    }
-    int used = draws;
-    if (__popc(accm) >= m) {  // the m-th acceptance ends this width
-      const int z = __ffs(__ballot_sync(0xffffffffu, ((accm >> lane) & 1u) &&
-                                                      __popc(accm & ((2u << lane) - 1u)) == m)) - 1;
-      used = z + 1;
-    }
-    const unsigned take = used < 32 ? accm & ((1u << used) - 1u) : accm;
-    if ((take >> lane) & 1u) jstep[i - __popc(take & below)] = (uint16_t)r;
-    i -= __popc(take);
-    pos += used;
-  }
+  twist_barrier();
 }
 
 // Exclusive scan over the CTA (thread order) of a 32-bit value, with the total.
@@ -412,112 +409,105 @@ __device__ __forceinline__ uint32_t cta_exscan32(uint32_t v, uint32_t* wsum, uin
   return (warp ? wsum[warp - 1] : 0u) + x - v;
 }
 
-// The shuffle's draws for the steps i, i - 1, ... that share i's draw width
-// (down to 2^(k-1) - 1, k = bit_length(i + 1)), resolved by the whole CTA from
-// the tempered outputs out[pos, avail), the same as shuffle_draws_warp: step s
-// takes words in order until one has r = word >> (32 - k) <= s, and j = r.
-// Word w (w = 0, 1, ... from pos) serves step i - A_w, A_w the number of
-// accepted words before it, so it is accepted for sure when r <= i - A_hi and
-// rejected for sure when r > i - A_lo, for any bounds A_lo <= A_w <= A_hi.
-// Each pass bounds A_w by prefix counts over the CTA of the words decided so
-// far (A_lo: accepted before w; A_hi: w less the rejected before w) and
-// decides what the bounds allow; the first undecided word always has exact
-// bounds, so a pass never ends without progress.  Thread t holds words
-// kDrawPer t .. kDrawPer t + kDrawPer - 1.  After at most kDrawPasses passes
-// the call stops at the first undecided word, or after the acceptance of the
-// width's last step, or at the end of the outputs; i and pos advance.  All
-// threads call it with the same i and pos (>= 1 step, >= 1 word left).  A
-// call takes at most 2 need + 64 words (a draw is accepted with probability
-// above 1/2): more words per call mean more passes, as a word's bounds widen
-// with the number of words before it.
-constexpr int kDrawPer = 5;       // 5120 words per call: one batch of kSelBatch blocks
-constexpr int kDrawPasses = 48;
-__device__ void shuffle_draws_cta(const uint32_t* out, int avail, int& pos, int& i, uint16_t* jstep,
-                                  uint32_t* wsum /* [2][32] */, int* cut /* [3] */) {
-  const int tid = threadIdx.x;
-  const int shift = __clz((uint32_t)i + 1u);
-  const int lo = max(1, (int)(0x80000000u >> shift) - 1);  // the width's last step
-  const int need = i - lo + 1;
-  const int nw = min(min(avail - pos, (int)blockDim.x * kDrawPer), 2 * need + 64);
-  const int w0 = tid * kDrawPer;
-  uint32_t r[kDrawPer];
-  uint32_t st = 0u;  // 2 bits per word: 0 undecided, 1 accepted, 2 rejected, 3 absent
+// The shuffle's draws for the steps i, i - 1, ..., 1 from the tempered outputs
+// out[pos, avail) (consecutive blocks of the stream): step s takes words in order
+// until one has r = word >> (32 - bit_length(s + 1)) <= s, and j = r goes to
+// jstep[s].  No swap is made.  Word w (w = 0, 1, ... from pos) serves step
+// i - A_w, A_w the number of accepted words before it, so the accepted words are
+// the one fixed point of "accept w if it fits step i - A_w": word 0's answer is
+// right in any iteration, word w's in the one after those before it.  Iterating
+// over all words at once is much faster than that bound, as a wrong A_w misjudges
+// only words whose r lies between the two steps.  It starts from the expected
+// number of acceptances (below), and 5000 words take 2 to 8 iterations while
+// steps are many and 10 to 20 at the end, all widths together.
+//
+// Warp v holds the words 160 v .. 160 v + 159, lane by lane; ballots give A_w
+// inside the warp, one barrier per iteration the counts of the warps before.  A warp
+// whose count before and whose answers did not change keeps them.  Every thread calls it with the same i >= 1 and
+// pos < avail; i and pos advance.  tot: 64 words, cut: one, of shared memory.
+// blockDim.x == 1024.
+//
+// A window of 10,000 steps: its draws with the twists take 26 us, 63 us by a call
+// per draw width with scans of thread counts and the last 2048 steps by one warp.
+constexpr int kDrawPer = 5;  // 5120 words per call: one batch of kSelBatch blocks
+// Whether step >= 1 takes the word: word >> clz(step + 1) <= step, that is
+// word < (step + 1) << clz(step + 1), which a float's mantissa holds (step < 2^23; a
+// conversion of its own, as clz and int-to-float run at a quarter of the rate or less).
+__device__ __forceinline__ bool draw_fits(uint32_t word, int step) {
+  const float x = __uint_as_float(0x4B000000u | (uint32_t)(step + 1)) - 8388608.0f;
+  return step >= 1 && word < (__float_as_uint(x) << 8 | 0x80000000u);
+}
+__device__ void shuffle_draws_cta(const uint32_t* out, int avail, int& pos, int& i, uint16_t* jstep, uint32_t* tot,
+                                  int* cut) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int nw = min(min(avail - pos, (int)blockDim.x * kDrawPer), 2 * i + 64);
+  const int w0 = warp * 32 * kDrawPer + lane;
+  // Steps of bit length k (2^(k - 1) - 1 <= s) accept with probability (s + 1) / 2^k,
+  // so s + 1 falls by 1 / 2^k of itself per word: from 2^k to 2^(k - 1) in
+  // 2^k ln 2 words, and with l ln 2 words left at bit length k,
+  // s + 1 = 2^(k - 2 + l / 2^k).
+  const int bits = 32 - __clz((uint32_t)i + 1u);
+  const float size = (float)(1u << bits);
+  const float left = size * (2.0f + __log2f((float)(i + 1) / size));  // l at word 0
+  uint32_t word[kDrawPer], accepted[kDrawPer];
+  int each[kDrawPer], count = 0;
 #pragma unroll
   for (int e = 0; e < kDrawPer; ++e) {
-    const int w = w0 + e;
-    r[e] = w < nw ? out[pos + w] >> shift : 0u;
-    if (w >= nw) st |= 3u << (2 * e);
+    const int w = w0 + 32 * e;
+    const bool in = w < nw;
+    word[e] = in ? out[pos + w] : ~0u;  // a word that never fits
+    const float l = left - (float)w * 1.442695f;
+    int step = 0;
+    if (l >= 1.0f) {  // k from the exponent, l / 2^k from the mantissa
+      const uint32_t l_bits = __float_as_uint(l);
+      const float quarter = __uint_as_float((l_bits & 0x7F800000u) - (2u << 23));  // 2^(k - 2)
+      const float ratio = __uint_as_float((l_bits & 0x007FFFFFu) | 0x3F800000u);
+      step = min(i, (int)(quarter * exp2f(ratio)) - 1);
+    }
+    accepted[e] = __ballot_sync(0xffffffffu, draw_fits(word[e], step));
+    count += each[e] = __popc(accepted[e]);
   }
-  // scanned counts: accepted | rejected << 16 (at most 5120 each); undecided = words - both
-  uint32_t before = 0u, total = 0u;
-  int la = 0, lu = 0;
-  for (int pass = 0; pass < kDrawPasses; ++pass) {
-    int a = (int)(before & 0xFFFFu), rj = (int)(before >> 16);
-    la = 0;
-    lu = 0;
-    int lr = 0;
+  int before = -1, all, changed = 1;
+  for (int it = 0;; it ^= 32) {
+    if (lane == 0) tot[it + warp] = (uint32_t)count;
+    const int any = __syncthreads_or(changed);
+    const uint32_t c = tot[it + lane];
+    if (!any) {
+      all = (int)__reduce_add_sync(0xffffffffu, c);
+      break;
+    }
+    const int now_before = (int)__reduce_add_sync(0xffffffffu, lane < warp ? c : 0u);
+    const bool settled = !changed && now_before == before;  // uniform in the warp
+    before = now_before;
+    changed = 0;
+    if (settled) continue;
+    // the counts of the previous answers: no word waits for another
+    int first = i - before;
+    count = 0;
 #pragma unroll
     for (int e = 0; e < kDrawPer; ++e) {
-      uint32_t d = (st >> (2 * e)) & 3u;
-      if (d == 0u) {
-        const int w = w0 + e;
-        if ((int)r[e] <= i - (w - rj)) d = 1u;
-        else if ((int)r[e] > i - a) d = 2u;
-        st |= d << (2 * e);
-      }
-      if (d == 1u) { ++a; ++la; }
-      else if (d == 2u) { ++rj; ++lr; }
-      else if (d == 0u) ++lu;
-    }
-    before = cta_exscan32((uint32_t)la | ((uint32_t)lr << 16), wsum + 32 * (pass & 1), total);
-    if ((int)(total & 0xFFFFu) + (int)(total >> 16) == nw) break;  // uniform: every word decided
-  }
-  // `before` counts exactly for the words before the first undecided one, F.
-  if (tid == 0) {
-    cut[0] = nw;       // F
-    cut[1] = INT_MAX;  // the word after the need-th acceptance
-  }
-  __syncthreads();
-  const int a0 = (int)(before & 0xFFFFu);
-  // no undecided word before this thread's (words before it: min(w0, nw))
-  const bool clean = a0 + (int)(before >> 16) == min(w0, nw);
-  if (clean && lu > 0) {  // this thread holds F
-    int acc = a0;
-    for (int e = 0; e < kDrawPer; ++e) {
-      const uint32_t d = (st >> (2 * e)) & 3u;
-      if (d == 0u) {
-        cut[0] = w0 + e;
-        cut[2] = acc;  // acceptances before F
-        break;
-      }
-      acc += d == 1u;
+      const int step = first - __popc(accepted[e] & below);
+      const unsigned now = __ballot_sync(0xffffffffu, draw_fits(word[e], step));
+      first -= each[e];
+      changed |= now != accepted[e];
+      accepted[e] = now;
+      count += each[e] = __popc(now);
     }
   }
-  if (a0 < need && a0 + la >= need) {  // this thread holds the need-th acceptance (exact if before F)
-    int acc = a0;
-    for (int e = 0; e < kDrawPer; ++e) {
-      if (((st >> (2 * e)) & 3u) == 1u && ++acc == need) {
-        cut[1] = w0 + e + 1;
-        break;
-      }
-    }
-  }
-  __syncthreads();
-  const int F = cut[0], cA = cut[1];
-  const int used = min(F, cA);
-  const int accepted = cA <= F ? need : (F == nw ? (int)(total & 0xFFFFu) : cut[2]);
-  {
-    int acc = a0;
+  // the words up to the last step's, or all
 #pragma unroll
-    for (int e = 0; e < kDrawPer; ++e) {
-      if (((st >> (2 * e)) & 3u) == 1u) {
-        if (w0 + e < used) jstep[i - acc] = (uint16_t)r[e];
-        ++acc;
-      }
+  for (int e = 0; e < kDrawPer; ++e) {
+    if ((accepted[e] >> lane) & 1u) {
+      const int step = i - (before + __popc(accepted[e] & below));
+      jstep[step] = (uint16_t)(word[e] >> __clz((uint32_t)step + 1u));
+      if (step == 1) *cut = w0 + 32 * e + 1;
     }
+    before += each[e];
   }
-  i -= accepted;
-  pos += used;
+  __syncthreads();
+  pos += all == i ? *cut : nw;
+  i -= all;
 }
 
 // --------------------------------------------------------------------------
@@ -527,13 +517,12 @@ constexpr int kSelThreads = 1024;
 constexpr int kMaxPopulation = 65536;
 constexpr int kMaxElite = 2048;
 constexpr int kSelBatch = 8;  // MT state blocks generated per batch for the shuffle's draws
-constexpr int kCtaDrawMin = 2048;  // steps from which the CTA resolves the draws (below: one warp)
 constexpr int kSelHistBins = 4096;  // one-pass selection when every score is below this
 static_assert(kSelBatch * kMT <= kSelThreads * kDrawPer, "one resolver call covers a batch");
 static_assert(kSelHistBins <= kSelBatch * kMT && kSelHistBins % 1024 == 0, "histogram in the MT words' space");
 
 constexpr int kSelWarps = kSelThreads / 32;
-static_assert(kSelWarps == 32, "the per-warp offsets are scanned by one warp, one lane per warp");
+static_assert(kSelWarps == 32, "a warp's lanes hold the counts of all warps");
 
 struct SelArgs {
   const int32_t* scores;  // [population]
@@ -546,15 +535,14 @@ struct SelArgs {
 // The draws of random.shuffle over `count` items (steps s = count - 1 .. 1,
 // j_s = _randbelow(s + 1)) into jstep[s], from the state in shared memory (mt,
 // the current block; idx the position in it, 624 when it is used up), with
-// no swap made.  The CTA twists and tempers the state blocks kSelBatch at a
-// time (words: kSelBatch blocks; out: their outputs and 32 words of padding);
-// the CTA resolves the draws while many steps are left (shuffle_draws_cta) and
-// warp 0 the last ones (shuffle_draws_warp).  On return mt and idx are the
-// state CPython leaves: the block of the last draw and the position after it.
-// Every thread calls it; idx is uniform.
+// no swap made.  The CTA twists and tempers the state blocks up to kSelBatch
+// at a time (words: kSelBatch blocks; out: their outputs) and resolves the draws
+// (shuffle_draws_cta).  On return mt and idx are the state CPython leaves: the
+// block of the last draw and the position after it.  Every thread calls it; idx
+// is uniform.
 __device__ void shuffle_steps_cta(uint32_t* mt, int& idx, int count, uint16_t* jstep, uint32_t* words, uint32_t* out,
-                                  uint32_t* wsum, int* cut, int* s_misc) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                  uint32_t* tot, int* cut) {
+  const int tid = threadIdx.x;
   int steps_left = count - 1;
   if (steps_left >= 1) {
     int pos = idx;
@@ -562,31 +550,21 @@ __device__ void shuffle_steps_cta(uint32_t* mt, int& idx, int count, uint16_t* j
       for (int k = tid; k < kMT; k += blockDim.x) words[k] = mt[k];
       __syncthreads();
     } else {  // the current block is used up: the first draw twists
-      mt_twist_cta(mt, words);
+      if (tid < kTwistThreads) mt_twist(mt, words);
       pos = 0;
     }
-    if (tid < 32) out[kSelBatch * kMT + tid] = 0u;  // the padding a last warp round reads
     for (;;) {
-      for (int g = 1; g < kSelBatch; ++g) mt_twist_cta(words + (g - 1) * kMT, words + g * kMT);
-      for (int k = tid; k < kSelBatch * kMT; k += blockDim.x) out[k] = mt_temper(words[k]);
+      // a step takes 1.4 words on average
+      const int blocks = min(kSelBatch, (pos + steps_left + steps_left / 2 + 64) / kMT + 1);
+      if (tid < kTwistThreads)
+        for (int g = 1; g < blocks; ++g) mt_twist(words + (g - 1) * kMT, words + g * kMT);
       __syncthreads();
-      while (steps_left >= kCtaDrawMin && pos < kSelBatch * kMT)
-        shuffle_draws_cta(out, kSelBatch * kMT, pos, steps_left, jstep, wsum, cut);
-      if (steps_left >= 1 && pos < kSelBatch * kMT) {  // uniform
-        if (warp == 0) {
-          shuffle_draws_warp(out, kSelBatch * kMT, pos, steps_left, jstep, lane);
-          if (lane == 0) {
-            s_misc[0] = steps_left;
-            s_misc[1] = pos;
-          }
-        }
-        __syncthreads();
-        steps_left = s_misc[0];
-        pos = s_misc[1];
-        __syncthreads();
-      }
+      for (int k = tid; k < blocks * kMT; k += blockDim.x) out[k] = mt_temper(words[k]);
+      __syncthreads();
+      while (steps_left >= 1 && pos < blocks * kMT)
+        shuffle_draws_cta(out, blocks * kMT, pos, steps_left, jstep, tot, cut);
       if (steps_left < 1) break;  // uniform
-      mt_twist_cta(words + (kSelBatch - 1) * kMT, words);  // the next batch starts after the last block
+      if (tid < kTwistThreads) mt_twist(words + (blocks - 1) * kMT, words);  // the next batch's first block
       pos = 0;
     }
     const int last = pos - 1;  // >= 0: every round uses at least one word
@@ -596,328 +574,345 @@ __device__ void shuffle_steps_cta(uint32_t* mt, int& idx, int count, uint16_t* j
   __syncthreads();
 }
 
-// Shuffled position p traced back through the steps after it: the item moves
-// to step s wherever j_s equals its position (s > its current step).  The warp
-// reads 256 steps at a time (8 packed 16-bit j per lane, compared two at a
-// time); a chunk with a match is re-read after each move, in step order.
-// jstep is 16-byte aligned and holds kMaxPopulation entries.
-__device__ __forceinline__ int trace_position(const uint16_t* jstep, int p, int n_window, int lane) {
-  int pos = p == 0 ? 0 : (int)jstep[p];
-  int cur = p;  // the steps up to cur are behind the item
-  const uint4* j8 = reinterpret_cast<const uint4*>(jstep);
-  for (int b = (p + 1) & ~7; b < n_window; b += 256) {
-    const int s0 = b + 8 * lane;
-    const uint4 v = s0 < kMaxPopulation ? j8[s0 >> 3] : make_uint4(0u, 0u, 0u, 0u);
-    for (;;) {
-      const uint32_t pp = (uint32_t)pos * 0x10001u;
-      const uint32_t e0 = __vcmpeq2(v.x, pp), e1 = __vcmpeq2(v.y, pp), e2 = __vcmpeq2(v.z, pp),
-                     e3 = __vcmpeq2(v.w, pp);
-      // bit h: step s0 + h has j == pos
-      uint32_t hits = (e0 & 1u) | ((e0 >> 15) & 2u) | ((e1 & 1u) << 2) | ((e1 >> 13) & 8u) | ((e2 & 1u) << 4) |
-                      ((e2 >> 11) & 32u) | ((e3 & 1u) << 6) | ((e3 >> 9) & 128u);
-      // only steps after cur and inside the window count
-      const int lo_h = cur + 1 - s0, hi_h = n_window - s0;  // valid h in [lo_h, hi_h)
-      if (lo_h > 0) hits &= lo_h >= 8 ? 0u : ~((1u << lo_h) - 1u);
-      if (hi_h < 8) hits &= hi_h <= 0 ? 0u : (1u << hi_h) - 1u;
-      const unsigned any = __ballot_sync(0xffffffffu, hits != 0u);
-      if (!any) break;  // uniform
-      const int fl = __ffs(any) - 1;
-      const uint32_t hm = __shfl_sync(0xffffffffu, hits, fl);
-      cur = b + 8 * fl + __ffs(hm) - 1;
-      pos = cur;
-    }
-  }
-  return pos;
-}
+// The scores are read from memory once: they stay in shared memory in 16 bits (in
+// jstep's space, free until the shuffle) if none is larger.  One CTA's latency
+// bounds it.  32,768 children, 64 picks, a window of 10,000: 41 us, of which the
+// draws take 26; 163 us with a score pass per step and the window traced by
+// warps reading all steps.
+struct SelSmem {
+  uint64_t keys[kMaxElite];              // the keys below T; then picked, start_next
+  uint32_t mt[kMT];
+  int32_t order[kMaxElite];              // score-order prefix
+  uint32_t mark[kMaxPopulation / 32];    // children picked
+  uint32_t window[kMaxPopulation / 32];  // children within the energy window
+  uint32_t offset[kMaxPopulation / 32];  // of these, those before the word's first
+  // draws' outputs and state blocks; before, the histogram; after, with what the
+  // window leaves of jstep, the table of step 5
+  uint16_t jstep[kMaxPopulation];  // j of shuffle step s; before, the scores
+  uint32_t words[2 * kSelBatch * kMT];
+  uint32_t hist[256];
+  uint32_t wsum[64];
+  int misc[4];
+};
+static_assert(sizeof(SelSmem) <= 227 * 1024, "select_kernel shared memory");
 
-// Warp w owns the children [w * seg, (w + 1) * seg) (seg a multiple of 32) and
-// reads them 32 at a time, so every pass over the scores is coalesced and every
-// ordered compaction is a per-warp running count plus one scan over the warps.
 __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const SelArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
+  SelSmem& S = *reinterpret_cast<SelSmem*>(smem);
   const int P = A.population, E = A.elite_size, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
-  uint64_t* keys = reinterpret_cast<uint64_t*>(smem);                 // [kMaxElite]
-  uint32_t* mt = reinterpret_cast<uint32_t*>(keys + kMaxElite);       // [624]
-  int32_t* order = reinterpret_cast<int32_t*>(mt + kMT);              // [kMaxElite] score-order prefix
-  uint32_t* mark = reinterpret_cast<uint32_t*>(order + kMaxElite);    // [kMaxPopulation / 32]
-  uint32_t* words = mark + kMaxPopulation / 32;                        // [kSelBatch][624] untempered MT blocks
-  uint32_t* tw = words + kSelBatch * kMT;                              // [kSelBatch * 624 + 32] their outputs
-  uint16_t* jstep = reinterpret_cast<uint16_t*>(tw + kSelBatch * kMT + 32);  // [population] j of shuffle step s
-  __shared__ uint32_t hist[256];
-  __shared__ int tie_off[kSelWarps], win_off[kSelWarps];
-  __shared__ int s_misc[4];
-  __shared__ uint32_t draw_wsum[64];
-  __shared__ int draw_cut[3];
   if (A.status[1] == 0) return;  // uniform: the search has reached E = 0
   const int64_t limit = A.status[1] + (int64_t)A.energy_window;
-  for (int i = tid; i < kMaxPopulation / 32; i += kSelThreads) mark[i] = 0u;
-  for (int i = tid; i < kMT; i += kSelThreads) mt[i] = A.rng[i];
-  const int seg = (P + kSelThreads - 1) / kSelThreads * 32;
-  const int s_lo = min(P, warp * seg), s_hi = min(P, s_lo + seg);
-  if (tid == 0) s_misc[2] = 0;
+  for (int i = tid; i < kMaxPopulation / 32; i += kSelThreads) S.mark[i] = 0u;
+  for (int i = tid; i < kMT; i += kSelThreads) S.mt[i] = A.rng[i];
 
-  // 1. T = the E-th smallest score: radix select over the 32-bit scores, 8 bits
-  //    a pass, from the highest byte that any score uses
+  // 1. T = the E-th smallest score.  One pass counts the scores below 4096, one
+  //    bin per value (in the MT words' space), and finds the highest; if all are
+  //    counted a scan over the bins tells T, otherwise a radix select over the
+  //    32-bit scores, 8 bits a pass, from the highest byte that any score uses.
+  uint32_t* const bins = S.words;
+  uint16_t* const kept = S.jstep;
+  for (int i = tid; i < kSelHistBins; i += kSelThreads) bins[i] = 0u;
+  if (tid == 0) S.misc[2] = 0;
+  __syncthreads();
   uint32_t top = 0u;
-  for (int b = s_lo; b < s_hi; b += 32)
-    if (b + lane < s_hi) top = max(top, (uint32_t)A.scores[b + lane]);
-  top = __reduce_max_sync(0xffffffffu, top);
-  if (lane == 0) hist[warp] = top;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t m = __reduce_max_sync(0xffffffffu, hist[lane]);
-    if (lane == 0) s_misc[3] = (int)m;
+#pragma unroll 8
+  for (int i = tid; i < P; i += kSelThreads) {
+    const uint32_t x = (uint32_t)A.scores[i];
+    top = max(top, x);
+    kept[i] = (uint16_t)x;
+    if (x < (uint32_t)kSelHistBins) atomicAdd(&bins[x], 1u);
   }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) S.hist[warp] = top;
   __syncthreads();
-  top = (uint32_t)s_misc[3];
-  int shift = 24;
-  while (shift > 0 && (top >> shift) == 0u) shift -= 8;  // the skipped high bytes are zero in every score
-  uint32_t prefix = 0u, mask = 0u;
-  int remaining = E;  // 1-based rank of the E-th element among those matching prefix
+  top = __reduce_max_sync(0xffffffffu, S.hist[lane]);
+  __syncthreads();
+  uint32_t T;
+  int remaining;  // 1-based rank of the E-th element among the scores equal to T
+  const bool in_16 = top <= 0xFFFFu;  // uniform
   if (top < (uint32_t)kSelHistBins) {
-    // every score below 4096: one pass, one bin per score value (in the MT words'
-    // space, free until the shuffle), then a scan over the bins
-    uint32_t* h12 = words;
-    for (int i = tid; i < kSelHistBins; i += kSelThreads) h12[i] = 0u;
-    __syncthreads();
-#pragma unroll 4
-    for (int b = s_lo; b < s_hi; b += 32) {
-      const int i = b + lane;
-      const bool valid = i < s_hi;
-      const uint32_t x = valid ? (uint32_t)A.scores[i] : 0u;
-      const unsigned act = __ballot_sync(0xffffffffu, valid);
-      if (valid) {
-        const unsigned peers = __match_any_sync(act, x);
-        if (lane == __ffs(peers) - 1) atomicAdd(&h12[x], (uint32_t)__popc(peers));
-      }
-    }
-    __syncthreads();
     constexpr int kPerT = kSelHistBins / kSelThreads;
     uint32_t c[kPerT], local = 0u;
 #pragma unroll
     for (int k = 0; k < kPerT; ++k) {
-      c[k] = h12[kPerT * tid + k];
+      c[k] = bins[kPerT * tid + k];
       local += c[k];
     }
     uint32_t tot;
-    int run = (int)cta_exscan32(local, draw_wsum, tot);
+    int run = (int)cta_exscan32(local, S.wsum, tot);
     if (run < E && run + (int)local >= E) {  // this thread's bins hold the E-th smallest score
 #pragma unroll
       for (int k = 0; k < kPerT; ++k) {
         if (run + (int)c[k] >= E) {
-          s_misc[0] = kPerT * tid + k;
-          s_misc[1] = E - run;
+          S.misc[0] = kPerT * tid + k;
+          S.misc[1] = E - run;
           break;
         }
         run += (int)c[k];
       }
     }
     __syncthreads();
-    prefix = (uint32_t)s_misc[0];
-    remaining = s_misc[1];
-    shift = -8;  // done
-    __syncthreads();
-  }
-  for (; shift >= 0; shift -= 8) {
-    for (int i = tid; i < 256; i += kSelThreads) hist[i] = 0u;
-    __syncthreads();
+    T = (uint32_t)S.misc[0];
+    remaining = S.misc[1];
+  } else {
+    int shift = 24;
+    while (shift > 0 && (top >> shift) == 0u) shift -= 8;  // the skipped high bytes are zero in every score
+    uint32_t prefix = 0u, mask = 0u;
+    remaining = E;
+    for (; shift >= 0; shift -= 8) {
+      for (int i = tid; i < 256; i += kSelThreads) S.hist[i] = 0u;
+      __syncthreads();
 #pragma unroll 4
-    for (int b = s_lo; b < s_hi; b += 32) {  // warp-uniform trip count; equal digits add once per warp
-      const int i = b + lane;
-      const uint32_t x = i < s_hi ? (uint32_t)A.scores[i] : 0u;
-      const bool valid = i < s_hi && (x & mask) == prefix;
-      const unsigned act = __ballot_sync(0xffffffffu, valid);
-      if (valid) {
-        const uint32_t digit = (x >> shift) & 255u;
-        const unsigned peers = __match_any_sync(act, digit);
-        if (lane == __ffs(peers) - 1) atomicAdd(&hist[digit], (uint32_t)__popc(peers));
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int before = 0, d = 0;
-      for (; d < 255; ++d) {
-        if (before + (int)hist[d] >= remaining) break;
-        before += (int)hist[d];
-      }
-      s_misc[0] = d;
-      s_misc[1] = remaining - before;
-    }
-    __syncthreads();
-    prefix |= (uint32_t)s_misc[0] << shift;
-    mask |= 255u << shift;
-    remaining = s_misc[1];
-    __syncthreads();
-  }
-  const uint32_t T = prefix;
-  const int n_less = E - remaining;  // scores below T; then `remaining` ties at T by index
-
-  // 2. one pass: the keys below T (at most E - 1), and per warp the ties at T
-  //    and the children within the energy window
-  int c_tie = 0, c_win = 0;
-#pragma unroll 4
-  for (int b = s_lo; b < s_hi; b += 32) {
-    const int i = b + lane;
-    const int x = i < s_hi ? A.scores[i] : 0;
-    const unsigned lt = __ballot_sync(0xffffffffu, i < s_hi && (uint32_t)x < T);
-    if (lt) {
-      int at = 0;
-      if (lane == 0) at = atomicAdd(&s_misc[2], __popc(lt));
-      at = __shfl_sync(0xffffffffu, at, 0);
-      if ((lt >> lane) & 1u) keys[at + __popc(lt & below)] = ((uint64_t)(uint32_t)x << 32) | (uint32_t)i;
-    }
-    c_tie += __popc(__ballot_sync(0xffffffffu, i < s_hi && (uint32_t)x == T));
-    c_win += __popc(__ballot_sync(0xffffffffu, i < s_hi && (int64_t)x <= limit));
-  }
-  if (lane == 0) {
-    tie_off[warp] = c_tie;
-    win_off[warp] = c_win;
-  }
-  __syncthreads();
-  if (warp == 0) {  // exclusive scans over the warps
-    int t = tie_off[lane], w = win_off[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int yt = __shfl_up_sync(0xffffffffu, t, o), yw = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) {
-        t += yt;
-        w += yw;
-      }
-    }
-    tie_off[lane] = t - tie_off[lane];
-    if (lane == 31) s_misc[0] = w;  // the window's size
-    win_off[lane] = w - win_off[lane];
-  }
-  int width = 1;
-  while (width < n_less) width <<= 1;
-  for (int i = n_less + tid; i < width; i += kSelThreads) keys[i] = ~0ull;
-  __syncthreads();
-  const int n_window = s_misc[0];
-
-  // 3. the first `remaining` ties at T in index order; the keys below T sorted
-  //    by (score, index) with a bitonic sort
-  {
-    int o = tie_off[warp];
-    for (int b = s_lo; b < s_hi && o < remaining; b += 32) {
-      const int i = b + lane;
-      const unsigned m = __ballot_sync(0xffffffffu, i < s_hi && (uint32_t)A.scores[i] == T);
-      if ((m >> lane) & 1u) {
-        const int r = o + __popc(m & below);
-        if (r < remaining) order[n_less + r] = i;
-      }
-      o += __popc(m);
-    }
-  }
-  for (int size = 2; size <= width; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < width; i += kSelThreads) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const uint64_t a = keys[i], b = keys[j];
-          if ((a > b) == up) {
-            keys[i] = b;
-            keys[j] = a;
-          }
+      for (int b = 32 * warp; b < P; b += kSelThreads) {  // warp-uniform trip count; equal digits add once per warp
+        const int i = b + lane;
+        const uint32_t x = i < P ? (uint32_t)A.scores[i] : 0u;
+        const bool valid = i < P && (x & mask) == prefix;
+        const unsigned act = __ballot_sync(0xffffffffu, valid);
+        if (valid) {
+          const uint32_t digit = (x >> shift) & 255u;
+          const unsigned peers = __match_any_sync(act, digit);
+          if (lane == __ffs(peers) - 1) atomicAdd(&S.hist[digit], (uint32_t)__popc(peers));
         }
       }
       __syncthreads();
+      if (tid == 0) {
+        int before = 0, d = 0;
+        for (; d < 255; ++d) {
+          if (before + (int)S.hist[d] >= remaining) break;
+          before += (int)S.hist[d];
+        }
+        S.misc[0] = d;
+        S.misc[1] = remaining - before;
+      }
+      __syncthreads();
+      prefix |= (uint32_t)S.misc[0] << shift;
+      mask |= 255u << shift;
+      remaining = S.misc[1];
+      __syncthreads();
     }
+    T = prefix;
   }
-  for (int i = tid; i < n_less; i += kSelThreads) order[i] = (int32_t)(uint32_t)keys[i];
+  const int n_less = E - remaining;  // scores below T; then `remaining` ties at T by index
+
+  // 2. a thread per 32 children: the keys below T (at most E - 1) in any order,
+  //    the first `remaining` ties at T in index order, and the children within
+  //    the energy window
+  int n_window = 0, n_tie = 0;
+  for (int w0 = 0; w0 < (P + 31) / 32; w0 += kSelThreads) {
+    const int w = w0 + tid, i0 = 32 * w;
+    uint32_t lt = 0u, tie = 0u, within = 0u;
+    if (i0 < P) {
+      if (in_16) {
+        const uint32_t* const two = reinterpret_cast<const uint32_t*>(kept) + 16 * w;
+        const int turn = tid & 15;  // the lanes in different banks
+        const int low = (int)min(limit, (int64_t)0xFFFF);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const uint32_t v = two[(k + turn) & 15];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int x = h ? (int)(v >> 16) : (int)(v & 0xFFFFu);
+            if (x < (int)T) lt |= 1u << (2 * k + h);
+            if (x == (int)T) tie |= 1u << (2 * k + h);
+            if (x <= low) within |= 1u << (2 * k + h);
+          }
+        }
+        lt = __funnelshift_l(lt, lt, 2 * turn);
+        tie = __funnelshift_l(tie, tie, 2 * turn);
+        within = __funnelshift_l(within, within, 2 * turn);
+      } else {
+        for (int k = 0; k < 32; ++k) {
+          const int x = A.scores[min(i0 + k, P - 1)];
+          if ((uint32_t)x < T) lt |= 1u << k;
+          if ((uint32_t)x == T) tie |= 1u << k;
+          if ((int64_t)x <= limit) within |= 1u << k;
+        }
+      }
+      const uint32_t valid = P - i0 < 32 ? (1u << (P - i0)) - 1u : ~0u;
+      lt &= valid;
+      tie &= valid;
+      within &= valid;
+    }
+    uint32_t tot;  // at most 32768 of each in a round
+    const uint32_t before = cta_exscan32((uint32_t)__popc(tie) << 16 | (uint32_t)__popc(within),
+                                         S.wsum + ((w0 / kSelThreads) & 1) * 32, tot);
+    if (i0 < P) {
+      S.window[w] = within;
+      S.offset[w] = (uint32_t)n_window + (before & 0xFFFFu);
+      int at = lt ? atomicAdd(&S.misc[2], __popc(lt)) : 0;
+      for (; lt; lt &= lt - 1u) {
+        const int i = i0 + __ffs(lt) - 1;
+        S.keys[at++] = (uint64_t)(uint32_t)(in_16 ? (int)kept[i] : A.scores[i]) << 32 | (uint32_t)i;
+      }
+      for (int r = n_tie + (int)(before >> 16); tie && r < remaining; tie &= tie - 1u, ++r)
+        S.order[n_less + r] = i0 + __ffs(tie) - 1;
+    }
+    n_window += (int)(tot & 0xFFFFu);
+    n_tie += (int)(tot >> 16);
+  }
+  // 3. the keys below T sorted by (score, index): up to 512 by counting the lower
+  //    ones, a warp per key (64 keys: 0.5 us, bitonic 2.9 us), more with a bitonic sort
+  if (n_less <= 512) {
+    __syncthreads();
+    for (int k = warp; k < n_less; k += kSelWarps) {
+      const uint64_t key = S.keys[k];
+      int lower = 0;
+      for (int j = lane; j < n_less; j += 32) lower += S.keys[j] < key;
+      lower = __reduce_add_sync(0xffffffffu, lower);
+      if (lane == 0) S.order[lower] = (int32_t)(uint32_t)key;
+    }
+  } else {
+    int width = 1;
+    while (width < n_less) width <<= 1;
+    for (int i = n_less + tid; i < width; i += kSelThreads) S.keys[i] = ~0ull;
+    __syncthreads();
+    for (int size = 2; size <= width; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int i = tid; i < width; i += kSelThreads) {
+          const int j = i ^ stride;
+          if (j > i) {
+            const bool up = (i & size) == 0;
+            const uint64_t a = S.keys[i], b = S.keys[j];
+            if ((a > b) == up) {
+              S.keys[i] = b;
+              S.keys[j] = a;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    }
+    for (int i = tid; i < n_less; i += kSelThreads) S.order[i] = (int32_t)(uint32_t)S.keys[i];
+  }
+  __syncthreads();  // the scores are no longer read, nor the keys
 
   // 4. the draws of the window list's shuffle (gpu_device_search.py:340-373):
   //    the j of every step s in jstep[s], no swap made (shuffle_steps_cta).
   {
     int idx = (int)A.rng[kMT];  // uniform
-    shuffle_steps_cta(mt, idx, n_window, jstep, words, tw, draw_wsum, draw_cut, s_misc);
+    shuffle_steps_cta(S.mt, idx, n_window, S.jstep, S.words, S.words + kSelBatch * kMT, S.wsum, &S.misc[0]);
     if (tid == 0) A.rng[kMT] = (uint32_t)idx;
   }
 
-  // 5. the first K = min(E, window) shuffled positions, one warp each.  Step s
-  //    fixes position s for good, so position p holds what sat at j_p before
-  //    step p; going back through the later steps p+1, p+2, ... (applied before
-  //    it), the item moves only where a step's j equals its position, to that
-  //    step.  The window position found is then mapped to its child through
-  //    the per-warp window offsets.
+  // 5. the first K = min(E, window) shuffled positions.  Step s fixes position s
+  //    for good, so position p holds what sat at j_p before step p; going back
+  //    through the later steps p+1, p+2, ... (applied before it), the item moves
+  //    only where a step's j equals its position, to that step.  From then on its
+  //    position is the step it came from, so what it needs is next[x], the first
+  //    step s > x with j_s = x; and for the start, the first step s > p with
+  //    j_s = j_p: j_p <= p < K, so a search of the steps below K, then start_next,
+  //    the first step from K on.  One pass over the steps fills both, the table
+  //    of next for a part of the positions at a time if the window leaves no room
+  //    for all (above 28,500).
   const int K = min(E, n_window);
-  int32_t* picked = reinterpret_cast<int32_t*>(keys);  // [K]; keys is free once order is written
-  for (int p = warp; p < K; p += kSelWarps) {
-    const int pos = trace_position(jstep, p, n_window, lane);
-    const unsigned owners = __ballot_sync(0xffffffffu, win_off[lane] <= pos);  // bit 0 always set
-    const int w = 31 - __clz(owners);
-    int rank = pos - win_off[w];
-    const int w_lo = min(P, w * seg), w_hi = min(P, w_lo + seg);
-    int child = -1;
-    for (int b = w_lo; b < w_hi; b += 32) {
-      const int i = b + lane;
-      const unsigned m = __ballot_sync(0xffffffffu, i < w_hi && (int64_t)A.scores[i] <= limit);
-      const int c = __popc(m);
-      if (rank < c) {  // uniform
-        const unsigned hitl = __ballot_sync(0xffffffffu, ((m >> lane) & 1u) && __popc(m & below) == rank);
-        child = b + __ffs(hitl) - 1;
-        break;
-      }
-      rank -= c;
+  int32_t* const picked = reinterpret_cast<int32_t*>(S.keys);        // [K] positions, then children
+  uint32_t* const start_next = reinterpret_cast<uint32_t*>(S.keys) + kMaxElite;  // [K]
+  const int table_at = (n_window + 1) & ~1;
+  uint32_t* const next = reinterpret_cast<uint32_t*>(S.jstep + table_at);
+  const int room = (kMaxPopulation - table_at) / 2 + 2 * kSelBatch * kMT;
+  for (int i = tid; i < K; i += kSelThreads) start_next[i] = UINT32_MAX;
+  for (int lo = 0; lo < n_window; lo += room) {
+    const int hi = min(n_window, lo + room);
+    for (int i = tid; i < hi - lo; i += kSelThreads) next[i] = UINT32_MAX;
+    __syncthreads();
+    for (int s = 1 + tid; s < n_window; s += kSelThreads) {
+      const int j = S.jstep[s];
+      if (j < s && j >= lo && j < hi) atomicMin(&next[j - lo], (uint32_t)s);
+      if (lo == 0 && s >= K && j < K) atomicMin(&start_next[j], (uint32_t)s);
     }
-    if (lane == 0) picked[p] = child;
+    __syncthreads();
+    if (lo == 0) {  // the starts, a warp each
+      for (int p = warp; p < K; p += kSelWarps) {
+        const int j = p ? (int)S.jstep[p] : 0;
+        uint32_t first = start_next[j];
+        for (int s0 = p + 1; s0 < K; s0 += 32) {
+          const unsigned m = __ballot_sync(0xffffffffu, s0 + lane < K && (int)S.jstep[s0 + lane] == j);
+          if (m) {  // uniform
+            first = (uint32_t)(s0 + __ffs(m) - 1);
+            break;
+          }
+        }
+        if (lane == 0) picked[p] = first == UINT32_MAX ? ~j : (int32_t)first;  // complemented: it stays there
+      }
+      __syncthreads();
+    }
+    for (int p = tid; p < K; p += kSelThreads) {
+      if (picked[p] < 0) continue;
+      uint32_t at = (uint32_t)picked[p];
+      while (at < (uint32_t)hi) {
+        const uint32_t to = next[at - (uint32_t)lo];
+        if (to == UINT32_MAX) break;
+        at = to;
+      }
+      picked[p] = at < (uint32_t)hi ? ~(int32_t)at : (int32_t)at;
+    }
+    __syncthreads();
   }
-  __syncthreads();
+  // the window's position to its child
+  for (int p = tid; p < K; p += kSelThreads) {
+    const uint32_t pos = (uint32_t)~picked[p];
+    int w = 0, w_end = (P + 31) / 32;  // the last word whose offset is not above pos
+    while (w_end - w > 1) {
+      const int mid = (w + w_end) >> 1;
+      if (S.offset[mid] <= pos) w = mid;
+      else w_end = mid;
+    }
+    uint32_t m = S.window[w];
+    for (uint32_t r = pos - S.offset[w]; r > 0u; --r) m &= m - 1u;
+    picked[p] = 32 * w + __ffs(m) - 1;
+  }
 
-  // 6. thread 0: the pick (gpu_device_search.py:340-373)
-  if (tid == 0) {
-    int sel = 0;
-    const int quality_keep = max(1, E / 4);
-    for (int r = 0; r < quality_keep; ++r) {
-      const int c = order[r];
-      mark[c >> 5] |= 1u << (c & 31);
-      A.selected[sel++] = c;
-    }
-    for (int k = 0; k < K && sel < E; ++k) {
-      const int c = picked[k];
-      if (c >= 0 && !(mark[c >> 5] & (1u << (c & 31)))) {
-        mark[c >> 5] |= 1u << (c & 31);
-        A.selected[sel++] = c;
-      }
-    }
-    for (int r = 0; r < E && sel < E; ++r) {
-      const int c = order[r];
-      if (!(mark[c >> 5] & (1u << (c & 31)))) {
-        mark[c >> 5] |= 1u << (c & 31);
-        A.selected[sel++] = c;
-      }
-    }
+  // 6. the pick (gpu_device_search.py:340-373): the best quarter, the shuffled
+  //    window without them (its children are distinct), then the score order
+  const int quality = max(1, E / 4);
+  for (int r = tid; r < quality; r += kSelThreads) {
+    const int c = S.order[r];
+    atomicOr(&S.mark[c >> 5], 1u << (c & 31));
+    A.selected[r] = c;
   }
   __syncthreads();
-  for (int i = tid; i < kMT; i += kSelThreads) A.rng[i] = mt[i];
+  int sel = quality;
+  for (int part = 0; part < 2; ++part) {
+    const int32_t* const list = part ? S.order : picked;
+    const int end = part ? E : K;
+    for (int r0 = 0; r0 < end && sel < E; r0 += kSelThreads) {  // uniform
+      const int r = r0 + tid;
+      const int c = r < end ? list[r] : 0;
+      const bool open = r < end && !((S.mark[c >> 5] >> (c & 31)) & 1u);
+      uint32_t tot;
+      const int at = sel + (int)cta_exscan32(open, S.wsum + ((r0 / kSelThreads + part) & 1) * 32, tot);
+      if (open && at < E) {
+        A.selected[at] = c;
+        if (part == 0) atomicOr(&S.mark[c >> 5], 1u << (c & 31));
+      }
+      sel += (int)tot;
+      __syncthreads();
+    }
+  }
+  for (int i = tid; i < kMT; i += kSelThreads) A.rng[i] = S.mt[i];
 }
 
 // The shuffle's draws alone (shuffle_steps_cta), for callers that apply the
 // permutation themselves and for tests: j of step s in jout[s], jout[0] = 0.
-constexpr size_t kStepsSmem = sizeof(uint32_t) * (kMT + 2 * kSelBatch * kMT + 32) + sizeof(uint16_t) * kMaxPopulation;
+constexpr size_t kStepsSmem = sizeof(uint32_t) * (kMT + 2 * kSelBatch * kMT) + sizeof(uint16_t) * kMaxPopulation;
 __global__ void __launch_bounds__(kSelThreads, 1) py_steps_kernel(uint32_t* state, int count, int32_t* jout) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* mt = reinterpret_cast<uint32_t*>(smem);
   uint32_t* words = mt + kMT;
   uint32_t* out = words + kSelBatch * kMT;
-  uint16_t* jstep = reinterpret_cast<uint16_t*>(out + kSelBatch * kMT + 32);
-  __shared__ uint32_t wsum[64];
-  __shared__ int cut[3], s_misc[4];
+  uint16_t* jstep = reinterpret_cast<uint16_t*>(out + kSelBatch * kMT);
+  __shared__ uint32_t tot[64];
+  __shared__ int cut;
   for (int i = threadIdx.x; i < kMT; i += blockDim.x) mt[i] = state[i];
   __syncthreads();
   int idx = (int)state[kMT];
-  shuffle_steps_cta(mt, idx, count, jstep, words, out, wsum, cut, s_misc);
+  shuffle_steps_cta(mt, idx, count, jstep, words, out, tot, &cut);
   for (int s = threadIdx.x; s < count; s += blockDim.x) jout[s] = s == 0 ? 0 : (int32_t)jstep[s];
   for (int i = threadIdx.x; i < kMT; i += blockDim.x) state[i] = mt[i];
   if (threadIdx.x == 0) state[kMT] = (uint32_t)idx;
 }
-
-constexpr size_t kSelSmem = sizeof(uint64_t) * kMaxElite + sizeof(uint32_t) * kMT + sizeof(int32_t) * kMaxElite +
-                            sizeof(uint32_t) * (kMaxPopulation / 32) + sizeof(uint32_t) * (2 * kSelBatch * kMT + 32) +
-                            sizeof(uint16_t) * kMaxPopulation;
-static_assert(kSelSmem <= 227 * 1024 - 2048, "select_kernel shared memory");
 
 // pick rows r = child rows selected[r]
 __global__ void gather_kernel(const int32_t* __restrict__ cp, const int32_t* __restrict__ cq,
@@ -938,7 +933,8 @@ __global__ void gather_kernel(const int32_t* __restrict__ cp, const int32_t* __r
 // Ranking (one CTA): rank_elites (gpu_device_search.py:185-197) is a stable
 // sort by elite_key = (E, max badness, sum of squared badness); each element's
 // rank is the number of keys before it.  Then the best-so-far update
-// (gpu_device_search.py:388-396; set-up: :305-310).
+// (gpu_device_search.py:388-396; set-up: :305-310).  A warp per state: 64 states
+// at n = 75 take 11 us, 23 us by a thread each.
 // --------------------------------------------------------------------------
 constexpr int kRankThreads = 1024;
 
@@ -965,42 +961,55 @@ __global__ void __launch_bounds__(kRankThreads, 1) rank_kernel(const RankArgs A)
   __shared__ int64_t s_ss[kMaxElite];
   __shared__ int s_first, s_improved;
   if (A.generation > 0 && A.status[1] == 0) return;  // uniform
-  const int C = A.count, m = 2 * A.n, tid = threadIdx.x;
-  for (int i = tid; i < C; i += kRankThreads) {
+  const int C = A.count, m = 2 * A.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = warp; i < C; i += kRankThreads / 32) {  // a warp per state
     int mx = INT32_MIN;
     int64_t ss = 0;
-    for (int s = 0; s < m; ++s) {
-      const int b = A.pbad[(size_t)i * m + s];
+#pragma unroll
+    for (int k = 0; k < kSlotsPerLane; ++k) {
+      const int s = lane + 32 * k;
+      const int b = s < m ? A.pbad[(size_t)i * m + s] : INT32_MIN;
       mx = max(mx, b);
-      ss += (int64_t)b * b;
+      if (s < m) ss += (int64_t)b * b;
     }
-    s_score[i] = A.ps[i];
-    s_max[i] = mx;
-    s_ss[i] = ss;
+    mx = __reduce_max_sync(0xffffffffu, mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) {
+      s_score[i] = A.ps[i];
+      s_max[i] = mx;
+      s_ss[i] = ss;
+    }
   }
   __syncthreads();
-  for (int i = tid; i < C; i += kRankThreads) {
+  for (int i = warp; i < C; i += kRankThreads / 32) {
     const int a0 = s_score[i], a1 = s_max[i];
     const int64_t a2 = s_ss[i];
     int r = 0;
-    for (int j = 0; j < C; ++j) {
+    for (int j = lane; j < C; j += 32) {
       const int b0 = s_score[j], b1 = s_max[j];
       const int64_t b2 = s_ss[j];
       const bool less = b0 < a0 || (b0 == a0 && (b1 < a1 || (b1 == a1 && (b2 < a2 || (b2 == a2 && j < i)))));
       r += less;
     }
-    s_rank[i] = r;
-    if (r == 0) s_first = i;
+    r = __reduce_add_sync(0xffffffffu, r);
+    if (lane == 0) {
+      s_rank[i] = r;
+      if (r == 0) s_first = i;
+    }
   }
   __syncthreads();
-  for (int e = tid; e < C * A.n; e += kRankThreads) {
-    const int i = e / A.n, k = e % A.n;
-    A.ep[(size_t)s_rank[i] * A.n + k] = A.pp[e];
-    A.eq[(size_t)s_rank[i] * A.n + k] = A.pq[e];
-  }
-  for (int e = tid; e < C * m; e += kRankThreads) {
-    const int i = e / m, k = e % m;
-    A.ebad[(size_t)s_rank[i] * m + k] = A.pbad[e];
+  for (int i = warp; i < C; i += kRankThreads / 32) {  // a warp per state
+    const size_t to = (size_t)s_rank[i], from = (size_t)i;
+#pragma unroll
+    for (int k = 0; k < kSlotsPerLane; ++k) {
+      const int s = lane + 32 * k;
+      if (s < m) A.ebad[to * m + s] = A.pbad[from * m + s];
+      if (s < A.n) {
+        A.ep[to * A.n + s] = A.pp[from * A.n + s];
+        A.eq[to * A.n + s] = A.pq[from * A.n + s];
+      }
+    }
   }
   for (int i = tid; i < C; i += kRankThreads) A.es[s_rank[i]] = s_score[i];
   if (tid == 0) {
@@ -1047,9 +1056,11 @@ static int launch_mutate(n3::beam::MutArgs A, int parents_bound, cudaStream_t st
   const int m = 2 * A.n;
   const int cap = (int)(kMutPrefixMaxBytes / (sizeof(int32_t) * (size_t)m));
   A.prefix_cap = parents_bound <= cap ? parents_bound : 0;
-  const size_t bytes = sizeof(int32_t) * (size_t)m * (kMutThreads + A.prefix_cap);
+  int threads = 64;
+  while (threads < kMutThreads && (A.population + threads - 1) / threads > sm_count()) threads *= 2;
+  const size_t bytes = (size_t)m * (sizeof(int16_t) * (size_t)threads + sizeof(int32_t) * (size_t)A.prefix_cap);
   N3_TRY(allow_smem(reinterpret_cast<const void*>(mutate_kernel), kMutSmemMax));
-  mutate_kernel<<<(A.population + kMutThreads - 1) / kMutThreads, kMutThreads, bytes, st>>>(A);
+  mutate_kernel<<<(A.population + threads - 1) / threads, threads, bytes, st>>>(A);
   return check_launch("beam mutate_kernel");
 }
 
@@ -1132,7 +1143,7 @@ int n3_beam_mutate(const int32_t* parent_p, const int32_t* parent_q, const int32
 
 int n3_py_random_seed(uint32_t* state, uint64_t seed, void* stream) {
   if (!state) return n3host::set_error(N3_ERR_ARG, "null RNG state");
-  n3::beam::py_seed_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(state, seed);
+  n3::beam::py_seed_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(state, seed);
   return n3host::check_launch("py_seed_kernel");
 }
 
@@ -1213,7 +1224,7 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   n3::beam::child_delta_kernel<<<dgrid < n3host::sm_count() ? dgrid : n3host::sm_count(), n3::beam::kDeltaWarps * 32,
                                  n3::beam::kDeltaSmem, st>>>(D);
   N3_TRY(n3host::check_launch("beam child_delta_kernel"));
-  N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::beam::select_kernel), n3::beam::kSelSmem));
+  N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::beam::select_kernel), sizeof(n3::beam::SelSmem)));
   n3::beam::SelArgs S;
   S.scores = b->child_scores;
   S.population = b->population;
@@ -1222,7 +1233,7 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   S.status = b->status;
   S.rng = b->rng;
   S.selected = b->selected;
-  n3::beam::select_kernel<<<1, n3::beam::kSelThreads, n3::beam::kSelSmem, st>>>(S);
+  n3::beam::select_kernel<<<1, n3::beam::kSelThreads, sizeof(n3::beam::SelSmem), st>>>(S);
   N3_TRY(n3host::check_launch("beam select_kernel"));
   n3::beam::gather_kernel<<<b->elite_size, 128, 0, st>>>(b->child_p, b->child_q, b->child_scores, b->child_badness,
                                                           b->selected, b->n, b->status, b->pick_p, b->pick_q,
