@@ -30,70 +30,105 @@
 
 namespace n3 {
 
-// Exact dE (and, if dbad != nullptr, this lane's badness changes for slots
-// lane + 32 t, plus the moved slots' changes in *dbad_u, *dbad_v) of a legal
-// move.  Uses the 4 centres u, v, u', v'; hist must be zeroed, is left zeroed.
-// lutf: the full signed direction table; key: this lane's slots' table keys
-// row * kLutW + column.
+// One legal move by 8-bit histograms over A, one centre at a time, for what
+// swap_delta_pair leaves: its dE and badness changes (BAD; change[t] for slot lane +
+// 32 t).  hist: kDirWords words, zero, left zero.
 template <bool BAD>
-__device__ __forceinline__ int swap_delta_hist(const int* __restrict__ cs, const int (&key)[kSlotsPerLane], int m,
-                                               int u, int v, const uint16_t* __restrict__ lutf,
-                                               uint32_t* __restrict__ hist, int lane, int (&dbad)[kSlotsPerLane],
-                                               int* dbad_u, int* dbad_v) {
-  const int ru = u >> 1, rv = v >> 1, cu = cs[u], cv = cs[v];
-  // centre order: u, v, u', v'
-  const int crow[4] = {ru, rv, ru, rv};
-  const int ccol[4] = {cu, cv, cv, cu};
-  int tX[4];
-  int j_old = 0, j_new = 0;
-  if (BAD) {
+__device__ __noinline__ int swap_delta_slow(const int (&key2)[kSlotsPerLane], int m, int lane, int u, int v, int cu,
+                                            int cv, const uint16_t* __restrict__ lut4, uint32_t* __restrict__ hist,
+                                            int (&change)[kSlotsPerLane]) {
+  const int ru = u >> 1, rv = v >> 1;
+  int t_sum[4], line_count[2] = {0, 0};
+  for (int t = 0; t < kSlotsPerLane; ++t) change[t] = 0;
 #pragma unroll
-    for (int t = 0; t < kSlotsPerLane; ++t) dbad[t] = 0;
-  }
+  for (int c = 0; c < 4; ++c) {  // u, v, u', v'
+    const int rx = (c & 1) ? rv : ru, centre = rx * kLutW + (c == 0 || c == 3 ? cu : cv);
+    int ids[kSlotsPerLane], part = 0;
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    int ids[kSlotsPerLane];
-    int part = 0;
-    {
-      const int rx = crow[c];
-      const uint16_t* base = lutf + kFullLutCentre - (rx * kLutW + ccol[c]);
-#pragma unroll
-      for (int t = 0; t < kSlotsPerLane; ++t) {
-        const int k = lane + 32 * t;
-        ids[t] = -1;
-        if (k < m && k != u && k != v && (k >> 1) != rx) {
-          const int id = base[key[t]];
-          ids[t] = id;
-          part += hist_add(hist, id);
-        }
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      const int k = lane + 32 * t;
+      ids[t] = -1;
+      if (k < m && k != u && k != v && (k >> 1) != rx) {
+        ids[t] = (int)(dir4(lut4, key2[t] >> 1, centre) >> 2);
+        part += hist_add(hist, ids[t]);
       }
     }
     __syncwarp();
-    tX[c] = warp_sum(part);
-    const int sign = c < 2 ? -1 : 1;
-    int line_id = -1;  // direction of the other moved point, for centres u and u'
-    if (c == 0) {
-      line_id = dir_id_full(lutf, rv - ru, cv - cu);
-      j_old = hist_get(hist, line_id);
-    } else if (c == 2) {
-      line_id = dir_id_full(lutf, rv - ru, cu - cv);
-      j_new = hist_get(hist, line_id);
+    t_sum[c] = warp_sum(part);
+    int line = -1;  // direction of the other moved point, for u and u'
+    if (!(c & 1)) {
+      line = (int)(dir4(lut4, rv * kLutW + (c ? cu : cv), centre) >> 2);
+      line_count[c >> 1] = hist_get(hist, line);
     }
     if (BAD) {
 #pragma unroll
-      for (int t = 0; t < kSlotsPerLane; ++t) {
-        if (ids[t] >= 0) dbad[t] += sign * (hist_get(hist, ids[t]) - 1 + (ids[t] == line_id));
-      }
+      for (int t = 0; t < kSlotsPerLane; ++t)
+        if (ids[t] >= 0) change[t] += (c < 2 ? -1 : 1) * (hist_get(hist, ids[t]) - 1 + (ids[t] == line));
     }
     __syncwarp();
     hist_release(hist, ids);
     __syncwarp();
   }
+  const int before_u = t_sum[0] + line_count[0], before_v = t_sum[1] + line_count[0];
+  const int after_u = t_sum[2] + line_count[1], after_v = t_sum[3] + line_count[1];
   if (BAD) {
-    *dbad_u = (tX[2] + j_new) - (tX[0] + j_old);
-    *dbad_v = (tX[3] + j_new) - (tX[1] + j_old);
+#pragma unroll
+    for (int t = 0; t < kSlotsPerLane; ++t) {
+      if (lane + 32 * t == u) change[t] = after_u - before_u;
+      if (lane + 32 * t == v) change[t] = after_v - before_v;
+    }
   }
-  return (tX[2] + tX[3] + j_new) - (tX[0] + tX[1] + j_old);
+  return after_u + after_v - line_count[1] - (before_u + before_v - line_count[0]);
+}
+
+// The same with 4-bit counters, u' and v' side by side and then u and v
+// (pair_move.cuh).  False, with nothing to use, if a counter may have wrapped.
+template <bool BAD, int NT>
+__device__ __forceinline__ bool swap_delta_pair(const WarpState& W, int u, int v, int cu, int cv,
+                                                const uint16_t* __restrict__ lut4, uint32_t* __restrict__ hist,
+                                                int& dE, int (&change)[kSlotsPerLane]) {
+  using Num = DenseNumbering;
+  uint32_t* const h1 = hist + Num::kWords;
+  const int ru = u >> 1, rv = v >> 1;
+  Directions a, b;
+  uint32_t line_new;
+  const PairCount p = count_pair<Num, NT, false>(W, lut4, hist, ru, rv, cu, cv, a, b, line_new);
+  if (BAD) {  // as pair_move takes them
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+      change[t] = centre_get(a, t) + centre_get(b, t) - (a.e[t] == Num::kRow || a.e[t] == Num::kCol) -
+                  (b.e[t] == Num::kRow || b.e[t] == Num::kCol) + (a.e[t] == line_new);
+  }
+  __syncwarp();
+  clear_centre<NT>(a);
+  clear_centre<NT>(b);
+  const int kU = 2 * (ru * kLutW + cu), kV = 2 * (rv * kLutW + cv);
+  const uint32_t line_old = dir4_2(lut4, kV, kU);
+  find_centre<Num, NT>(W, lut4, hist, kU, a);
+  find_centre<Num, NT>(W, lut4, h1, kV, b);
+  __syncwarp();
+  const uint32_t part = count_centres<NT>(W, a, b);
+  __syncwarp();
+  const int joint = (int)counter_of(hist, line_old) - 1;
+  if (BAD) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) change[t] -= centre_get(a, t) + centre_get(b, t) - (b.e[t] == line_old);
+  }
+  const uint32_t sums = __reduce_add_sync(0xffffffffu, part);
+  const int bad_u = (int)(sums & 0xFFFu), bad_v = (int)(sums >> 12);
+  __syncwarp();
+  clear_centre<NT>(a);
+  clear_centre<NT>(b);
+  __syncwarp();
+  dE = p.ta + p.tb + p.j_new - (bad_u + bad_v - joint);
+  if (BAD) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      if (W.slot(t) == u) change[t] = p.ta + p.j_new - bad_u;
+      if (W.slot(t) == v) change[t] = p.tb + p.j_new - bad_v;
+    }
+  }
+  return !p.wide && bad_u < kMoveSum && bad_v < kMoveSum;
 }
 
 // The reference formulation (tempering.py:68-89), pair by pair.  Returns this
@@ -146,87 +181,91 @@ __device__ int swap_delta_pairs(const int* __restrict__ cs, int m, int u, int v,
   return delta;
 }
 
-constexpr int kDeltaWarps = 8;
-
-struct DeltaSmem {
-  static constexpr size_t lut_bytes = kFullLutBytes;  // the full signed direction table
-  static constexpr size_t bytes =
-      lut_bytes + sizeof(uint32_t) * kDirWords * kDeltaWarps + sizeof(int) * kMaxM * kDeltaWarps * 2;
+// Batched swap deltas: moves[mv] = (state, u, v), a warp each.  dE = N3_SENTINEL
+// for illegal moves or bad indices (then the badness changes are 0).
+struct MoveArgs {
+  const int16_t* cols;
+  const int32_t* moves;
+  int B, n, M;
+  const uint16_t* lut4;
+  int32_t* dE;
+  int32_t* dbad;  // [M][2n] or nullptr
 };
 
-__device__ __forceinline__ void load_lut_and_clear(unsigned char* smem, const uint16_t* __restrict__ g_lut,
-                                                   uint16_t*& lut, uint32_t*& hist_all, int*& cs_all, int*& aux_all) {
-  lut = reinterpret_cast<uint16_t*>(smem);
-  hist_all = reinterpret_cast<uint32_t*>(smem + DeltaSmem::lut_bytes);
-  cs_all = reinterpret_cast<int*>(hist_all + kDirWords * kDeltaWarps);
-  aux_all = cs_all + kMaxM * kDeltaWarps;
-  full_lut_copy(lut, g_lut);
-  for (int i = threadIdx.x; i < kDirWords * kDeltaWarps; i += blockDim.x) hist_all[i] = 0u;
-  __syncthreads();
+// The reference formulation.
+constexpr int kPairsWarps = 8;
+__global__ void __launch_bounds__(kPairsWarps * 32) swap_delta_pairs_kernel(const MoveArgs A) {
+  __shared__ int cs_all[kPairsWarps][kMaxM], db_all[kPairsWarps][kMaxM];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = 2 * A.n;
+  int *cs = cs_all[warp], *db = db_all[warp];
+  for (int mv = blockIdx.x * kPairsWarps + warp; mv < A.M; mv += gridDim.x * kPairsWarps) {
+    const int b = A.moves[3 * mv], u = A.moves[3 * mv + 1], v = A.moves[3 * mv + 2];
+    const bool in_range = b >= 0 && b < A.B && u >= 0 && u < m && v >= 0 && v < m;
+    if (in_range)
+      for (int s = lane; s < m; s += 32) cs[s] = A.cols[(size_t)b * m + s];
+    for (int s = lane; s < m; s += 32) db[s] = 0;
+    __syncwarp();
+    int d = N3_SENTINEL;
+    if (in_range && legal_swap(cs, u, v)) d = warp_sum(swap_delta_pairs(cs, m, u, v, lane, A.dbad ? db : nullptr));
+    __syncwarp();
+    if (A.dbad)
+      for (int s = lane; s < m; s += 32) A.dbad[(size_t)mv * m + s] = db[s];
+    if (lane == 0) A.dE[mv] = d;
+    __syncwarp();
+  }
 }
 
-// Batched swap deltas: moves[mv] = (state, u, v).  PAIRS selects the literal
-// reference formulation.  dE = N3_SENTINEL for illegal moves or bad indices.
-template <bool PAIRS>
-__global__ void __launch_bounds__(kDeltaWarps * 32) swap_delta_kernel(const int16_t* __restrict__ cols, int B, int n,
-                                                                        const int32_t* __restrict__ moves, int M,
-                                                                        const uint16_t* __restrict__ g_lut,
-                                                                        int32_t* __restrict__ dE,
-                                                                        int32_t* __restrict__ dbad) {
+// By direction histograms.  Shared-memory operations bound it: 20 table loads, 20
+// counts and 20 clears per move, 3 to 3.5 cycles each for 32 lanes at random (95 %
+// of the cycles).  65,536 moves of 4096 n = 75 states: 63 us, 77 us with four 8-bit
+// histograms one after the other; with badness changes 89 and 103 us.
+constexpr int kDeltaWarps = 30;
+constexpr size_t kDeltaSmem = kCompactLutBytes + sizeof(uint32_t) * 2 * DenseNumbering::kWords * kDeltaWarps;
+static_assert(kDeltaSmem <= 227 * 1024, "swap_delta_kernel shared memory");
+static_assert(2 * DenseNumbering::kWords >= kDirWords, "swap_delta_slow's counters");
+
+template <bool BAD, int NT>
+__global__ void __launch_bounds__(kDeltaWarps * 32, 1) swap_delta_kernel(const MoveArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  uint16_t* lut;
-  uint32_t* hist_all;
-  int *cs_all, *aux_all;
-  load_lut_and_clear(smem, g_lut, lut, hist_all, cs_all, aux_all);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = 2 * n;
-  int* cs = cs_all + warp * kMaxM;
-  int* db = aux_all + warp * kMaxM;
-  uint32_t* hist = hist_all + warp * kDirWords;
-  for (int mv = blockIdx.x * kDeltaWarps + warp; mv < M; mv += gridDim.x * kDeltaWarps) {
-    const int b = moves[3 * mv], u = moves[3 * mv + 1], v = moves[3 * mv + 2];
-    const bool in_range = b >= 0 && b < B && u >= 0 && u < m && v >= 0 && v < m;
-    int key[kSlotsPerLane];
+  uint16_t* lut4 = reinterpret_cast<uint16_t*>(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, m = 2 * A.n;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + kCompactLutBytes) + warp * 2 * DenseNumbering::kWords;
+  compact_lut_copy(lut4, A.lut4);
+  for (int i = lane; i < 2 * DenseNumbering::kWords; i += 32) hist[i] = 0u;
+  __syncthreads();
+  WarpState W;
+  W.m = m;
+  W.lane = lane;
+  W.cs = nullptr;
+  W.bs = nullptr;
+  for (int mv = blockIdx.x * warps + warp; mv < A.M; mv += gridDim.x * warps) {
+    const int b = A.moves[3 * mv], u = A.moves[3 * mv + 1], v = A.moves[3 * mv + 2];
+    int d = N3_SENTINEL, change[kSlotsPerLane];
 #pragma unroll
-    for (int t = 0; t < kSlotsPerLane; ++t) {  // this lane's slots and their table keys
-      const int k = lane + 32 * t;
-      const int c = in_range && k < m ? (int)cols[(size_t)b * m + k] : 0;
-      if (in_range && k < m) cs[k] = c;
-      key[t] = (k >> 1) * kLutW + c;
-    }
-    __syncwarp();
-    if (!in_range || !legal_swap(cs, u, v)) {
-      if (lane == 0) dE[mv] = N3_SENTINEL;
-      if (dbad)
-        for (int s = lane; s < m; s += 32) dbad[(size_t)mv * m + s] = 0;
-      __syncwarp();
-      continue;
-    }
-    int d;
-    if (PAIRS) {
-      if (dbad)
-        for (int s = lane; s < m; s += 32) db[s] = 0;
-      __syncwarp();
-      d = warp_sum(swap_delta_pairs(cs, m, u, v, lane, dbad ? db : nullptr));
-      __syncwarp();
-      if (dbad)
-        for (int s = lane; s < m; s += 32) dbad[(size_t)mv * m + s] = db[s];
-    } else {
-      int local[kSlotsPerLane];
-      int du = 0, dv = 0;
-      if (dbad) {
-        d = swap_delta_hist<true>(cs, key, m, u, v, lut, hist, lane, local, &du, &dv);
+    for (int t = 0; t < kSlotsPerLane; ++t) change[t] = 0;
+    if (b >= 0 && b < A.B && u >= 0 && u < m && v >= 0 && v < m) {  // uniform in the warp
+      const int16_t* cols = A.cols + (size_t)b * m;
 #pragma unroll
-        for (int t = 0; t < kSlotsPerLane; ++t) {
-          const int k = lane + 32 * t;
-          if (k < m) dbad[(size_t)mv * m + k] = k == u ? du : (k == v ? dv : local[t]);
-        }
-      } else {
-        d = swap_delta_hist<false>(cs, key, m, u, v, lut, hist, lane, local, &du, &dv);
+      for (int t = 0; t < kSlotsPerLane; ++t) {
+        const int k = W.slot(t);
+        W.key2[t] = t < NT && k < m ? 2 * ((k >> 1) * kLutW + cols[k]) : 0;
+      }
+      const int cu = cols[u], cv = cols[v], pu = cols[u ^ 1], pv = cols[v ^ 1];
+      if ((u >> 1) != (v >> 1) && cu != cv && pu != cv && pv != cu) {  // uniform
+        // a cell held twice has no direction to itself
+        const bool twin = pu == cu || pv == cv;
+        if (twin || !swap_delta_pair<BAD, NT>(W, u, v, cu, cv, lut4, hist, d, change))
+          d = swap_delta_slow<BAD>(W.key2, m, lane, u, v, cu, cv, lut4, hist, change);
       }
     }
-    if (lane == 0) dE[mv] = d;
-    __syncwarp();
+    if (BAD) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int k = W.slot(t);
+        if (k < m) A.dbad[(size_t)mv * m + k] = change[t];
+      }
+    }
+    if (lane == 0) A.dE[mv] = d;
   }
 }
 
@@ -455,13 +494,27 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
 namespace n3host {
 
 template <class K>
-static int prepare(K kernel, size_t bytes = n3::DeltaSmem::bytes) {
+static int prepare(K kernel, size_t bytes) {
   return allow_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
+// swap_delta_kernel for 2n slots, NT = ceil(2n / 32) a lane.
+static void (*delta_kernel(bool bad, int n))(const n3::MoveArgs) {
+  using namespace n3;
+  switch ((2 * n + 31) / 32) {
+    case 5: return bad ? swap_delta_kernel<true, 5> : swap_delta_kernel<false, 5>;
+    case 4: return bad ? swap_delta_kernel<true, 4> : swap_delta_kernel<false, 4>;
+    case 3: return bad ? swap_delta_kernel<true, 3> : swap_delta_kernel<false, 3>;
+    case 2: return bad ? swap_delta_kernel<true, 2> : swap_delta_kernel<false, 2>;
+    default: return bad ? swap_delta_kernel<true, 1> : swap_delta_kernel<false, 1>;
+  }
+}
+
 int prepare_delta() {
-  N3_TRY(prepare(n3::swap_delta_kernel<true>));
-  N3_TRY(prepare(n3::swap_delta_kernel<false>));
+  for (int n = 16; n <= 80; n += 16) {
+    N3_TRY(prepare(delta_kernel(true, n), n3::kDeltaSmem));
+    N3_TRY(prepare(delta_kernel(false, n), n3::kDeltaSmem));
+  }
   N3_TRY(prepare(n3::partner_scores_kernel<true>, sizeof(n3::PartnerSmem)));
   return prepare(n3::partner_scores_kernel<false>, sizeof(n3::PartnerSmem));
 }
@@ -480,18 +533,20 @@ static int launch_swap(bool pairs, const int16_t* cols, int B, int n, const int3
   if (M == 0) return N3_OK;
   if (moves == nullptr || dE == nullptr) return set_error(N3_ERR_ARG, "null move or output pointer");
   N3_TRY(ensure_device_tables());
-  const uint16_t* lut = dir_lut_full_device_ptr();
-  const int want = (M + n3::kDeltaWarps - 1) / n3::kDeltaWarps;
-  const int grid = want < sm_count() * 2 ? want : sm_count() * 2;
+  const n3::MoveArgs A = {cols, moves, B, n, M, dir4_lut_device_ptr(), dE, dbad};
+  const int sms = sm_count();
   if (pairs) {
-    N3_TRY(prepare(n3::swap_delta_kernel<true>));
-    n3::swap_delta_kernel<true><<<grid, n3::kDeltaWarps * 32, n3::DeltaSmem::bytes, st>>>(cols, B, n, moves, M, lut,
-                                                                                          dE, dbad);
-  } else {
-    N3_TRY(prepare(n3::swap_delta_kernel<false>));
-    n3::swap_delta_kernel<false><<<grid, n3::kDeltaWarps * 32, n3::DeltaSmem::bytes, st>>>(cols, B, n, moves, M, lut,
-                                                                                           dE, dbad);
+    const int want = (M + n3::kPairsWarps - 1) / n3::kPairsWarps;
+    n3::swap_delta_pairs_kernel<<<want < 8 * sms ? want : 8 * sms, n3::kPairsWarps * 32, 0, st>>>(A);
+    return check_launch("swap_delta_pairs_kernel");
   }
+  // One CTA per SM; fewer warps in each for few moves, but enough to copy the table.
+  int warps = (M + sms - 1) / sms;
+  warps = warps < 8 ? 8 : (warps > n3::kDeltaWarps ? n3::kDeltaWarps : warps);
+  const int want = (M + warps - 1) / warps;
+  const auto kernel = delta_kernel(dbad != nullptr, n);
+  N3_TRY(prepare(kernel, n3::kDeltaSmem));
+  kernel<<<want < sms ? want : sms, warps * 32, n3::kDeltaSmem, st>>>(A);
   return check_launch("swap_delta_kernel");
 }
 

@@ -215,13 +215,13 @@ __device__ __forceinline__ bool call_slow_move(WarpState& W, const uint16_t* __r
 struct PairCount {
   int ta, tb;    // t(u'), t(v') over A
   int j_new;     // points of A on the line (u', v')
-  int joint;     // points of A on the line (u, v)
+  int joint;     // points of A on the line (u, v) (JOINT)
   bool wide;     // a counter may have wrapped: the rest is not to be used
 };
 
 // Counts them into hist (two zero histograms of Num::kWords words each) and leaves
 // the centres' directions in a and b: the caller clears those words.
-template <class Num, int NT>
+template <class Num, int NT, bool JOINT = true>
 __device__ __forceinline__ PairCount count_pair(const WarpState& W, const uint16_t* __restrict__ lut4,
                                                 uint32_t* __restrict__ hist, int ru, int rv, int cu, int cv,
                                                 Directions& a, Directions& b, uint32_t& line_new) {
@@ -232,7 +232,8 @@ __device__ __forceinline__ PairCount count_pair(const WarpState& W, const uint16
   find_centre<Num, NT>(W, lut4, h0, kA, a);
   find_centre<Num, NT>(W, lut4, h1, kB, b);
   // pair sums in 12 bits each, the points on the line (u, v), both included, in the top byte
-  const uint32_t part = count_centres<NT>(W, a, b) + ((uint32_t)W.on_line<NT>(ru, cu, rv - ru, cv - cu) << 24);
+  uint32_t part = count_centres<NT>(W, a, b);
+  if (JOINT) part += (uint32_t)W.on_line<NT>(ru, cu, rv - ru, cv - cu) << 24;
   __syncwarp();
   PairCount p;
   p.j_new = (int)counter_of(h0, line_new);
