@@ -22,9 +22,9 @@
 // both on tcgen05 with fp32 accumulators in tensor memory.
 // Training uses MSE on dE / kTargetScale with Adam: the five GEMMs of a step
 // (two forward layers, two weight gradients, the backward through layer 2) run
-// on tcgen05 with bf16 operands and fp32 accumulators (tc_gemm_kernel), the
-// head, bias gradients and Adam in fp32 SIMT; the packed bf16 images are
-// rebuilt after each update.  fp32 master weights.
+// on tcgen05 with bf16 operands and fp32 accumulators (tc_tile), the head, bias
+// gradients and Adam in fp32 SIMT; each update writes the packed bf16 images too.
+// fp32 master weights.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <mutex>
@@ -703,25 +703,26 @@ struct Batch {
 
 // Draws batch row b from the first `filled` ring slots, filled =
 // min(capacity, steps recorded * chains); the draw is keyed by the training
-// step counter.
-__global__ void gather_kernel(const uint16_t* __restrict__ rb_feat, const uint8_t* __restrict__ rb_bad,
-                              const int16_t* __restrict__ rb_dE, const uint64_t* __restrict__ counters,
-                              int64_t capacity, int n_chains, int B, uint32_t k0, uint32_t k1, float* __restrict__ X,
-                              float* __restrict__ y) {
-  const int b = blockIdx.x;
-  __shared__ int64_t slot_s;
-  if (threadIdx.x == 0) {
-    const uint64_t steps = counters[0], t = counters[1];
-    const uint64_t recorded = steps * (uint64_t)n_chains;
-    const uint64_t filled = recorded < (uint64_t)capacity ? (recorded ? recorded : 1) : (uint64_t)capacity;
-    const U4 r = philox4x32_10(U4{(uint32_t)t, (uint32_t)(t >> 32), (uint32_t)b, 0x7A000000u}, k0, k1);
-    const uint64_t x = ((uint64_t)r.x << 32) | r.y;
-    slot_s = (int64_t)(x % filled);
-    y[b] = (float)rb_dE[slot_s] / kTargetScale;
-  }
-  __syncthreads();
-  const int64_t s = slot_s;
-  for (int k = threadIdx.x; k < kIn; k += blockDim.x) {
+// step counter.  A warp per row.  The launch also clears what the step adds into:
+// the gradient, and at `loss` the loss and update_kernel's count of blocks.
+constexpr int kGatherRows = 8;
+__global__ void __launch_bounds__(kGatherRows * 32) gather_kernel(
+    const uint16_t* __restrict__ rb_feat, const uint8_t* __restrict__ rb_bad, const int16_t* __restrict__ rb_dE,
+    const uint64_t* __restrict__ counters, int64_t capacity, int n_chains, int B, uint32_t k0, uint32_t k1,
+    float* __restrict__ X, float* __restrict__ y, float* __restrict__ grads, float* __restrict__ loss) {
+  const int lane = threadIdx.x & 31, b = blockIdx.x * kGatherRows + (threadIdx.x >> 5);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) grads[i] = 0.f;
+  if (blockIdx.x == 0 && threadIdx.x < 2) loss[threadIdx.x] = 0.f;
+  if (b >= B) return;
+  const uint64_t steps = counters[0], t = counters[1];
+  const uint64_t recorded = steps * (uint64_t)n_chains;
+  const uint64_t filled = recorded < (uint64_t)capacity ? (recorded ? recorded : 1) : (uint64_t)capacity;
+  const U4 r = philox4x32_10(U4{(uint32_t)t, (uint32_t)(t >> 32), (uint32_t)b, 0x7A000000u}, k0, k1);
+  const int64_t s = (int64_t)((((uint64_t)r.x << 32) | r.y) % filled);
+  if (lane == 0) y[b] = (float)rb_dE[s] / kTargetScale;
+#pragma unroll
+  for (int j = 0; j < kIn / 32; ++j) {
+    const int k = lane + 32 * j;
     float v = 0.f;
     if (k < kCandFeat) {
       const uint16_t h = rb_feat[s * kCandFeat + k];
@@ -733,80 +734,101 @@ __global__ void gather_kernel(const uint16_t* __restrict__ rb_feat, const uint8_
   }
 }
 
-
-// out = H2 . w3 + b3, d = 2 (out - y) / B, dZ2 = d w3 (Z2 > 0), loss += (out - y)^2
 // GEMMs on the tensor cores (tcgen05, kind::f16): C (M x N, fp32) =
 // sum_k A(m, k) B(k, n) for fp32 operands given by element strides (A(m, k) at
-// A[m sam + k sak], B(k, n) at Bm[k sbk + n sbn]), with the epilogues of the
-// training step: EPI 0 store (or add, with a K split over gridDim.z: the
+// A[m sam + k sak], B(k, n) at B[k sbk + n sbn]), with the epilogues of the
+// training step: EPI 0 store (or add, with a K split over several CTAs: the
 // weight gradients), EPI 1 Z = acc + bias, H = relu(Z) (the forward layers),
-// EPI 2 acc masked by Z > 0 (back through a ReLU); and EPI 3 acc + bias (the
-// chain part of layer 1 before inference).
+// EPI 2 acc masked by Z > 0 (back through a ReLU) and its column sums added to
+// `sums`; and EPI 3 acc + bias (the chain part of layer 1 before inference).
 //
-// A CTA of 4 warps owns a 128 x kTcN output tile.  Per K slice of 64 it rounds
+// A CTA of 8 warps owns a 128 x kTcN output tile.  Per K slice of 64 it rounds
 // the operands to bf16 while staging them into 128B-swizzled K-major shared
 // tiles (two buffers: the next slice is staged while the tensor core reads the
 // current one), thread 0 issues the slice's four K = 16 MMAs into a 128 x kTcN
 // fp32 accumulator in tensor memory and commits them to the buffer's mbarrier,
 // and the epilogue reads the accumulator back with tcgen05.ld (warp w: rows
-// 32 w .. 32 w + 31).  Every mbarrier wait is bounded; an expired wait sets
-// error bit 8 and skips the epilogue.
+// 32 (w % 4) .. + 31, columns 32 (w / 4) .. + 31).  Every mbarrier wait is bounded;
+// an expired wait sets error bit 8 and skips the epilogue.
+//
+// The products are small (0.4 to 0.5 GFLOP), so staging latency bounds them:
+// a thread rounds eight values along K into one 16-byte store, and its loads are
+// all in flight before the first conversion.
 constexpr int kTcN = 64;                            // output columns per CTA (tensor-memory columns)
+constexpr int kTcThreads = 256;
 constexpr uint32_t kTcA = 128 * 128;                // bytes of one A slice (128 rows x 64 bf16)
 constexpr uint32_t kTcB = kTcN * 128;               // bytes of one B slice
 constexpr uint32_t kTcBar = 2 * (kTcA + kTcB);      // two mbarriers and the tensor-memory address
 constexpr uint32_t kTcSmem = kTcBar + 64 + 1024;    // + alignment slack
 
+struct GemmArgs {
+  int M, N, K;
+  const float* A;
+  int sam, sak;
+  const float* B;
+  int sbk, sbn;
+  float* C;
+  int ldc;
+  const float* bias;
+  float* aux;
+  float* sums;
+};
+
 // Stages ROWS x 64 elements of an operand, element (r, k) at src[(r0 + r) sr + (k0 + k) sk],
-// zero outside r0 + r < R, k0 + k < Ke, into an SW128 K-major bf16 tile.  All
-// of a thread's loads are issued before any conversion (a fixed count per
-// thread, in registers), so their latencies overlap.
+// zero outside r0 + r < R, k0 + k < Ke, into an SW128 K-major bf16 tile.
 template <int ROWS>
 __device__ __forceinline__ void tc_stage(uint8_t* tile, const float* __restrict__ src, int sr, int sk, int r0, int R,
                                          int k0, int Ke, int tid) {
-  constexpr int kPer = ROWS * 64 / 128;  // elements per thread
-  float v[kPer];
-  if (sk == 1) {  // k contiguous: a warp reads 64 consecutive floats (two per lane) of one row
+  constexpr int kChunks = ROWS * 8 / kTcThreads;  // 16-byte chunks (8 elements) per thread
+  float v[kChunks][8];
+  // uniform; the training scratch and the chain rows are only 8-byte aligned for some sizes
+  const bool whole = sk == 1 && k0 + 64 <= Ke;
+  const bool vec = whole && ((reinterpret_cast<uintptr_t>(src) & 15u) | (sr & 3)) == 0;
+  const bool vec2 = whole && ((reinterpret_cast<uintptr_t>(src) & 7u) | (sr & 1)) == 0;
+  const bool by_rows = sk != 1;  // consecutive rows contiguous (or neither): the lanes take rows
 #pragma unroll
-    for (int e = 0; e < kPer / 2; ++e) {
-      const int i = tid + 128 * e, r = i >> 5, k = 2 * (i & 31);
-      const bool rin = r0 + r < R;
-      const float* q = src + (size_t)(r0 + r) * sr + (k0 + k);
-      v[2 * e] = rin && k0 + k < Ke ? __ldg(q) : 0.f;
-      v[2 * e + 1] = rin && k0 + k + 1 < Ke ? __ldg(q + 1) : 0.f;
-    }
+  for (int e = 0; e < kChunks; ++e) {
+    const int i = tid + kTcThreads * e;
+    const int r = by_rows ? i % ROWS : i >> 3, c = by_rows ? i / ROWS : i & 7;
+    const bool rin = r0 + r < R;
+    const float* q = src + (size_t)(r0 + r) * sr + (size_t)(k0 + 8 * c) * sk;
+    if (vec) {
+      const float4 lo = rin ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 hi = rin ? __ldg(reinterpret_cast<const float4*>(q) + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[e][0] = lo.x, v[e][1] = lo.y, v[e][2] = lo.z, v[e][3] = lo.w;
+      v[e][4] = hi.x, v[e][5] = hi.y, v[e][6] = hi.z, v[e][7] = hi.w;
+    } else if (vec2) {
 #pragma unroll
-    for (int e = 0; e < kPer / 2; ++e) {
-      const int i = tid + 128 * e, r = i >> 5, k = 2 * (i & 31);
-      *reinterpret_cast<uint32_t*>(tile + umma::sw128_offset(r, k, ROWS)) = bf16x2_bits(v[2 * e], v[2 * e + 1]);
-    }
-  } else {  // rows contiguous (or neither): a warp reads 32 consecutive rows of one k
+      for (int j = 0; j < 4; ++j) {
+        const float2 two = rin ? __ldg(reinterpret_cast<const float2*>(q) + j) : make_float2(0.f, 0.f);
+        v[e][2 * j] = two.x, v[e][2 * j + 1] = two.y;
+      }
+    } else {
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-      const int i = tid + 128 * e, k = i / ROWS, r = i % ROWS;
-      v[e] = r0 + r < R && k0 + k < Ke ? __ldg(src + (size_t)(r0 + r) * sr + (size_t)(k0 + k) * sk) : 0.f;
+      for (int j = 0; j < 8; ++j) v[e][j] = rin && k0 + 8 * c + j < Ke ? __ldg(q + (size_t)j * sk) : 0.f;
     }
+  }
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-      const int i = tid + 128 * e, k = i / ROWS, r = i % ROWS;
-      *reinterpret_cast<uint16_t*>(tile + umma::sw128_offset(r, k, ROWS)) = bf16_bits(v[e]);
-    }
+  for (int e = 0; e < kChunks; ++e) {
+    const int i = tid + kTcThreads * e;
+    const int r = by_rows ? i % ROWS : i >> 3, c = by_rows ? i / ROWS : i & 7;
+    *reinterpret_cast<uint4*>(tile + umma::sw128_offset(r, 8 * c, ROWS)) =
+        make_uint4(bf16x2_bits(v[e][0], v[e][1]), bf16x2_bits(v[e][2], v[e][3]), bf16x2_bits(v[e][4], v[e][5]),
+                   bf16x2_bits(v[e][6], v[e][7]));
   }
 }
 
+// The tile of columns n0 .., rows m0 .., from K split `split` of `splits`.
 template <int EPI>
-__global__ void __launch_bounds__(128) tc_gemm_kernel(int M, int N, int K, const float* __restrict__ A, int sam,
-                                                      int sak, const float* __restrict__ Bm, int sbk, int sbn,
-                                                      float* __restrict__ C, int ldc, const float* __restrict__ bias,
-                                                      float* __restrict__ aux, uint32_t* error_word) {
+__device__ __forceinline__ void tc_tile(const GemmArgs& G, int n0, int m0, int split, int splits,
+                                        uint32_t* error_word) {
   extern __shared__ __align__(16) uint8_t tc_smem[];
   const uint32_t raw = umma::smem_addr(tc_smem);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* sm = tc_smem + (base - raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * 128, n0 = blockIdx.x * kTcN;
-  const int kchunk = ((K + (int)gridDim.z - 1) / (int)gridDim.z + 63) / 64 * 64;
-  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
+  const int kchunk = ((G.K + splits - 1) / splits + 63) / 64 * 64;
+  const int kb = split * kchunk, ke = min(G.K, kb + kchunk);
   const int slices = kb < ke ? (ke - kb + 63) / 64 : 0;
   if (slices == 0) return;  // a K split with nothing to add (uniform across the CTA)
   const uint32_t bar0 = base + kTcBar, bar1 = bar0 + 8, taddr_slot = bar0 + 16;
@@ -833,8 +855,8 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(int M, int N, int K, const
     uint8_t* ta = sm + buf * (kTcA + kTcB);
     uint8_t* tb = ta + kTcA;
     const int k0 = kb + 64 * s;
-    tc_stage<128>(ta, A, sam, sak, m0, M, k0, ke, tid);
-    tc_stage<kTcN>(tb, Bm, sbn, sbk, n0, N, k0, ke, tid);
+    tc_stage<128>(ta, G.A, G.sam, G.sak, m0, G.M, k0, ke, tid);
+    tc_stage<kTcN>(tb, G.B, G.sbn, G.sbk, n0, G.N, k0, ke, tid);
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
@@ -854,40 +876,42 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(int M, int N, int K, const
   ok = __syncthreads_and(ok);
   umma::fence_after_sync();
   if (ok) {
-    // Each thread reads its row's 32 columns of a chunk from tensor memory; the
-    // warp's 32 x 32 block goes through shared memory (the staging tiles are
-    // free now) so that each store instruction writes one row's 32 columns.
+    // Each thread reads its row's 32 columns from tensor memory; the warp's
+    // 32 x 32 block goes through shared memory (the staging tiles are free now) so
+    // that each store instruction writes one row's 32 columns.
     float* blk = reinterpret_cast<float*>(sm) + warp * (32 * 33);
-#pragma unroll 1
-    for (int c0 = 0; c0 < kTcN; c0 += 32) {
-      float v[32];
-      umma::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+    const int quarter = warp & 3, c0 = 32 * (warp >> 2);
+    float v[32];
+    umma::tmem_ld32(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)c0, v);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) blk[lane * 33 + j] = v[j];
-      __syncwarp();
-      const int nn = n0 + c0 + lane;
-#pragma unroll 4
-      for (int rr = 0; rr < 32; ++rr) {
-        const int row = m0 + 32 * warp + rr;
-        if (row >= M || nn >= N) continue;
+    for (int j = 0; j < 32; ++j) blk[lane * 33 + j] = v[j];
+    __syncwarp();
+    const int nn = n0 + c0 + lane, row0 = m0 + 32 * quarter, rows = min(32, G.M - row0);
+    if (nn < G.N && rows > 0) {
+      const float bias = EPI == 1 || EPI == 3 ? G.bias[nn] : 0.f;
+      float sum = 0.f;
+#pragma unroll 8
+      for (int rr = 0; rr < rows; ++rr) {
         const float x = blk[rr * 33 + lane];
-        const size_t o = (size_t)row * ldc + nn;
+        const size_t o = (size_t)(row0 + rr) * G.ldc + nn;
         if (EPI == 0) {
-          if (gridDim.z > 1)
-            atomicAdd(C + o, x);
+          if (splits > 1)
+            atomicAdd(G.C + o, x);
           else
-            C[o] = x;
+            G.C[o] = x;
         } else if (EPI == 1) {
-          const float z = x + bias[nn];
-          aux[o] = z;
-          C[o] = fmaxf(z, 0.f);
+          const float z = x + bias;
+          G.aux[o] = z;
+          G.C[o] = fmaxf(z, 0.f);
         } else if (EPI == 3) {
-          C[o] = x + bias[nn];
+          G.C[o] = x + bias;
         } else {
-          C[o] = aux[o] > 0.f ? x : 0.f;
+          const float dz = G.aux[o] > 0.f ? x : 0.f;
+          G.C[o] = dz;
+          sum += dz;
         }
       }
-      __syncwarp();
+      if (EPI == 2) atomicAdd(G.sums + nn, sum);
     }
   } else if (tid == 0 && error_word) {
     atomicOr(error_word, kErrTimeout);
@@ -897,68 +921,135 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(int M, int N, int K, const
   if (warp == 0) umma::tmem_dealloc(tmem, kTcN);
 }
 
-__global__ void head_kernel(int B, const float* __restrict__ H2, const float* __restrict__ Z2,
-                            const float* __restrict__ P, const float* __restrict__ y, float* __restrict__ d,
-                            float* __restrict__ dZ2, float* __restrict__ loss) {
-  const int b = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (b >= B) return;
-  float acc = 0.f;
-  for (int k = lane; k < kH; k += 32) acc = fmaf(H2[(size_t)b * kH + k], P[oW3 + k], acc);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  const float out = acc + P[oB3];
-  const float e = out - y[b];
-  const float g = 2.f * e / (float)B;
-  if (lane == 0) {
-    d[b] = g;
-    atomicAdd(loss, e * e);
+template <int EPI>
+__global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const GemmArgs G, uint32_t* error_word) {
+  tc_tile<EPI>(G, blockIdx.x * kTcN, blockIdx.y * 128, blockIdx.z, gridDim.z, error_word);
+}
+
+// dZ1 (EPI 2, its tiles first) and layer 2's weight gradient (EPI 0, kH x kH), which
+// wait for the same kernel, in one launch.
+__global__ void __launch_bounds__(kTcThreads) tc_back_kernel(const GemmArgs Z, const GemmArgs W, int z_tiles, int splits,
+                                                             uint32_t* error_word) {
+  constexpr int kN = kH / kTcN;
+  const int t = blockIdx.x;
+  if (t < z_tiles) {
+    tc_tile<2>(Z, (t % kN) * kTcN, (t / kN) * 128, 0, 1, error_word);
+  } else {
+    const int w = t - z_tiles;
+    tc_tile<0>(W, (w % kN) * kTcN, (w / kN % (kH / 128)) * 128, w / (kN * (kH / 128)), splits, error_word);
   }
-  for (int k = lane; k < kH; k += 32) dZ2[(size_t)b * kH + k] = Z2[(size_t)b * kH + k] > 0.f ? g * P[oW3 + k] : 0.f;
 }
 
-// Column sums added into a zeroed `out`: out[n] += sum_b M[b][n] (* scale[b]).
-// Block (x, y) sums rows [y * kColRows, ...) of columns x * blockDim.x + t.
-constexpr int kColRows = 128;
-__global__ void colsum_kernel(int B, int N, const float* __restrict__ Mx, const float* __restrict__ scale,
-                              float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const int b0 = blockIdx.y * kColRows, b1 = min(B, b0 + kColRows);
-  float acc = 0.f;
-  for (int b = b0; b < b1; ++b) acc = fmaf(Mx[(size_t)b * N + n], scale ? scale[b] : 1.f, acc);
-  atomicAdd(out + n, acc);
-}
-
-__global__ void sum_kernel(int B, const float* __restrict__ v, float* __restrict__ out) {
-  float acc = 0.f;
-  for (int b = threadIdx.x; b < B; b += blockDim.x) acc += v[b];
+// out = H2 . w3 + b3, d = 2 (out - y) / B, dZ2 = d w3 (Z2 > 0), and the sums over
+// the batch: loss += (out - y)^2, gradients of w3 (d H2), b3 (d) and b2 (dZ2).  H2 is
+// relu(Z2).  A warp takes every (warps)-th row, lane l columns l, l + 32, ...; its
+// sums stay in registers to the end, so each block adds once per column.  (One
+// addition to the loss per row cost 12 us for 4096 rows, a pass per column
+// sum 12 to 20 us.)
+constexpr int kHeadWarps = 8;
+__global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const float* __restrict__ Z2,
+                                                               const float* __restrict__ P,
+                                                               const float* __restrict__ y, float* __restrict__ d,
+                                                               float* __restrict__ dZ2, float* __restrict__ grads,
+                                                               float* __restrict__ loss) {
+  constexpr int kC = kH / 32;
+  __shared__ float s_w3[kHeadWarps][kH], s_b2[kHeadWarps][kH], s_loss[kHeadWarps], s_b3[kHeadWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float w3[kC], g_w3[kC], g_b2[kC], loss_sum = 0.f, b3_sum = 0.f;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  __shared__ float part[32];
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x / 32] = acc;
+  for (int j = 0; j < kC; ++j) {
+    w3[j] = P[oW3 + lane + 32 * j];
+    g_w3[j] = g_b2[j] = 0.f;
+  }
+  const float b3 = P[oB3];
+  for (int b = blockIdx.x * kHeadWarps + warp; b < B; b += gridDim.x * kHeadWarps) {
+    float z[kC], acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < kC; ++j) z[j] = Z2[(size_t)b * kH + lane + 32 * j];
+#pragma unroll
+    for (int j = 0; j < kC; ++j) acc = fmaf(fmaxf(z[j], 0.f), w3[j], acc);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const float out = acc + b3;
+    const float e = out - y[b];
+    const float g = 2.f * e / (float)B;
+    if (lane == 0) d[b] = g;
+    loss_sum += e * e;
+    b3_sum += g;
+#pragma unroll
+    for (int j = 0; j < kC; ++j) {
+      const float dz = z[j] > 0.f ? g * w3[j] : 0.f;
+      dZ2[(size_t)b * kH + lane + 32 * j] = dz;
+      g_b2[j] += dz;
+      g_w3[j] = fmaf(fmaxf(z[j], 0.f), g, g_w3[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kC; ++j) {
+    s_w3[warp][lane + 32 * j] = g_w3[j];
+    s_b2[warp][lane + 32 * j] = g_b2[j];
+  }
+  if (lane == 0) {
+    s_loss[warp] = loss_sum;
+    s_b3[warp] = b3_sum;
+  }
   __syncthreads();
+  for (int n = threadIdx.x; n < kH; n += blockDim.x) {
+    float a = 0.f, c = 0.f;
+#pragma unroll
+    for (int w = 0; w < kHeadWarps; ++w) {
+      a += s_w3[w][n];
+      c += s_b2[w][n];
+    }
+    atomicAdd(grads + oW3 + n, a);
+    atomicAdd(grads + oB2 + n, c);
+  }
   if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int i = 0; i < (int)(blockDim.x / 32); ++i) t += part[i];
-    *out = t;
+    float a = 0.f, c = 0.f;
+    for (int w = 0; w < kHeadWarps; ++w) {
+      a += s_loss[w];
+      c += s_b3[w];
+    }
+    atomicAdd(loss, a);
+    atomicAdd(grads + oB3, c);
   }
 }
 
 // Adam (Kingma & Ba) with bias correction; the step number is counters[1] + 1.
-__global__ void adam_kernel(int count, float* __restrict__ P, const float* __restrict__ G, float* __restrict__ Mo,
-                            float* __restrict__ V, float lr, float b1, float b2, float eps,
-                            const uint64_t* __restrict__ counters) {
+// Each new weight also goes into the tensor-core images (as pack_kernel puts it),
+// and the last block to finish advances the counter and hands the loss out.  done: 0.
+__global__ void update_kernel(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ Mo,
+                              float* __restrict__ V, float lr, float b1, float b2, float eps, uint64_t* counters,
+                              uint8_t* __restrict__ w2_img, uint8_t* __restrict__ w1a_img, const float* loss,
+                              float* loss_out, uint32_t* done) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const float t = (float)(counters[1] + 1);
-  const float c1 = 1.f - powf(b1, t), c2 = 1.f - powf(b2, t);
-  const float g = G[i];
-  const float m = b1 * Mo[i] + (1.f - b1) * g;
-  const float v = b2 * V[i] + (1.f - b2) * g * g;
-  Mo[i] = m;
-  V[i] = v;
-  P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+  if (i < kParams) {
+    const float t = (float)(*(volatile uint64_t*)(counters + 1) + 1);
+    const float c1 = 1.f - powf(b1, t), c2 = 1.f - powf(b2, t);
+    const float g = G[i];
+    const float m = b1 * Mo[i] + (1.f - b1) * g;
+    const float v = b2 * V[i] + (1.f - b2) * g * g;
+    Mo[i] = m;
+    V[i] = v;
+    const float w = P[i] - lr * (m / c1) / (sqrtf(v / c2) + eps);
+    P[i] = w;
+    if (i >= oW2 && i < oB2) {
+      const int n = (i - oW2) / kH, k = (i - oW2) % kH;
+      *reinterpret_cast<uint16_t*>(w2_img + umma::sw128_offset(n, k, kH)) = bf16_bits(w);
+    } else if (i < oB1) {
+      const int n = i / kIn, k = i % kIn;
+      if (k < 16)
+        *reinterpret_cast<uint16_t*>(w1a_img + umma::inter16_offset(n, k)) = bf16_bits(k < kCandFeat ? w : 0.0f);
+    }
+  }
+  __syncthreads();  // every thread has read the counter
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(done, 1u) == gridDim.x - 1u) {
+      counters[1] += 1;
+      if (loss_out) *loss_out = *loss;
+    }
+  }
 }
 
 __global__ void bump_kernel(uint64_t* counters, int which) { counters[which] += 1; }
@@ -988,9 +1079,11 @@ int prepare_mlp() {
 namespace n3host {
 
 // One training step: gather a batch from the ring buffer, forward, backward,
-// Adam, repack the tensor-core weight images.  `scratch` holds the batch
+// Adam with the tensor-core weight images.  `scratch` holds the batch
 // activations (n3_mlp_scratch_floats(batch) floats), `grads` the gradient
-// (kParams floats); both entry points below call this body.
+// (kParams floats); both entry points below call this body.  Seven launches, each
+// waiting for the one before, bound it: a batch of 4096 takes 70 us, 154 us in
+// 17 launches with passes of their own for the sums, the counter and the images.
 static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t seed, float* scratch, float* grads,
                       float* adam_m, float* adam_v, cudaStream_t st) {
   using namespace n3::mlp;
@@ -1005,47 +1098,38 @@ static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t s
   float* dZ1 = dZ2 + (size_t)B * kH;
   float* loss = dZ1 + (size_t)B * kH;
   float* P = M->params;
-  // the gradient and the loss are accumulated: clear them first
-  if (cudaMemsetAsync(grads, 0, sizeof(float) * kParams, st) != cudaSuccess ||
-      cudaMemsetAsync(loss, 0, sizeof(float), st) != cudaSuccess)
-    return check_launch("MLP training: clearing the gradient");
-  gather_kernel<<<B, 64, 0, st>>>(M->rb_feat, M->rb_bad, M->rb_dE, M->counters, M->rb_capacity, n_chains, B,
-                                  (uint32_t)seed, (uint32_t)(seed >> 32), X, y);
-  // tensor-core GEMMs (tc_gemm_kernel): 128-row tiles of kTcN columns; the
-  // weight gradients split K = batch over up to 16 CTAs per tile
+  gather_kernel<<<(B + kGatherRows - 1) / kGatherRows, kGatherRows * 32, 0, st>>>(
+      M->rb_feat, M->rb_bad, M->rb_dE, M->counters, M->rb_capacity, n_chains, B, (uint32_t)seed, (uint32_t)(seed >> 32),
+      X, y, grads, loss);
+  // tensor-core GEMMs (tc_tile): 128-row tiles of kTcN columns; the weight
+  // gradients split K = batch over up to 16 CTAs per tile
   N3_TRY(allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<0>), kTcSmem));
   N3_TRY(allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<1>), kTcSmem));
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<2>), kTcSmem));
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(tc_back_kernel), kTcSmem));
   const int row_tiles = (B + 127) / 128;
   const int splits = B >= 4096 ? 16 : B >= 512 ? B / 256 : 1;
   uint32_t* ew = M->error_word;
   // Z1 = X W1^T + b1 ; H1 = relu(Z1)     (W1 [256][192]: B(k, n) = W1[n*192 + k])
-  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), 128, kTcSmem, st>>>(B, kH, kIn, X, kIn, 1, P + oW1, 1, kIn,
-                                                                          H1, kH, P + oB1, Z1, ew);
-  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), 128, kTcSmem, st>>>(B, kH, kH, H1, kH, 1, P + oW2, 1, kH,
-                                                                          H2, kH, P + oB2, Z2, ew);
-  head_kernel<<<(B + 7) / 8, 256, 0, st>>>(B, H2, Z2, P, y, d, dZ2, loss);
-  // gradients of the head and layer 2
-  colsum_kernel<<<dim3((kH + 127) / 128, (B + kColRows - 1) / kColRows), 128, 0, st>>>(B, kH, H2, d, grads + oW3);
-  sum_kernel<<<1, 1024, 0, st>>>(B, d, grads + oB3);
+  const GemmArgs l1 = {B, kH, kIn, X, kIn, 1, P + oW1, 1, kIn, H1, kH, P + oB1, Z1, nullptr};
+  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st>>>(l1, ew);
+  const GemmArgs l2 = {B, kH, kH, H1, kH, 1, P + oW2, 1, kH, H2, kH, P + oB2, Z2, nullptr};
+  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st>>>(l2, ew);
+  const int head_blocks = (B + kHeadWarps - 1) / kHeadWarps;
+  head_kernel<<<head_blocks < sm_count() ? head_blocks : sm_count(), kHeadWarps * 32, 0, st>>>(B, Z2, P, y, d, dZ2,
+                                                                                               grads, loss);
+  // dZ1 = (dZ2 W2) * (Z1 > 0)            (B(k, n) = W2[k*256 + n]), and b1's gradient
+  const GemmArgs z1 = {B, kH, kH, dZ2, kH, 1, P + oW2, kH, 1, dZ1, kH, nullptr, Z1, grads + oB1};
   // gW2[n][k] = sum_b dZ2[b][n] H1[b][k]
-  tc_gemm_kernel<0><<<dim3(kH / kTcN, kH / 128, splits), 128, kTcSmem, st>>>(kH, kH, B, dZ2, 1, kH, H1, kH, 1,
-                                                                              grads + oW2, kH, nullptr, nullptr, ew);
-  colsum_kernel<<<dim3((kH + 127) / 128, (B + kColRows - 1) / kColRows), 128, 0, st>>>(B, kH, dZ2, nullptr, grads + oB2);
-  // dZ1 = (dZ2 W2) * (Z1 > 0)            (B(k, n) = W2[k*256 + n])
-  tc_gemm_kernel<2><<<dim3(kH / kTcN, row_tiles, 1), 128, kTcSmem, st>>>(B, kH, kH, dZ2, kH, 1, P + oW2, kH, 1,
-                                                                          dZ1, kH, nullptr, Z1, ew);
+  const GemmArgs w2 = {kH, kH, B, dZ2, 1, kH, H1, kH, 1, grads + oW2, kH, nullptr, nullptr, nullptr};
+  const int z_tiles = kH / kTcN * row_tiles;
+  tc_back_kernel<<<z_tiles + kH / kTcN * (kH / 128) * splits, kTcThreads, kTcSmem, st>>>(z1, w2, z_tiles, splits, ew);
   // gW1[n][k] = sum_b dZ1[b][n] X[b][k]
-  tc_gemm_kernel<0><<<dim3(kIn / kTcN, kH / 128, splits), 128, kTcSmem, st>>>(kH, kIn, B, dZ1, 1, kH, X, kIn, 1,
-                                                                               grads + oW1, kIn, nullptr, nullptr, ew);
-  colsum_kernel<<<dim3((kH + 127) / 128, (B + kColRows - 1) / kColRows), 128, 0, st>>>(B, kH, dZ1, nullptr, grads + oB1);
-  adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(kParams, P, grads, adam_m, adam_v, lr, 0.9f, 0.999f, 1e-8f,
-                                                     M->counters);
-  bump_kernel<<<1, 1, 0, st>>>(M->counters, 1);
-  if (M->loss_out && cudaMemcpyAsync(M->loss_out, loss, sizeof(float), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-    return check_launch("MLP training: loss copy");
-  N3_TRY(check_launch("mlp training kernels"));
-  return launch_pack(M, st);
+  const GemmArgs w1 = {kH, kIn, B, dZ1, 1, kH, X, kIn, 1, grads + oW1, kIn, nullptr, nullptr, nullptr};
+  tc_gemm_kernel<0><<<dim3(kIn / kTcN, kH / 128, splits), kTcThreads, kTcSmem, st>>>(w1, ew);
+  update_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(P, grads, adam_m, adam_v, lr, 0.9f, 0.999f, 1e-8f, M->counters,
+                                                       M->w2_img, M->w1a_img, loss, M->loss_out,
+                                                       reinterpret_cast<uint32_t*>(loss + 1));
+  return check_launch("mlp training kernels");
 }
 
 }  // namespace n3host
@@ -1091,9 +1175,9 @@ int n3_mlp_candidates(const n3_chains* ch, const n3_mlp* M, uint64_t seed, int b
   // in three slices.
   const int C = ch->n_chains;
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<3>), kTcSmem));
-  tc_gemm_kernel<3><<<dim3(kH / kTcN, (C + 127) / 128, 1), 128, kTcSmem, st>>>(
-      C, kH, kChainFeat, M->badn, kChainFeat, 1, M->params + oW1 + kCandFeat, 1, kIn, M->c1, kH, M->params + oB1,
-      nullptr, M->error_word);
+  const GemmArgs g = {C, kH, kChainFeat, M->badn, kChainFeat, 1, M->params + oW1 + kCandFeat, 1, kIn,
+                      M->c1, kH, M->params + oB1, nullptr, nullptr};
+  tc_gemm_kernel<3><<<dim3(kH / kTcN, (C + 127) / 128, 1), kTcThreads, kTcSmem, st>>>(g, M->error_word);
   return n3host::check_launch("chain part (tc_gemm_kernel<3>)");
 }
 
