@@ -95,6 +95,7 @@ struct Remainder {
 };
 
 __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_parent[kMutThreads];
   int parent_count = A.parent_count, quality_count = A.quality_count, active = A.active_strength;
@@ -262,6 +263,7 @@ struct DeltaArgs {
 };
 
 __global__ void __launch_bounds__(kDeltaWarps * 32, 1) child_delta_kernel(const DeltaArgs A) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   if (A.status[1] == 0) return;  // uniform: the search has reached E = 0
   uint16_t* lut4 = reinterpret_cast<uint16_t*>(smem);
@@ -597,6 +599,7 @@ struct SelSmem {
 static_assert(sizeof(SelSmem) <= 227 * 1024, "select_kernel shared memory");
 
 __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const SelArgs A) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   SelSmem& S = *reinterpret_cast<SelSmem*>(smem);
   const int P = A.population, E = A.elite_size, tid = threadIdx.x;
@@ -919,6 +922,7 @@ __global__ void gather_kernel(const int32_t* __restrict__ cp, const int32_t* __r
                               const int32_t* __restrict__ cs, const int32_t* __restrict__ cbad,
                               const int32_t* __restrict__ selected, int n, const int64_t* status, int32_t* pp,
                               int32_t* pq, int32_t* ps, int32_t* pbad) {
+  chain_begin();
   if (status[1] == 0) return;
   const int r = blockIdx.x, c = selected[r];
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -957,6 +961,7 @@ struct RankArgs {
 };
 
 __global__ void __launch_bounds__(kRankThreads, 1) rank_kernel(const RankArgs A) {
+  chain_begin();
   __shared__ int32_t s_score[kMaxElite], s_max[kMaxElite], s_rank[kMaxElite];
   __shared__ int64_t s_ss[kMaxElite];
   __shared__ int s_first, s_improved;
@@ -1060,8 +1065,7 @@ static int launch_mutate(n3::beam::MutArgs A, int parents_bound, cudaStream_t st
   while (threads < kMutThreads && (A.population + threads - 1) / threads > sm_count()) threads *= 2;
   const size_t bytes = (size_t)m * (sizeof(int16_t) * (size_t)threads + sizeof(int32_t) * (size_t)A.prefix_cap);
   N3_TRY(allow_smem(reinterpret_cast<const void*>(mutate_kernel), kMutSmemMax));
-  mutate_kernel<<<(A.population + threads - 1) / threads, threads, bytes, st>>>(A);
-  return check_launch("beam mutate_kernel");
+  return launch_chained("beam mutate_kernel", mutate_kernel, (A.population + threads - 1) / threads, threads, bytes, st, A);
 }
 
 static int check_beam(const n3_beam* b) {
@@ -1221,9 +1225,9 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   D.badness = b->child_badness;
   D.error_word = b->error_word;
   const int dgrid = (b->population + n3::beam::kDeltaWarps - 1) / n3::beam::kDeltaWarps;
-  n3::beam::child_delta_kernel<<<dgrid < n3host::sm_count() ? dgrid : n3host::sm_count(), n3::beam::kDeltaWarps * 32,
-                                 n3::beam::kDeltaSmem, st>>>(D);
-  N3_TRY(n3host::check_launch("beam child_delta_kernel"));
+  N3_TRY(n3host::launch_chained("beam child_delta_kernel", n3::beam::child_delta_kernel,
+                                dgrid < n3host::sm_count() ? dgrid : n3host::sm_count(), n3::beam::kDeltaWarps * 32,
+                                n3::beam::kDeltaSmem, st, D));
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::beam::select_kernel), sizeof(n3::beam::SelSmem)));
   n3::beam::SelArgs S;
   S.scores = b->child_scores;
@@ -1233,14 +1237,13 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   S.status = b->status;
   S.rng = b->rng;
   S.selected = b->selected;
-  n3::beam::select_kernel<<<1, n3::beam::kSelThreads, sizeof(n3::beam::SelSmem), st>>>(S);
-  N3_TRY(n3host::check_launch("beam select_kernel"));
-  n3::beam::gather_kernel<<<b->elite_size, 128, 0, st>>>(b->child_p, b->child_q, b->child_scores, b->child_badness,
-                                                          b->selected, b->n, b->status, b->pick_p, b->pick_q,
-                                                          b->pick_scores, b->pick_badness);
-  N3_TRY(n3host::check_launch("beam gather_kernel"));
-  n3::beam::rank_kernel<<<1, n3::beam::kRankThreads, 0, st>>>(n3host::rank_args(b, b->elite_size, generation));
-  return n3host::check_launch("beam rank_kernel");
+  N3_TRY(n3host::launch_chained("beam select_kernel", n3::beam::select_kernel, 1, n3::beam::kSelThreads,
+                                sizeof(n3::beam::SelSmem), st, S));
+  N3_TRY(n3host::launch_chained("beam gather_kernel", n3::beam::gather_kernel, b->elite_size, 128, 0, st, b->child_p,
+                                b->child_q, b->child_scores, b->child_badness, b->selected, b->n, b->status, b->pick_p,
+                                b->pick_q, b->pick_scores, b->pick_badness));
+  return n3host::launch_chained("beam rank_kernel", n3::beam::rank_kernel, 1, n3::beam::kRankThreads, 0, st,
+                                n3host::rank_args(b, b->elite_size, generation));
 }
 
 }  // extern "C"

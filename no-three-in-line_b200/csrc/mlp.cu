@@ -139,6 +139,7 @@ __device__ __forceinline__ void candidate_features(const ColT* cols, const BadT*
 }
 
 __global__ void __launch_bounds__(kCand) candidates_kernel(const CandArgs A) {
+  chain_begin();
   __shared__ int s_cols[kChainFeat], s_bad[kChainFeat], s_pre[kChainFeat];
   const int c = blockIdx.x;
   const int n = A.ladder_n[c / A.ladder_size], m = 2 * n;
@@ -315,6 +316,7 @@ __device__ __forceinline__ void issue_layer1(uint32_t base, int a1buf, uint32_t 
 // the 128 rows), columns 128 ((w / 4) % 2) ..: each thread owns one row and
 // half of the 256 columns.
 __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(const InferArgs A) {
+  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = umma::smem_addr(smem_raw);
   uint8_t* sm = smem_raw + ((1024u - (raw & 1023u)) & 1023u);  // 1024-aligned base
@@ -515,6 +517,7 @@ constexpr size_t kStepSmem = kCompactLutBytes + kStepChains * kStepChainBytes;
 static_assert(kStepSmem <= 227 * 1024 && kStepChainBytes % 16 == 0, "learned_step_kernel shared memory");
 
 __global__ void __launch_bounds__(kStepChains * 32, 1) learned_step_kernel(const StepArgs A) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   const n3_chains& ch = A.ch;
   uint16_t* lut4 = reinterpret_cast<uint16_t*>(smem);
@@ -710,6 +713,7 @@ __global__ void __launch_bounds__(kGatherRows * 32) gather_kernel(
     const uint16_t* __restrict__ rb_feat, const uint8_t* __restrict__ rb_bad, const int16_t* __restrict__ rb_dE,
     const uint64_t* __restrict__ counters, int64_t capacity, int n_chains, int B, uint32_t k0, uint32_t k1,
     float* __restrict__ X, float* __restrict__ y, float* __restrict__ grads, float* __restrict__ loss) {
+  chain_begin();
   const int lane = threadIdx.x & 31, b = blockIdx.x * kGatherRows + (threadIdx.x >> 5);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) grads[i] = 0.f;
   if (blockIdx.x == 0 && threadIdx.x < 2) loss[threadIdx.x] = 0.f;
@@ -822,6 +826,7 @@ __device__ __forceinline__ void tc_stage(uint8_t* tile, const float* __restrict_
 template <int EPI>
 __device__ __forceinline__ void tc_tile(const GemmArgs& G, int n0, int m0, int split, int splits,
                                         uint32_t* error_word) {
+  chain_begin();
   extern __shared__ __align__(16) uint8_t tc_smem[];
   const uint32_t raw = umma::smem_addr(tc_smem);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -952,6 +957,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const floa
                                                                const float* __restrict__ y, float* __restrict__ d,
                                                                float* __restrict__ dZ2, float* __restrict__ grads,
                                                                float* __restrict__ loss) {
+  chain_begin();
   constexpr int kC = kH / 32;
   __shared__ float s_w3[kHeadWarps][kH], s_b2[kHeadWarps][kH], s_loss[kHeadWarps], s_b3[kHeadWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1022,6 +1028,7 @@ __global__ void update_kernel(float* __restrict__ P, const float* __restrict__ G
                               float* __restrict__ V, float lr, float b1, float b2, float eps, uint64_t* counters,
                               uint8_t* __restrict__ w2_img, uint8_t* __restrict__ w1a_img, const float* loss,
                               float* loss_out, uint32_t* done) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < kParams) {
     const float t = (float)(*(volatile uint64_t*)(counters + 1) + 1);
@@ -1052,7 +1059,10 @@ __global__ void update_kernel(float* __restrict__ P, const float* __restrict__ G
   }
 }
 
-__global__ void bump_kernel(uint64_t* counters, int which) { counters[which] += 1; }
+__global__ void bump_kernel(uint64_t* counters, int which) {
+  chain_begin();
+  counters[which] += 1;
+}
 
 }  // namespace mlp
 }  // namespace n3
@@ -1082,8 +1092,9 @@ namespace n3host {
 // Adam with the tensor-core weight images.  `scratch` holds the batch
 // activations (n3_mlp_scratch_floats(batch) floats), `grads` the gradient
 // (kParams floats); both entry points below call this body.  Seven launches, each
-// waiting for the one before, bound it: a batch of 4096 takes 70 us, 154 us in
-// 17 launches with passes of their own for the sums, the counter and the images.
+// waiting for the one before, bound it: a batch of 4096 takes 60 us chained, 70 us
+// launched plainly, and took 154 us in 17 launches with passes of their own for the
+// sums, the counter and the images.
 static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t seed, float* scratch, float* grads,
                       float* adam_m, float* adam_v, cudaStream_t st) {
   using namespace n3::mlp;
@@ -1111,25 +1122,26 @@ static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t s
   uint32_t* ew = M->error_word;
   // Z1 = X W1^T + b1 ; H1 = relu(Z1)     (W1 [256][192]: B(k, n) = W1[n*192 + k])
   const GemmArgs l1 = {B, kH, kIn, X, kIn, 1, P + oW1, 1, kIn, H1, kH, P + oB1, Z1, nullptr};
-  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st>>>(l1, ew);
+  N3_TRY(launch_chained("mlp layer 1", tc_gemm_kernel<1>, dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st, l1, ew));
   const GemmArgs l2 = {B, kH, kH, H1, kH, 1, P + oW2, 1, kH, H2, kH, P + oB2, Z2, nullptr};
-  tc_gemm_kernel<1><<<dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st>>>(l2, ew);
+  N3_TRY(launch_chained("mlp layer 2", tc_gemm_kernel<1>, dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st, l2, ew));
   const int head_blocks = (B + kHeadWarps - 1) / kHeadWarps;
-  head_kernel<<<head_blocks < sm_count() ? head_blocks : sm_count(), kHeadWarps * 32, 0, st>>>(B, Z2, P, y, d, dZ2,
-                                                                                               grads, loss);
+  N3_TRY(launch_chained("mlp head_kernel", head_kernel, head_blocks < sm_count() ? head_blocks : sm_count(),
+                        kHeadWarps * 32, 0, st, B, Z2, P, y, d, dZ2, grads, loss));
   // dZ1 = (dZ2 W2) * (Z1 > 0)            (B(k, n) = W2[k*256 + n]), and b1's gradient
   const GemmArgs z1 = {B, kH, kH, dZ2, kH, 1, P + oW2, kH, 1, dZ1, kH, nullptr, Z1, grads + oB1};
   // gW2[n][k] = sum_b dZ2[b][n] H1[b][k]
   const GemmArgs w2 = {kH, kH, B, dZ2, 1, kH, H1, kH, 1, grads + oW2, kH, nullptr, nullptr, nullptr};
   const int z_tiles = kH / kTcN * row_tiles;
-  tc_back_kernel<<<z_tiles + kH / kTcN * (kH / 128) * splits, kTcThreads, kTcSmem, st>>>(z1, w2, z_tiles, splits, ew);
+  N3_TRY(launch_chained("mlp tc_back_kernel", tc_back_kernel, z_tiles + kH / kTcN * (kH / 128) * splits, kTcThreads,
+                        kTcSmem, st, z1, w2, z_tiles, splits, ew));
   // gW1[n][k] = sum_b dZ1[b][n] X[b][k]
   const GemmArgs w1 = {kH, kIn, B, dZ1, 1, kH, X, kIn, 1, grads + oW1, kIn, nullptr, nullptr, nullptr};
-  tc_gemm_kernel<0><<<dim3(kIn / kTcN, kH / 128, splits), kTcThreads, kTcSmem, st>>>(w1, ew);
-  update_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(P, grads, adam_m, adam_v, lr, 0.9f, 0.999f, 1e-8f, M->counters,
-                                                       M->w2_img, M->w1a_img, loss, M->loss_out,
-                                                       reinterpret_cast<uint32_t*>(loss + 1));
-  return check_launch("mlp training kernels");
+  N3_TRY(launch_chained("mlp layer 1 gradient", tc_gemm_kernel<0>, dim3(kIn / kTcN, kH / 128, splits), kTcThreads,
+                        kTcSmem, st, w1, ew));
+  return launch_chained("mlp update_kernel", update_kernel, (kParams + 255) / 256, 256, 0, st, P, grads, adam_m, adam_v,
+                        lr, 0.9f, 0.999f, 1e-8f, M->counters, M->w2_img, M->w1a_img, loss, M->loss_out,
+                        reinterpret_cast<uint32_t*>(loss + 1));
 }
 
 }  // namespace n3host
@@ -1177,8 +1189,8 @@ int n3_mlp_candidates(const n3_chains* ch, const n3_mlp* M, uint64_t seed, int b
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(tc_gemm_kernel<3>), kTcSmem));
   const GemmArgs g = {C, kH, kChainFeat, M->badn, kChainFeat, 1, M->params + oW1 + kCandFeat, 1, kIn,
                       M->c1, kH, M->params + oB1, nullptr, nullptr};
-  tc_gemm_kernel<3><<<dim3(kH / kTcN, (C + 127) / 128, 1), kTcThreads, kTcSmem, st>>>(g, M->error_word);
-  return n3host::check_launch("chain part (tc_gemm_kernel<3>)");
+  return n3host::launch_chained("chain part (tc_gemm_kernel<3>)", tc_gemm_kernel<3>, dim3(kH / kTcN, (C + 127) / 128, 1),
+                                kTcThreads, kTcSmem, st, g, M->error_word);
 }
 
 int n3_mlp_infer(const n3_mlp* M, int tiles, void* stream) {
@@ -1196,8 +1208,7 @@ int n3_mlp_infer(const n3_mlp* M, int tiles, void* stream) {
   A.tiles = tiles;
   A.error_word = M->error_word;
   const int grid = tiles < n3host::sm_count() ? tiles : n3host::sm_count();
-  infer_kernel<<<grid, kInferThreads, kInferSmem, (cudaStream_t)stream>>>(A);
-  return n3host::check_launch("infer_kernel");
+  return n3host::launch_chained("infer_kernel", infer_kernel, grid, kInferThreads, kInferSmem, (cudaStream_t)stream, A);
 }
 
 int n3_mlp_step_team(const n3_chains* ch, const n3_mlp* M, const float* temps, uint64_t seed, int moves,
@@ -1226,10 +1237,8 @@ int n3_mlp_step_team(const n3_chains* ch, const n3_mlp* M, const float* temps, u
   A.moves = moves;
   const int grid = (ch->n_chains + kStepChains - 1) / kStepChains;
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(learned_step_kernel), kStepSmem));
-  learned_step_kernel<<<grid, kStepChains * 32, kStepSmem, (cudaStream_t)stream>>>(A);
-  N3_TRY(n3host::check_launch("learned_step_kernel"));
-  bump_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(M->counters, 0);
-  return n3host::check_launch("bump_kernel");
+  N3_TRY(n3host::launch_chained("learned_step_kernel", learned_step_kernel, grid, kStepChains * 32, kStepSmem, (cudaStream_t)stream, A));
+  return n3host::launch_chained("bump_kernel", bump_kernel, 1, 1, 0, (cudaStream_t)stream, M->counters, 0);
 }
 
 int n3_mlp_step(const n3_chains* ch, const n3_mlp* M, const float* temps, uint64_t seed, int moves, void* stream) {

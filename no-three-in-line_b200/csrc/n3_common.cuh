@@ -28,6 +28,14 @@ enum : uint32_t {
   kErrCapacity = 1u << 5,      // an output list was longer than the caller's capacity
 };
 
+// First in a kernel launched by launch_chained: lets the next kernel of the chain be
+// brought onto the SMs, then waits until the one before has finished and its
+// writes are visible.  Nothing before it in the kernel may touch memory or hold
+// tensor memory.  Without effect in a kernel launched otherwise.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
 }  // namespace n3
@@ -39,6 +47,29 @@ int check_launch(const char* what);
 int ensure_device_tables();
 int sm_count();
 int allow_smem(const void* kernel, size_t bytes);
+
+// A launch whose blocks may be brought onto the SMs while the kernel before it in
+// the stream still runs (programmatic stream serialization), for short kernels
+// that follow each other; the kernel begins with n3::chain_begin().  It saves 1 to
+// 2 us per launch: a training step of seven 70 -> 60 us, a learned step of five
+// 107 -> 99 us, a beam generation of five 188 -> 183 us.
+template <class... Params, class... Args>
+int launch_chained(const char* what, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                   Args... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = st;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) return set_error(N3_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  return check_launch(what);
+}
 }  // namespace n3host
 
 #define N3_TRY(expr)                      \
