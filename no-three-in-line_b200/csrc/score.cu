@@ -198,6 +198,27 @@ __host__ __device__ constexpr size_t tag_smem(int warps) { return kCompactLutByt
 static_assert(tag_smem(kTagWarps) <= 227 * 1024, "tag_kernel shared memory");
 static_assert(kDirCount >= (int)sizeof(int) * kMaxM, "a state's columns fit in a warp's tags");
 
+// State b's table keys for tag_state, its word[] cleared; returns the error bits of
+// columns outside [0, limit) and equal points in a row (the same in every lane).
+template <class Src>
+__device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int limit, int lane,
+                                             int (&key)[kSlotsPerLane], uint32_t* __restrict__ word) {
+  uint32_t err = 0;
+#pragma unroll
+  for (int t = 0; t < kSlotsPerLane; ++t) {
+    const int s = lane + 32 * t;
+    const bool in = s < 2 * n;
+    const int c = in ? src.col(b, n, s) : 0;
+    // the two points of a row are neighbouring lanes
+    const int c2 = __shfl_xor_sync(0xffffffffu, c, 1);
+    if (in && (c < 0 || c >= limit)) err |= kErrColumnRange;
+    if (in && c == c2) err |= kErrDuplicate;
+    key[t] = in ? (s >> 1) * kLutW + c : -1;
+    if (in) word[s] = 0u;
+  }
+  return __reduce_or_sync(0xffffffffu, err);
+}
+
 template <class Src, int MODE, bool BAD, bool SPLIT>
 __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, int n, int W, int parts,
                                                                  const uint16_t* __restrict__ g_lut,
@@ -228,21 +249,8 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
   };
   for (int b = blockIdx.x * (W / parts) + group; b < B; b += gridDim.x * (W / parts)) {
     int key[kSlotsPerLane];
-    uint32_t err = 0;
-#pragma unroll
-    for (int t = 0; t < kSlotsPerLane; ++t) {
-      const int s = lane + 32 * t;
-      const bool in = s < m;
-      const int c = in ? src.col(b, n, s) : 0;
-      // the two points of a row are neighbouring lanes
-      const int c2 = __shfl_xor_sync(0xffffffffu, c, 1);
-      if (in && (c < 0 || c >= (MODE == kCount ? kMaxN : n))) err |= kErrColumnRange;
-      if (in && c == c2) err |= kErrDuplicate;
-      key[t] = in ? (s >> 1) * kLutW + c : -1;
-      if (in) word[s] = 0u;
-    }
+    const uint32_t err = tag_load(src, b, n, MODE == kCount ? kMaxN : n, lane, key, word);
     if (part == 0 && lane == 0) *total = 0;
-    err = __reduce_or_sync(0xffffffffu, err);  // the same in every warp of the group
     group_sync();
     if (err) {  // no line count exists
       if (part == 0) {
@@ -289,6 +297,111 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
         for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = (int)bad[s];
     }
     group_sync();
+  }
+}
+
+// Both counts of the checked score side by side: the determinants wait for the
+// multiply-add pipe (71 % of issue slots used), the tags for shared memory (70 %), so
+// `tag_warps` of a CTA's 32 warps take the tags and the rest the determinants, a
+// quarter of a state's pivot rows at a time.  A CTA owns `per` consecutive states
+// and compares the two counts kCheckedStates states at a time.
+constexpr int kCheckedStates = 56;
+struct CheckedShared {
+  int det[kCheckedStates], slope[kCheckedStates];
+  uint32_t err[kCheckedStates], off_grid[kCheckedStates];
+  int next_det, next_tag;
+};
+__host__ __device__ constexpr size_t checked_smem(int tag_warps, int n) {
+  return kCompactLutBytes + (size_t)tag_warps * kTagWarpBytes + (size_t)kCheckedStates * n * sizeof(float4) +
+         sizeof(CheckedShared);
+}
+
+constexpr size_t kCheckedMaxSmem = checked_smem(14, kMaxN);
+static_assert(kCheckedMaxSmem <= 227 * 1024, "checked_kernel shared memory");
+
+template <bool BAD>
+__global__ void __launch_bounds__(1024, 1) checked_kernel(ColSource src, int B, int n, int per, int tag_warps,
+                                                          const uint16_t* __restrict__ g_lut,
+                                                          int32_t* __restrict__ scores,
+                                                          int32_t* __restrict__ badness,
+                                                          int32_t* __restrict__ mismatch,
+                                                          uint32_t* __restrict__ error_word) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
+  float4* rows = reinterpret_cast<float4*>(smem + kCompactLutBytes);  // [kCheckedStates][n]
+  unsigned char* tags = smem + kCompactLutBytes + (size_t)kCheckedStates * n * sizeof(float4);
+  CheckedShared& S = *reinterpret_cast<CheckedShared*>(tags + (size_t)tag_warps * kTagWarpBytes);
+  compact_lut_copy(lut, g_lut);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, det_warps = 32 - tag_warps, m = 2 * n;
+  const int b_end = min(B, (int)(blockIdx.x + 1) * per);
+  for (int b0 = blockIdx.x * per; b0 < b_end; b0 += kCheckedStates) {
+    const int count = min(kCheckedStates, b_end - b0);
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+      S.det[i] = 0;
+      S.off_grid[i] = 0u;
+    }
+    if (threadIdx.x == 0) S.next_det = S.next_tag = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < count * n; i += blockDim.x) {
+      const int k = i / n, r = i - k * n;
+      const int c0 = src.col(b0 + k, n, 2 * r), c1 = src.col(b0 + k, n, 2 * r + 1);
+      if ((unsigned)c0 >= (unsigned)kMaxN || (unsigned)c1 >= (unsigned)kMaxN) S.off_grid[k] = 1u;
+      rows[i] = make_float4((float)c0, (float)c0, (float)c1, (float)c1);
+    }
+    __syncthreads();
+    if (warp < det_warps) {
+      for (;;) {
+        int task = 0;
+        if (lane == 0) task = atomicAdd(&S.next_det, 1);
+        task = __shfl_sync(0xffffffffu, task, 0);
+        if (task >= 4 * count) break;
+        const int k = task >> 2, part = task & 3;
+        float4* rows4 = rows + k * n;
+        int cnt = 0;
+        if (!S.off_grid[k]) {  // uniform
+          cnt = det_state_f<false>(rows4, n, lane, part, 4, nullptr);
+        } else if (part == 0) {
+          int* cs = reinterpret_cast<int*>(rows4);
+          for (int s = lane; s < m; s += 32) cs[s] = src.col(b0 + k, n, s);
+          __syncwarp();
+          cnt = det_state<false>(cs, n, lane, nullptr);
+        }
+        cnt = warp_sum(cnt);
+        if (lane == 0 && cnt) atomicAdd(&S.det[k], cnt);
+      }
+    } else {
+      uint8_t* tag = tags + (size_t)(warp - det_warps) * kTagWarpBytes;
+      uint32_t* word = reinterpret_cast<uint32_t*>(tag + kDirCount);
+      for (;;) {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(&S.next_tag, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= count) break;
+        int key[kSlotsPerLane], e = -1;
+        const uint32_t err = tag_load(src, b0 + k, n, n, lane, key, word);
+        __syncwarp();
+        if (!err) e = tag_state<BAD>(key, m, lut, tag, lane, word, word);
+        __syncwarp();
+        if (lane == 0) {
+          S.slope[k] = e;
+          S.err[k] = err;
+        }
+        if (BAD)
+          for (int s = lane; s < m; s += 32) badness[(size_t)(b0 + k) * m + s] = err ? -1 : (int)word[s];
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < count; k += blockDim.x) {
+      uint32_t err = S.err[k];
+      scores[b0 + k] = err ? -1 : S.det[k];
+      if (!err && S.slope[k] != S.det[k]) err = kErrMismatch;
+      if (err) {
+        atomicAdd(mismatch, 1);
+        if (error_word) atomicOr(error_word, err);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -410,7 +523,34 @@ static int prepare_tag() {
   return allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, false>), tag_smem(kTagWarps));
 }
 
+// The two counts of the checked score in one kernel (checked_kernel) for many
+// states of larger grids.  us with badness, two kernels against one: 4096 states
+// n = 75: 373 / 352, 61: 242 / 226, 47: 146 / 136, 38: 105 / 101, 32: 82 / 82; 20,011
+// states: 1687 / 1628, 1077 / 1030, 632 / 611, 441 / 458, 337 / 364; 4300 states, which
+// leave the determinants a last wave of few blocks: 491 / 372, 328 / 240, 205 / 166.
+// n = 75, 1200 states: 181 / 124; 900: 109 / 118 (fewer states get more warps each in
+// the two kernels).  Warps for the tags: 12 from n = 56 on, 14 below (n = 50: 14
+// take 150 us for 4096 states, 12 take 173; n = 75: 352 both).
+constexpr int kCheckedMinN = 44, kCheckedMinPerSm = 8;
+constexpr int kCheckedTagWarps = 12, kCheckedTagWarpsSmall = 14, kCheckedSmallN = 56;
+
+static int launch_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+                          uint32_t* error_word, cudaStream_t st) {
+  using namespace n3;
+  N3_TRY(ensure_device_tables());
+  const int sms = sm_count(), per = (B + sms - 1) / sms;
+  const int tag_warps = n < kCheckedSmallN ? kCheckedTagWarpsSmall : kCheckedTagWarps;
+  const auto kernel = badness ? checked_kernel<true> : checked_kernel<false>;
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(kernel), kCheckedMaxSmem));
+  kernel<<<(B + per - 1) / per, 1024, checked_smem(tag_warps, n), st>>>(
+      ColSource{cols}, B, n, per, tag_warps, dir_lut_device_ptr(), scores, badness, mismatch, error_word);
+  return check_launch("checked_kernel");
+}
+
 int prepare_score() {
+  using namespace n3;
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(checked_kernel<true>), kCheckedMaxSmem));
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(checked_kernel<false>), kCheckedMaxSmem));
   N3_TRY((prepare_tag<n3::PQSource, n3::kCount>()));
   N3_TRY((prepare_tag<n3::ColSource, n3::kCount>()));
   N3_TRY((prepare_tag<n3::ColSource, n3::kSlope>()));
@@ -443,6 +583,8 @@ int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t
   N3_TRY(n3host::check_common(B, n, cols, scores));
   if (B > 0 && mismatch == nullptr) return n3host::set_error(N3_ERR_ARG, "null mismatch counter");
   if (B == 0) return N3_OK;
+  if (n >= n3host::kCheckedMinN && B >= n3host::kCheckedMinPerSm * n3host::sm_count())
+    return n3host::launch_checked(cols, B, n, scores, badness, mismatch, error_word, (cudaStream_t)stream);
   // Two launches on one stream: the determinant count at full occupancy, then
   // the independent slope count, which validates each state, compares, and
   // gives the badness if it is wanted.
