@@ -48,10 +48,10 @@ KERNEL_TESTS_PER_STATE = TESTS_PER_STATE - N * (2 * N - 2)  # 540,200
 OPS_PER_TEST = 2
 L2_FLUSH_BYTES = 256 << 20             # > 126 MB L2
 WORKLOAD = "n=75 population scoring, 4096 states, determinant + slope cross-check + badness"
-# dram__bytes_read.sum + dram__bytes_write.sum of one det_kernel launch over the
-# 4096-state population, from an ncu capture (1,253,632 B read, 0 B written; the
-# algorithmic input is 1,228,800 B of int16 columns plus the 16 KB of counts).
-DET_TRAFFIC_BYTES = 1253632
+# dram__bytes_read.sum + dram__bytes_write.sum of one checked_kernel launch over the
+# 4096-state population, from an ncu capture (the algorithmic input is 1,228,800 B
+# of int16 columns; the 2.5 MB of counts and badness stay in L2).
+CHECKED_TRAFFIC_BYTES = 1317120
 
 
 def parse():
@@ -64,7 +64,7 @@ def parse():
     ap.add_argument("--mode", choices=["checked", "det", "slope", "tempering", "learned", "time-to-target", "beam",
                                        "scan", "lines", "exhaustive"],
                     default="checked",
-                    help="kernel a step runs: fused checked scoring (default), determinant only, slope only; "
+                    help="kernel a step runs: fused checked scoring (default), the population count alone (det), slope only; "
                          "tempering / learned chain rounds; one device beam-search generation (beam); one "
                          "four-cycle + double-switch neighbourhood scan (scan); the n = 75 line tables "
                          "and both table scorers (lines); one exhaustive 2-switch beam generation (exhaustive); "
@@ -286,7 +286,7 @@ def secondary_measurements(dev, p, q):
     b.synchronize()
     legal = int((dE != gpu_delta.SENTINEL).sum().item())
     out["swap_delta_batch"] = {"moves": M, "legal": legal, "deltas_per_s": 10 * M / (a.elapsed_time(b) / 1e3),
-                               "kernel": "n3::swap_delta_kernel<false> (direction-class, no badness output)"}
+                               "kernel": "n3::swap_delta_kernel<false, 5> (direction-class, no badness output)"}
     launches += 13
     # every 2-switch partner of every slot of 64 n=75 states (the reference plugin's
     # two_switch_scores, gpu_delta.py:19-75): 9600 anchors x 150 partners
@@ -483,7 +483,7 @@ def run_search_mode(args):
         counter = iter(range(1, gens + 1))
         step = lambda: beam.generation(next(counter))  # noqa: E731
         per_step, unit, what = pop, "children/s", "device beam search generations (mutate, score, select, rank)"
-        launches = 6
+        launches = 5
     else:
         anchor = gpu_neighborhood.bad_anchor_indices(init, 1)[0]
         dp = torch.tensor(init.P, dtype=torch.int32, device="cuda")
@@ -495,7 +495,7 @@ def run_search_mode(args):
                                                          out.data_ptr(), out.data_ptr() + 16,
                                                          int(stream.cuda_stream)), "n3_neighborhood_scan")
         per_step, unit, what = 64824 * 8 * 9, "candidates/s", "four-cycle + double-switch candidates scored exactly"
-        launches = 1
+        launches = 2
     for _ in range(max(3, args.warmup) if args.mode == "scan" else args.warmup):
         step()
     torch.cuda.synchronize()
@@ -833,13 +833,14 @@ def run_b200(args):
         dist.all_reduce(t_e2e, op=dist.ReduceOp.MAX)
     e2e_ms = float(t_e2e.item())
 
-    # the dominant kernel alone (the determinant count), for the roofline
+    # one checked launch alone, for the roofline
     det_ms = []
     for k in range(12):
         flush.fill_(k)
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record(stream)
-        _lib.check(L.n3_score_columns(cols.data_ptr(), B, N, scores.data_ptr(), None, sptr), "n3_score_columns")
+        _lib.check(L.n3_score_checked(cols.data_ptr(), B, N, scores.data_ptr(), badness.data_ptr(), flags.data_ptr(),
+                                      flags.data_ptr() + 4, sptr), "n3_score_checked")
         b.record(stream)
         det_ms.append((a, b))
     torch.cuda.synchronize()
@@ -875,7 +876,7 @@ def run_b200(args):
     if rank == 0:
         ms_per_step = total_ms / args.steps
         tests_per_s = value * TESTS_PER_STATE
-        # the determinant kernel's own launches: 4096 states x 540,200 tested triples
+        # the determinants alone: 4096 states x 540,200 tested triples per launch
         kernel_tests = B * KERNEL_TESTS_PER_STATE / det_launch_s
         pipe_tests = min(pipe_rate["imad"], pipe_rate["alu"])  # one op of each pipe per test
         achieved = kernel_tests * OPS_PER_TEST / 1e9
@@ -893,10 +894,11 @@ def run_b200(args):
                     "h2d_bytes_per_step": int(cols_host.nbytes),
                     "d2h_bytes_per_step": int(h_scores.numel() * 4 + h_flags.numel() * 4),
                     "copies": "pinned host buffers; H2D of step k+1 and read-back of step k on a second stream beside the compute"},
-            "gpu_launches": args.steps * (2 if args.mode == "checked" else 1),
+            "gpu_launches": args.steps * (2 if args.mode == "checked" and B < 8 * sms else 1),
             "roofline": {"bound": "int32 pipes (FMA pipe for products, ALU pipe for compares)",
-                         "kernel": "n3::det_kernel<ColSource,false> (the larger of the checked step's two "
-                                   "launches; the other is n3::slope4_kernel<2>), timed alone",
+                         "kernel": "n3::checked_kernel<true> (the step's one launch: determinants on the multiply-add "
+                                   "pipe beside the slope count on shared memory), timed alone; the operations "
+                                   "counted are the determinants'",
                          "kernel_launch_us": det_launch_s * 1e6,
                          "kernel_tests_per_s": kernel_tests,
                          "achieved": achieved, "peak": peak, "unit": "Gop/s", "frac": achieved / peak,
@@ -909,7 +911,7 @@ def run_b200(args):
                                                 "frac": kernel_tests / ceiling_tests,
                                                 "source": "n3_calibrate_det_ceiling: the scorer's test "
                                                           "expression with per-test counting, on registers"},
-                         "traffic": DET_TRAFFIC_BYTES,
+                         "traffic": CHECKED_TRAFFIC_BYTES,
                          "hbm_context": {"bytes_per_step": int(cols_host.nbytes + B * 4 + B * 2 * N * 4),
                                          "hbm_gbs_peak": peaks.get("hbm_gbs"), "peak_kind": peak_kind}},
             "wall_s_timed": wall,

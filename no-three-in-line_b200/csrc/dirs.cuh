@@ -48,7 +48,7 @@ __device__ __forceinline__ void hist_clear(uint32_t* hist, int id) { hist[id >> 
 constexpr int kSlotsPerLane = (kMaxM + 31) / 32;  // 5
 
 // Full direction table (signed dx, no normalisation at lookup), kept in shared
-// memory by the kernels that evaluate moves: entry (dx + kMaxN - 1) * kLutW +
+// memory by analyze_kernel, three_cycle_kernel and scan_any_kernel: entry (dx + kMaxN - 1) * kLutW +
 // dy + kMaxN - 1 holds the id of (dx, dy); (0, 0) holds 0 and is never read.
 // With key(r, c) = r * kLutW + c the entry of the difference a - b sits at
 // key(a) - key(b) + kFullLutCentre, one add per lookup.

@@ -14,7 +14,7 @@
 //     is the reference's descriptor order: elite, anchor u ascending, partner v
 //     ascending, skipping u's row and anchors v < u.
 //  2. n3_two_switch_scores: the exact score after each (elite, u, v) swap, from
-//     the elite's maintained badness and two direction histograms per partner.
+//     the elite's maintained badness and its cover table.
 //  3. compact_kernel (a warp per anchor): each kept partner's score at its
 //     candidate index, 2^29 where the swap is illegal (the reference's marker
 //     for invalid children, gpu_exhaustive_beam.py:179), plus its descriptor.

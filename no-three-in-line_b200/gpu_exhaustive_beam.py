@@ -9,7 +9,7 @@ and elite ranking.  Where it runs differs (libn3 ``n3_exh_*``):
 
 * every candidate of a generation, all legal 2-switches of all elites that
   touch a bad slot (all slots every ``global_every`` generations), is scored on
-  the device exactly from its parent (two direction histograms per partner),
+  the device exactly from its parent (a cover table per elite),
   without building the child; the reference builds every child and rescores
   it in full;
 * the quality pool (the first 24 x elite_size candidates of the stable score
