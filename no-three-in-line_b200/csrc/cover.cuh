@@ -126,6 +126,64 @@ static __device__ __noinline__ void cover_swap(const uint8_t* __restrict__ cs, u
   }
 }
 
+// Points of the state on each lane's line through (r0, c0) and (r1, c1), those two
+// cells left out; 0 for lanes without `valid` and for cells of one row or column.  bits:
+// a bit per cell, number row * n + column.  The cells are numbered through as in
+// cover_line; a cell in 40 holds a point, which adds to its line's counter.  scratch:
+// the warp's 32 uint2; count: its 32 words.  All lanes call it.
+static __device__ __noinline__ int count_lines(const uint32_t* __restrict__ bits, int n, int r0, int c0, int r1, int c1,
+                                               bool valid, const uint16_t* __restrict__ prim4,
+                                               const uint32_t* __restrict__ recip, uint2* __restrict__ scratch,
+                                               uint32_t* __restrict__ count, int lane) {
+  const int key = (int)(dir4(prim4, r1 * kLutW + c1, r0 * kLutW + c0) >> 2);
+  int a = (key + kMaxN - 1) / kLutW, b = key - a * kLutW;
+  valid = valid && a != 0 && b != 0;
+  if (!valid) a = b = 1;
+  const uint32_t ia = recip[a], ib = recip[abs(b)];
+  const int right = n - 1 - c0, down = n - 1 - r0;
+  const int fwd = min((int)((uint32_t)down * ia >> 16), (int)((uint32_t)(b > 0 ? right : c0) * ib >> 16));
+  const int back = min((int)((uint32_t)r0 * ia >> 16), (int)((uint32_t)(b > 0 ? c0 : right) * ib >> 16));
+  const int apart = (int)((uint32_t)abs(r1 - r0) * ia >> 16);
+  const int step = a * n + b, first = r0 * n + c0 - back * step;
+  const int at_0 = back, at_1 = r1 > r0 ? back + apart : back - apart;
+  const int cells = valid ? fwd + back - 1 : 0;
+  int offset = cells;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, offset, o);
+    if (lane >= o) offset += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, offset, 31);
+  offset -= cells;
+  const unsigned some = __ballot_sync(0xffffffffu, cells > 0);
+  const int mine = __popc(some & ((1u << lane) - 1u));
+  __syncwarp();
+  count[lane] = 0u;
+  if (cells > 0)
+    scratch[mine] = make_uint2((uint32_t)first | ((uint32_t)min(at_0, at_1) << 16) | ((uint32_t)max(at_0, at_1) << 23),
+                               (uint32_t)step | ((uint32_t)offset << 16));
+  __syncwarp();
+  int line = -1;  // lines begun before the chunk, less one
+#pragma unroll 2
+  for (int base = 0; base < total; base += 32) {
+    const unsigned in_chunk = (unsigned)(offset - base);
+    const unsigned starts = __reduce_or_sync(0xffffffffu, cells > 0 && in_chunk < 32u ? 1u << in_chunk : 0u);
+    const int i = base + lane;
+    if (i < total) {
+      const int at = line + __popc(starts & (0xffffffffu >> (31 - lane)));
+      const uint2 d = scratch[at];
+      int s = i - (int)(d.y >> 16);
+      s += s >= (int)((d.x >> 16) & 127u);
+      s += s >= (int)(d.x >> 23);
+      const int cell = (int)(d.x & 0xFFFFu) + s * (int)(d.y & 0xFFFFu);
+      if ((bits[cell >> 5] >> (cell & 31)) & 1u) atomicAdd(count + at, 1u);
+    }
+    line += __popc(starts);
+  }
+  __syncwarp();
+  return cells > 0 ? (int)count[mine] : 0;
+}
+
 // Occupancy of the grid: three words a row, bit c & 31 of word c >> 5 for column c.
 constexpr int kOccWords = 3 * kMaxN;
 

@@ -284,11 +284,13 @@ __global__ void __launch_bounds__(kDeltaWarps * 32, 1) swap_delta_kernel(const M
 // run of consecutive anchors of one state:
 //   kRunCover or more   the CTA builds the cover table of the state once; then a
 //       warp per anchor takes joint(u, v) of all partners from one histogram
-//       around u, t(u') and t(v') from the table, and j(u', v') by walking the
-//       line over the occupancy bits (4.6 cells on average), a lane per partner
+//       around u, t(u') and t(v') from the table, and j(u', v') by the cells of
+//       32 partners' lines numbered through (4.6 on average, but 40 in the longest,
+//       so a walk per lane took 8 us more); the last anchors of a run share
+//       their partners among the warps left (4 us)
 //   fewer               a warp per partner, both new centres' histograms side by
 //       side (pair_move.cuh), whatever the columns hold
-// 64 n = 75 states, every slot: 85 us, 835 us with two histograms per partner one
+// 64 n = 75 states, every slot: 70 us, 834 us with two histograms per partner one
 // after the other; 1024 states with a slot each, partners of its layer: 48 and 60 us.
 constexpr int kPartnerWarps = 24;
 constexpr int kRunCover = 8;
@@ -299,9 +301,10 @@ struct PartnerSmem {
   uint16_t dir4[kCompactLutBytes / 2];
   uint32_t recip[kMaxN + 1];
   uint32_t T[kPartnerRegion];
-  uint32_t occ[kOccWords + 3];
+  uint32_t bits[(kMaxN * kMaxN + 31) / 32];  // the state's cells
   uint32_t hist[kPartnerWarps][2 * DenseNumbering::kWords];
   uint2 scratch[kPartnerWarps][32];
+  uint32_t count[kPartnerWarps][32];
   int columns[kMaxN];
   uint8_t cs[152];
 };
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
     bool cover = a1 - a0 >= kRunCover;
     if (cover) {
       for (int i = tid; i < kMaxN; i += blockDim.x) S.columns[i] = 0;
-      for (int i = tid; i < kOccWords; i += blockDim.x) S.occ[i] = 0u;
+      for (int i = tid; i < (kMaxN * kMaxN + 31) / 32; i += blockDim.x) S.bits[i] = 0u;
       for (int i = tid; i < kPartnerRegion; i += blockDim.x) S.T[i] = 0u;
       __syncthreads();
     }
@@ -433,8 +436,9 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
       S.cs[s] = (uint8_t)min(max(c, 0), n - 1);
       if (cover && on_grid) {
         atomicAdd(&S.columns[c], 1);
-        const uint32_t bit = 1u << (c & 31);
-        if (atomicOr(&S.occ[3 * (s >> 1) + (c >> 5)], bit) & bit) regular = false;
+        const int cell = (s >> 1) * n + c;
+        const uint32_t bit = 1u << (cell & 31);
+        if (atomicOr(&S.bits[cell >> 5], bit) & bit) regular = false;
       }
     }
     __syncthreads();
@@ -445,10 +449,15 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
     if (cover) {
       cover_build(S.cs, S.T, n, S.prim4, S.recip, S.scratch[warp], lane, warp, kPartnerWarps);
       __syncthreads();
-      for (int a = a0 + warp; a < a1; a += kPartnerWarps) {
+      for (int first = a0; first < a1; first += kPartnerWarps) {
+        // a warp per anchor; the last ones share their partners among several warps
+        const int left = a1 - first, parts = left < kPartnerWarps ? kPartnerWarps / left : 1;
+        const int a = first + warp / parts, w_first = 32 * (warp % parts), w_step = 32 * parts;
+        if (a >= a1) break;  // uniform in the warp
         const int u = anchors[2 * a + 1];
         if (u < 0 || u >= m) {  // uniform in the warp
-          for (int w = lane; w < width; w += 32) out[(size_t)a * width + w] = N3_SENTINEL;
+          for (int w0 = w_first; w0 < width; w0 += w_step)
+            if (w0 + lane < width) out[(size_t)a * width + w0 + lane] = N3_SENTINEL;
           continue;
         }
         const int ru = u >> 1, cu = S.cs[u], centre = ru * kLutW + cu, bad_u = bad[u];
@@ -460,15 +469,18 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
           if (ids[t] >= 0) hist_add(hist, ids[t]);
         }
         __syncwarp();
-        for (int w = lane; w < width; w += 32) {
-          const int v = SAME_LAYER ? 2 * w + (u & 1) : w;
+        for (int w0 = w_first; w0 < width; w0 += w_step) {
+          const int w = w0 + lane, v = min(SAME_LAYER ? 2 * w + (u & 1) : w, m - 1);
           const int rv = v >> 1, cv = S.cs[v];
+          const bool legal = w < width && rv != ru && cv != S.cs[u ^ 1] && cu != S.cs[v ^ 1];
+          const int line = count_lines(S.bits, n, ru, cv, rv, cu, legal, S.prim4, S.recip, S.scratch[warp],
+                                       S.count[warp], lane);
+          if (w >= width) continue;
           int score = N3_SENTINEL;
-          if (rv != ru && cv != S.cs[u ^ 1] && cu != S.cs[v ^ 1]) {
+          if (legal) {
             // the others on the line (u, v) (a column holds no third point)
             const int joint = hist_get(hist, (int)(dir4(S.dir4, rv * kLutW + cv, centre) >> 2)) - 1;
-            score = cur - (bad_u + bad[v] - joint) + cover_get(S.T, ru * n + cv) + cover_get(S.T, rv * n + cu) +
-                    points_on_line(S.occ, n, S.prim4, ru, cv, rv, cu);
+            score = cur - (bad_u + bad[v] - joint) + cover_get(S.T, ru * n + cv) + cover_get(S.T, rv * n + cu) + line;
           }
           out[(size_t)a * width + w] = score;
         }
@@ -561,7 +573,8 @@ static int launch_partners(bool same_layer, const int16_t* cols, const int32_t* 
   // Consecutive anchors to a CTA, one CTA per SM.  Callers list a state's anchors
   // together; with enough of them each CTA gets whole states or a share of one, as
   // it would if all states had the same number, so that few build two cover tables
-  // (64 states of 150 anchors: 128 CTAs of 75 take 85 us, 148 of 65 take 111 us).
+  // (64 states of 150 anchors, with a walk per lane: 128 CTAs of 75 took 85 us, 148 of
+  // 65 took 111 us).
   int per_cta = (A + sms - 1) / sms;
   const int each = B > 0 ? A / B : 0;
   if (each >= 2 * n3::kRunCover && each * (int64_t)B == A) {
