@@ -60,7 +60,7 @@ def score_population_gpu(p_batch, q_batch, *, badness: bool = False, stream=None
 
 
 def score_columns_gpu(columns, *, badness: bool = False, stream=None):
-    """Determinant count over slot-layout columns ([B, 2n] int16 tensor or array)."""
+    """Exact triple count over slot-layout columns ([B, 2n] int16 tensor or array)."""
     t = _lib.torch()
     device = _lib.require_device()
     host = not _lib.is_tensor(columns)
