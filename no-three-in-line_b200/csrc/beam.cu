@@ -566,7 +566,15 @@ __device__ void shuffle_steps_cta(uint32_t* mt, int& idx, int count, uint16_t* j
       while (steps_left >= 1 && pos < blocks * kMT)
         shuffle_draws_cta(out, blocks * kMT, pos, steps_left, jstep, tot, cut);
       if (steps_left < 1) break;  // uniform
-      if (tid < kTwistThreads) mt_twist(words + (blocks - 1) * kMT, words);  // the next batch's first block
+      // the next batch's first block, twisted out of place: a batch of one block
+      // moves to the outputs, which are used up
+      const uint32_t* from = words + (blocks - 1) * kMT;
+      if (blocks == 1) {  // uniform
+        for (int k = tid; k < kMT; k += blockDim.x) out[k] = words[k];
+        __syncthreads();
+        from = out;
+      }
+      if (tid < kTwistThreads) mt_twist(from, words);
       pos = 0;
     }
     const int last = pos - 1;  // >= 0: every round uses at least one word
