@@ -926,10 +926,9 @@ __global__ void __launch_bounds__(kSelThreads, 1) py_steps_kernel(uint32_t* stat
 }
 
 // pick rows r = child rows selected[r]
-__global__ void gather_kernel(const int32_t* __restrict__ cp, const int32_t* __restrict__ cq,
-                              const int32_t* __restrict__ cs, const int32_t* __restrict__ cbad,
-                              const int32_t* __restrict__ selected, int n, const int64_t* status, int32_t* pp,
-                              int32_t* pq, int32_t* ps, int32_t* pbad) {
+__global__ void gather_kernel(const int32_t* cp, const int32_t* cq, const int32_t* cs, const int32_t* cbad,
+                              const int32_t* selected, int n, const int64_t* status, int32_t* __restrict__ pp,
+                              int32_t* __restrict__ pq, int32_t* __restrict__ ps, int32_t* __restrict__ pbad) {
   chain_begin();
   if (status[1] == 0) return;
   const int r = blockIdx.x, c = selected[r];

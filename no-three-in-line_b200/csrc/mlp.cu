@@ -710,9 +710,9 @@ struct Batch {
 // the gradient, and at `loss` the loss and update_kernel's count of blocks.
 constexpr int kGatherRows = 8;
 __global__ void __launch_bounds__(kGatherRows * 32) gather_kernel(
-    const uint16_t* __restrict__ rb_feat, const uint8_t* __restrict__ rb_bad, const int16_t* __restrict__ rb_dE,
-    const uint64_t* __restrict__ counters, int64_t capacity, int n_chains, int B, uint32_t k0, uint32_t k1,
-    float* __restrict__ X, float* __restrict__ y, float* __restrict__ grads, float* __restrict__ loss) {
+    const uint16_t* rb_feat, const uint8_t* rb_bad, const int16_t* rb_dE, const uint64_t* counters, int64_t capacity,
+    int n_chains, int B, uint32_t k0, uint32_t k1, float* __restrict__ X, float* __restrict__ y,
+    float* __restrict__ grads, float* __restrict__ loss) {
   chain_begin();
   const int lane = threadIdx.x & 31, b = blockIdx.x * kGatherRows + (threadIdx.x >> 5);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) grads[i] = 0.f;
@@ -778,49 +778,57 @@ struct GemmArgs {
   float* sums;
 };
 
-// Stages ROWS x 64 elements of an operand, element (r, k) at src[(r0 + r) sr + (k0 + k) sk],
-// zero outside r0 + r < R, k0 + k < Ke, into an SW128 K-major bf16 tile.
+// Loads ROWS x 64 elements of an operand, element (r, k) at src[(r0 + r) sr + (k0 + k) sk],
+// zero outside r0 + r < R, k0 + k < Ke: 16-byte chunks (8 elements along k) per thread.
 template <int ROWS>
-__device__ __forceinline__ void tc_stage(uint8_t* tile, const float* __restrict__ src, int sr, int sk, int r0, int R,
-                                         int k0, int Ke, int tid) {
-  constexpr int kChunks = ROWS * 8 / kTcThreads;  // 16-byte chunks (8 elements) per thread
+struct TcChunks {
+  static constexpr int kChunks = ROWS * 8 / kTcThreads;
   float v[kChunks][8];
-  // uniform; the training scratch and the chain rows are only 8-byte aligned for some sizes
-  const bool whole = sk == 1 && k0 + 64 <= Ke;
-  const bool vec = whole && ((reinterpret_cast<uintptr_t>(src) & 15u) | (sr & 3)) == 0;
-  const bool vec2 = whole && ((reinterpret_cast<uintptr_t>(src) & 7u) | (sr & 1)) == 0;
-  const bool by_rows = sk != 1;  // consecutive rows contiguous (or neither): the lanes take rows
+
+  // The chunk's row and its place in the row; by_rows: the lanes take rows.
+  static __device__ __forceinline__ int row(int i, bool by_rows) { return by_rows ? i % ROWS : i >> 3; }
+  static __device__ __forceinline__ int place(int i, bool by_rows) { return by_rows ? i / ROWS : i & 7; }
+
+  __device__ __forceinline__ void load(const float* src, int sr, int sk, int r0, int R, int k0, int Ke, int tid) {
+    // uniform; the training scratch and the chain rows are only 8-byte aligned for some sizes
+    const bool whole = sk == 1 && k0 + 64 <= Ke;
+    const bool vec = whole && ((reinterpret_cast<uintptr_t>(src) & 15u) | (sr & 3)) == 0;
+    const bool vec2 = whole && ((reinterpret_cast<uintptr_t>(src) & 7u) | (sr & 1)) == 0;
+    const bool by_rows = sk != 1;  // consecutive rows contiguous (or neither)
 #pragma unroll
-  for (int e = 0; e < kChunks; ++e) {
-    const int i = tid + kTcThreads * e;
-    const int r = by_rows ? i % ROWS : i >> 3, c = by_rows ? i / ROWS : i & 7;
-    const bool rin = r0 + r < R;
-    const float* q = src + (size_t)(r0 + r) * sr + (size_t)(k0 + 8 * c) * sk;
-    if (vec) {
-      const float4 lo = rin ? __ldg(reinterpret_cast<const float4*>(q)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 hi = rin ? __ldg(reinterpret_cast<const float4*>(q) + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[e][0] = lo.x, v[e][1] = lo.y, v[e][2] = lo.z, v[e][3] = lo.w;
-      v[e][4] = hi.x, v[e][5] = hi.y, v[e][6] = hi.z, v[e][7] = hi.w;
-    } else if (vec2) {
+    for (int e = 0; e < kChunks; ++e) {
+      const int i = tid + kTcThreads * e, r = row(i, by_rows), c = place(i, by_rows);
+      const bool rin = r0 + r < R;
+      const float* q = src + (size_t)(r0 + r) * sr + (size_t)(k0 + 8 * c) * sk;
+      if (vec) {
+        const float4 lo = rin ? reinterpret_cast<const float4*>(q)[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 hi = rin ? reinterpret_cast<const float4*>(q)[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[e][0] = lo.x, v[e][1] = lo.y, v[e][2] = lo.z, v[e][3] = lo.w;
+        v[e][4] = hi.x, v[e][5] = hi.y, v[e][6] = hi.z, v[e][7] = hi.w;
+      } else if (vec2) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 two = rin ? __ldg(reinterpret_cast<const float2*>(q) + j) : make_float2(0.f, 0.f);
-        v[e][2 * j] = two.x, v[e][2 * j + 1] = two.y;
+        for (int j = 0; j < 4; ++j) {
+          const float2 two = rin ? reinterpret_cast<const float2*>(q)[j] : make_float2(0.f, 0.f);
+          v[e][2 * j] = two.x, v[e][2 * j + 1] = two.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[e][j] = rin && k0 + 8 * c + j < Ke ? q[(size_t)j * sk] : 0.f;
       }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[e][j] = rin && k0 + 8 * c + j < Ke ? __ldg(q + (size_t)j * sk) : 0.f;
     }
   }
+
+  // Rounded to bf16 into an SW128 K-major tile.
+  __device__ __forceinline__ void put(uint8_t* tile, int sk, int tid) const {
 #pragma unroll
-  for (int e = 0; e < kChunks; ++e) {
-    const int i = tid + kTcThreads * e;
-    const int r = by_rows ? i % ROWS : i >> 3, c = by_rows ? i / ROWS : i & 7;
-    *reinterpret_cast<uint4*>(tile + umma::sw128_offset(r, 8 * c, ROWS)) =
-        make_uint4(bf16x2_bits(v[e][0], v[e][1]), bf16x2_bits(v[e][2], v[e][3]), bf16x2_bits(v[e][4], v[e][5]),
-                   bf16x2_bits(v[e][6], v[e][7]));
+    for (int e = 0; e < kChunks; ++e) {
+      const int i = tid + kTcThreads * e, r = row(i, sk != 1), c = place(i, sk != 1);
+      *reinterpret_cast<uint4*>(tile + umma::sw128_offset(r, 8 * c, ROWS)) =
+          make_uint4(bf16x2_bits(v[e][0], v[e][1]), bf16x2_bits(v[e][2], v[e][3]), bf16x2_bits(v[e][4], v[e][5]),
+                     bf16x2_bits(v[e][6], v[e][7]));
+    }
   }
-}
+};
 
 // The tile of columns n0 .., rows m0 .., from K split `split` of `splits`.
 template <int EPI>
@@ -860,8 +868,12 @@ __device__ __forceinline__ void tc_tile(const GemmArgs& G, int n0, int m0, int s
     uint8_t* ta = sm + buf * (kTcA + kTcB);
     uint8_t* tb = ta + kTcA;
     const int k0 = kb + 64 * s;
-    tc_stage<128>(ta, G.A, G.sam, G.sak, m0, G.M, k0, ke, tid);
-    tc_stage<kTcN>(tb, G.B, G.sbn, G.sbk, n0, G.N, k0, ke, tid);
+    TcChunks<128> a;  // both operands' loads before the first conversion
+    TcChunks<kTcN> b;
+    a.load(G.A, G.sam, G.sak, m0, G.M, k0, ke, tid);
+    b.load(G.B, G.sbn, G.sbk, n0, G.N, k0, ke, tid);
+    a.put(ta, G.sak, tid);
+    b.put(tb, G.sbk, tid);
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
@@ -952,11 +964,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_back_kernel(const GemmArgs Z, c
 // addition to the loss per row cost 12 us for 4096 rows, a pass per column
 // sum 12 to 20 us.)
 constexpr int kHeadWarps = 8;
-__global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const float* __restrict__ Z2,
-                                                               const float* __restrict__ P,
-                                                               const float* __restrict__ y, float* __restrict__ d,
-                                                               float* __restrict__ dZ2, float* __restrict__ grads,
-                                                               float* __restrict__ loss) {
+__global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const float* Z2, const float* P, const float* y,
+                                                               float* __restrict__ d, float* __restrict__ dZ2,
+                                                               float* __restrict__ grads, float* __restrict__ loss) {
   chain_begin();
   constexpr int kC = kH / 32;
   __shared__ float s_w3[kHeadWarps][kH], s_b2[kHeadWarps][kH], s_loss[kHeadWarps], s_b3[kHeadWarps];
@@ -1024,7 +1034,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const floa
 // Adam (Kingma & Ba) with bias correction; the step number is counters[1] + 1.
 // Each new weight also goes into the tensor-core images (as pack_kernel puts it),
 // and the last block to finish advances the counter and hands the loss out.  done: 0.
-__global__ void update_kernel(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ Mo,
+__global__ void update_kernel(float* __restrict__ P, const float* G, float* __restrict__ Mo,
                               float* __restrict__ V, float lr, float b1, float b2, float eps, uint64_t* counters,
                               uint8_t* __restrict__ w2_img, uint8_t* __restrict__ w1a_img, const float* loss,
                               float* loss_out, uint32_t* done) {

@@ -31,7 +31,11 @@ enum : uint32_t {
 // First in a kernel launched by launch_chained: lets the next kernel of the chain be
 // brought onto the SMs, then waits until the one before has finished and its
 // writes are visible.  Nothing before it in the kernel may touch memory or hold
-// tensor memory.  Without effect in a kernel launched otherwise.
+// tensor memory.  Without effect in a kernel launched otherwise.  Such a kernel
+// lives while the ones before it still write, so it reads nothing of theirs through
+// the read-only path: no __ldg and no `const T* __restrict__` in its parameters or in
+// what it passes them to (its outputs may be restricted); the wait orders ordinary
+// loads only.
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
