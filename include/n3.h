@@ -85,12 +85,17 @@ int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* 
  * plus the column-range / duplicate-point checks.  scores = determinant E,
  * badness = slope badness, or NULL: then the slope side counts E alone.
  * *mismatch (device int32, accumulated, caller zeroes it) counts states whose
- * two counts differ;
+ * two counts differ or whose badness does not sum to 3E;
  * *error_word (device uint32, OR-ed, caller zeroes it, may be NULL) collects
  * the device error bits (1: column range, 2: duplicate point, 4: mismatch).  The reference runs this audit on the host
  * (src/no_three_75/gpu.py:131 exact_match, src/no_three_75/tempering.py:193-204). */
 int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness,
                      int32_t* mismatch, uint32_t* error_word, void* stream);
+
+/* The rule by which n3_score_checked judges a state, on the host: 0, or the
+ * mismatch bit (4) if the two counts of E differ or, with has_badness, the
+ * badness does not sum to 3E. */
+int n3_checked_error(int determinant_e, int slope_e, int has_badness, int badness_sum);
 
 /* ---------------------------------------------------------------------------
  * (b) Exact incremental swap deltas.

@@ -37,6 +37,7 @@ _SIGNATURES: dict[str, list] = {
     "n3_score_columns": [_P, _I, _I, _P, _P, _P],
     "n3_score_slope": [_P, _I, _I, _P, _P, _P],
     "n3_score_checked": [_P, _I, _I, _P, _P, _P, _P, _P],
+    "n3_checked_error": [_I, _I, _I, _I],
     "n3_calibrate_det_ceiling": [_I, _I, _P, _P],
     "n3_calibrate_int_pipe": [_I, _I, _I, _P, _P],
     "n3_calibrate_l2_gather": [_P, _I64, _I, _I, _P, _P],

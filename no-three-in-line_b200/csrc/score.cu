@@ -188,8 +188,8 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
 //            counted by determinants (det_state), so the results are the
 //            determinant count's for every input.
 //   kSlope   the same, but such a state gets -1 (and the error bits, if wanted).
-//   kChecked compared with the determinant counts already in `scores` (written
-//            by det_kernel on the same stream).
+//   kChecked E and the badness's sum compared with the determinant counts already
+//            in `scores` (written by det_kernel on the same stream).
 enum TagMode { kCount, kSlope, kChecked };
 constexpr int kTagWarps = 28;  // 28 x 148 = 4144 states at once; 32 would need 6.4 KB each beside the table
 constexpr int kTagMaxParts = 16;     // warps that share a state
@@ -285,16 +285,23 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
       __syncwarp();
     }
     if (part == 0) {
+      int bad_sum = 0;
+      if (BAD)
+        for (int s = lane; s < m; s += 32) {
+          const int v = (int)bad[s];
+          badness[(size_t)b * m + s] = v;
+          bad_sum += v;
+        }
       if (MODE == kChecked) {  // scores[b] holds the determinant count of this state
-        if (lane == 0 && e != scores[b]) {
+        if (BAD) bad_sum = warp_sum(bad_sum);
+        const uint32_t differ = checked_error(scores[b], e, BAD, bad_sum);
+        if (lane == 0 && differ) {
           atomicAdd(mismatch, 1);
-          if (error_word) atomicOr(error_word, kErrMismatch);
+          if (error_word) atomicOr(error_word, differ);
         }
       } else if (lane == 0) {
         scores[b] = e;
       }
-      if (BAD)
-        for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = (int)bad[s];
     }
     group_sync();
   }
@@ -304,10 +311,10 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
 // multiply-add pipe (71 % of issue slots used), the tags for shared memory (70 %), so
 // `tag_warps` of a CTA's 32 warps take the tags and the rest the determinants, a
 // quarter of a state's pivot rows at a time.  A CTA owns `per` consecutive states
-// and compares the two counts kCheckedStates states at a time.
+// and compares the counts (checked_error) kCheckedStates states at a time.
 constexpr int kCheckedStates = 56;
 struct CheckedShared {
-  int det[kCheckedStates], slope[kCheckedStates];
+  int det[kCheckedStates], slope[kCheckedStates], bad_sum[kCheckedStates];
   uint32_t err[kCheckedStates], off_grid[kCheckedStates];
   int next_det, next_tag;
 };
@@ -382,12 +389,20 @@ __global__ void __launch_bounds__(1024, 1) checked_kernel(ColSource src, int B, 
         __syncwarp();
         if (!err) e = tag_state<BAD>(key, m, lut, tag, lane, word, word);
         __syncwarp();
+        int bad_sum = 0;
+        if (BAD) {
+          for (int s = lane; s < m; s += 32) {
+            const int v = err ? -1 : (int)word[s];
+            badness[(size_t)(b0 + k) * m + s] = v;
+            bad_sum += v;
+          }
+          bad_sum = warp_sum(bad_sum);
+        }
         if (lane == 0) {
           S.slope[k] = e;
+          S.bad_sum[k] = bad_sum;
           S.err[k] = err;
         }
-        if (BAD)
-          for (int s = lane; s < m; s += 32) badness[(size_t)(b0 + k) * m + s] = err ? -1 : (int)word[s];
         __syncwarp();
       }
     }
@@ -395,7 +410,7 @@ __global__ void __launch_bounds__(1024, 1) checked_kernel(ColSource src, int B, 
     for (int k = threadIdx.x; k < count; k += blockDim.x) {
       uint32_t err = S.err[k];
       scores[b0 + k] = err ? -1 : S.det[k];
-      if (!err && S.slope[k] != S.det[k]) err = kErrMismatch;
+      if (!err) err = checked_error(S.det[k], S.slope[k], BAD, S.bad_sum[k]);
       if (err) {
         atomicAdd(mismatch, 1);
         if (error_word) atomicOr(error_word, err);
@@ -576,6 +591,10 @@ int n3_score_columns(const int16_t* cols, int B, int n, int32_t* scores, int32_t
 int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
   N3_TRY(n3host::check_common(B, n, cols, scores));
   return n3host::launch_slope<n3::kSlope>(cols, B, n, scores, badness, nullptr, nullptr, (cudaStream_t)stream);
+}
+
+int n3_checked_error(int determinant_e, int slope_e, int has_badness, int badness_sum) {
+  return (int)n3::checked_error(determinant_e, slope_e, has_badness != 0, badness_sum);
 }
 
 int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,

@@ -214,6 +214,13 @@ __device__ __forceinline__ int det_state(const int* __restrict__ cs, int n, int 
   return cnt;
 }
 
+// Error bits of a state whose counts are to agree: the determinants' E, the slope
+// side's E and, if the slope side gave badness, its sum, which holds every triple
+// three times (the badness is added up beside E, so E alone would not show a slip in it).
+__host__ __device__ inline uint32_t checked_error(int det, int slope, bool has_badness, int badness_sum) {
+  return det == slope && (!has_badness || badness_sum == 3 * det) ? 0u : kErrMismatch;
+}
+
 // Normalised-slope line count of one state by tags: E for the whole warp.
 //
 // From each centre a, in slot order, the later slots k of other rows are told

@@ -98,7 +98,7 @@ def score_slope_gpu(columns, *, stream=None):
 class CheckedScores:
     scores: object      # determinant E per state
     badness: object     # slope badness per slot
-    mismatches: int     # states whose determinant and slope counts differ
+    mismatches: int     # states whose determinant and slope counts differ or whose badness does not sum to 3E
     error_word: int     # device error bits (1 column range, 2 duplicate point, 4 mismatch)
 
 
