@@ -64,7 +64,7 @@ def parse():
     ap.add_argument("--mode", choices=["checked", "det", "slope", "tempering", "learned", "time-to-target", "beam",
                                        "scan", "lines", "exhaustive"],
                     default="checked",
-                    help="kernel a step runs: fused checked scoring (default), the population count alone (det), slope only; "
+                    help="kernel a step runs: fused checked scoring (default), determinant only, slope only; "
                          "tempering / learned chain rounds; one device beam-search generation (beam); one "
                          "four-cycle + double-switch neighbourhood scan (scan); the n = 75 line tables "
                          "and both table scorers (lines); one exhaustive 2-switch beam generation (exhaustive); "
@@ -561,7 +561,7 @@ def run_lines_mode(args):
     for _ in range(max(3, args.warmup)):
         step()
     torch.cuda.synchronize()
-    want = np.asarray(gpu.score_population_gpu(p, q))
+    want = np.asarray(gpu.score_determinants_gpu(state.pq_to_columns(p, q)))
     if not (np.array_equal(pair_scores.cpu().numpy(), want) and np.array_equal(csr_scores.cpu().numpy(), want)
             and int(err.abs().sum()) == 0):
         raise AssertionError("line-table scores differ from the determinant scores")
@@ -728,7 +728,8 @@ def run_b200(args):
 
     def step():
         if args.mode == "det":
-            _lib.check(L.n3_score_columns(cols.data_ptr(), B, N, scores.data_ptr(), None, sptr), "n3_score_columns")
+            _lib.check(L.n3_score_determinants(cols.data_ptr(), B, N, scores.data_ptr(), None, sptr),
+                       "n3_score_determinants")
         elif args.mode == "slope":
             _lib.check(L.n3_score_slope(cols.data_ptr(), B, N, scores.data_ptr(), badness.data_ptr(), sptr),
                        "n3_score_slope")

@@ -73,6 +73,12 @@ int n3_score_population(const int32_t* p, const int32_t* q, int B, int n, int32_
 int n3_score_columns(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness,
                      void* stream);
 
+/* The determinant count alone, at every size: one exact cross product per triple.
+ * It shares no method with n3_score_slope, so the two check each other.
+ *   cols int16 [B][2n]     scores int32 [B]     badness int32 [B][2n] or NULL */
+int n3_score_determinants(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness,
+                          void* stream);
+
 /* Independent normalised-slope line count: for each anchor the other points
  * are grouped by gcd-reduced undirected direction (src/no_three_75/verifier_b.py:8-19);
  * badness[s] = sum over directions of C(c,2) (src/no_three_75/conflicts.py:376-378)

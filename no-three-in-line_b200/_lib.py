@@ -35,6 +35,7 @@ _SIGNATURES: dict[str, list] = {
     "n3_init_device": [],
     "n3_score_population": [_P, _P, _I, _I, _P, _P, _P],
     "n3_score_columns": [_P, _I, _I, _P, _P, _P],
+    "n3_score_determinants": [_P, _I, _I, _P, _P, _P],
     "n3_score_slope": [_P, _I, _I, _P, _P, _P],
     "n3_score_checked": [_P, _I, _I, _P, _P, _P, _P, _P],
     "n3_checked_error": [_I, _I, _I, _I],

@@ -19,8 +19,9 @@
 //   tabulated once per device by build_dir_lut_kernel.
 //
 // The plain scores (n3_score_population, n3_score_columns) take the faster of
-// the two for the grid size; n3_score_slope is the second, n3_score_checked
-// runs both and flags disagreement on the device.
+// the two for the grid size; n3_score_determinants is the first alone,
+// n3_score_slope the second, n3_score_checked runs both and flags disagreement on
+// the device.
 //
 // What bounds them, at 4096 n = 75 states:
 //   det_kernel<.., 1, false>   278 us (304 us on 32-bit integers).  Four tests are
@@ -586,6 +587,14 @@ int n3_score_population(const int32_t* p, const int32_t* q, int B, int n, int32_
 int n3_score_columns(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
   N3_TRY(n3host::check_common(B, n, cols, scores));
   return n3host::launch_count(n3::ColSource{cols}, B, n, scores, badness, (cudaStream_t)stream);
+}
+
+int n3_score_determinants(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
+  N3_TRY(n3host::check_common(B, n, cols, scores));
+  if (B == 0) return N3_OK;
+  const n3::ColSource src{cols};
+  return badness ? n3host::launch_det<n3::ColSource, true>(src, B, n, scores, badness, (cudaStream_t)stream)
+                 : n3host::launch_det<n3::ColSource, false>(src, B, n, scores, nullptr, (cudaStream_t)stream);
 }
 
 int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {

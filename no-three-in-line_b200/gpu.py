@@ -78,6 +78,26 @@ def score_columns_gpu(columns, *, badness: bool = False, stream=None):
     return (scores, bad) if badness else scores
 
 
+def score_determinants_gpu(columns, *, badness: bool = False, stream=None):
+    """The determinant count alone over slot-layout columns ([B, 2n]), whatever the grid size:
+    for a comparison with ``score_slope_gpu``, which shares no method with it."""
+    t = _lib.torch()
+    device = _lib.require_device()
+    host = not _lib.is_tensor(columns)
+    c = _lib.as_device(columns, t.int16, device)
+    if c.ndim != 2 or c.shape[1] % 2 or c.shape[1] < 4:
+        raise ValueError("columns must have shape (B, 2n) with n >= 2")
+    B, n = int(c.shape[0]), int(c.shape[1]) // 2
+    _check_n(n)
+    scores = t.empty(B, dtype=t.int32, device=device)
+    bad = t.empty((B, 2 * n), dtype=t.int32, device=device) if badness else None
+    _lib.call("n3_score_determinants", _lib.ptr(c), B, n, _lib.ptr(scores), _lib.ptr(bad), _lib.stream_ptr(stream))
+    if host:
+        out = scores.cpu().numpy()
+        return (out, bad.cpu().numpy()) if badness else out
+    return (scores, bad) if badness else scores
+
+
 def score_slope_gpu(columns, *, stream=None):
     """Normalised-slope line count: (E [B], badness [B, 2n])."""
     t = _lib.torch()

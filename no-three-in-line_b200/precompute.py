@@ -225,11 +225,10 @@ def _timed(score, calls: int) -> tuple[int, float]:
 
 def benchmark_precomputation(n: int, points) -> dict[str, object]:
     """precompute.py:92-127 with the device scorers: A the determinant count
-    (``accelerated.score_and_badness``), B the pair table, C the direction-class
+    (``gpu.score_determinants_gpu``, with badness), B the pair table, C the direction-class
     line count (the slope scorer, this engine's canonical-line form), D the CSR
     scan.  The four must agree (AssertionError otherwise)."""
-    from .accelerated import score_and_badness
-    from .gpu import score_slope_gpu
+    from .gpu import score_determinants_gpu, score_slope_gpu
     from .state import pq_to_columns, points_to_permutations
 
     pq = points_to_permutations(points, n)
@@ -237,12 +236,12 @@ def benchmark_precomputation(n: int, points) -> dict[str, object]:
     columns = pq_to_columns(p[None], q[None])
     tables = build_geometry_tables(n)
     scorers = {  # name in the result -> (scorer, calls timed)
-        "A_numba_determinants": (lambda: score_and_badness(p, q)[0], 100),
+        "A_numba_determinants": (lambda: score_determinants_gpu(columns, badness=True)[0][0], 100),
         "B_pair_to_line": (lambda: score_pair_table(points, tables), 100),
         "C_canonical_line_dict": (lambda: score_slope_gpu(columns)[0][0], 5),
         "D_csr_line_scan": (lambda: score_csr(points, tables), 20),
     }
-    score_and_badness(p, q)  # first launch outside the timing
+    score_determinants_gpu(columns, badness=True)  # first launch outside the timing
     results = {name: _timed(fn, calls) for name, (fn, calls) in scorers.items()}
     scores = {score for score, _ in results.values()}
     if len(scores) != 1:

@@ -670,7 +670,9 @@ class TemperingChains:
         rngs = np.asarray(z["rngs"], np.uint64) if "rngs" in z else np.zeros(1, np.uint64)
         obj = cls(cols, np.asarray(z["temperatures"]), int(rngs[0]))
         # the reference's chains sit at their replica positions: identity labels
-        scores, bad = obj.energy.cpu().numpy(), obj.badness_dev.cpu().numpy()[:, :cols.shape[1]]
+        from .gpu import score_determinants_gpu
+
+        scores, bad = score_determinants_gpu(np.asarray(cols, np.int16), badness=True)
         if "scores" in z and not np.array_equal(np.asarray(z["scores"], np.int64), scores.astype(np.int64)):
             raise AssertionError("checkpoint scores differ from the full determinant check")
         if "badness" in z and not np.array_equal(np.asarray(z["badness"], np.int64), bad.astype(np.int64)):
