@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
       const int c = cols[(size_t)b * m + s];
       const bool on_grid = c >= 0 && c < n;
       regular = regular && on_grid;
-      S.cs[s] = (uint8_t)min(max(c, 0), n - 1);
+      S.cs[s] = (uint8_t)min(max(c, 0), kMaxN - 1);  // the histograms take columns beyond n as well
       if (cover && on_grid) {
         atomicAdd(&S.columns[c], 1);
         const int cell = (s >> 1) * n + c;
