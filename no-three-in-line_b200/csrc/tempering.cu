@@ -317,9 +317,9 @@ __global__ void __launch_bounds__(512, 1) temper_kernel(const TemperArgs A) {
   W.cs = cs;
   W.bs = bs;
   for (int i = lane; i < kRegionWords; i += 32) region[i] = 0u;
-  // The state; a column off the grid stops the chain (error bit 1), and columns
-  // that do not hold two points each, or a cell that holds two, keep it from the
-  // cover table.
+  // The state; a column off the largest grid stops the chain (error bit 1), and one
+  // off the state's own, columns that do not hold two points each, or a cell that
+  // holds two, keep it from the cover table.
   bool on_grid = true, factor = true;
 #pragma unroll
   for (int t = 0; t < kSlotsPerLane; ++t) {
@@ -327,7 +327,8 @@ __global__ void __launch_bounds__(512, 1) temper_kernel(const TemperArgs A) {
     W.key2[t] = 0;
     if (s < m) {
       const int col = ch.cols[(size_t)c * kMaxM + s];
-      on_grid = on_grid && col >= 0 && col < n;
+      on_grid = on_grid && col >= 0 && col < kMaxN;
+      factor = factor && col < n;
       W.key2[t] = 2 * ((s >> 1) * kLutW + col);
       cs[s] = (uint8_t)col;
       bs[s] = ch.badness[(size_t)c * kMaxM + s];

@@ -5,7 +5,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from no_three_in_line_b200 import accelerated, gpu, gpu_delta, state
+from no_three_in_line_b200 import accelerated, gpu, gpu_delta, state, tempering
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +32,36 @@ def test_partner_scores(n, oracle, cuda):
         assert np.array_equal(line[legal], want[legal]) and (line[~legal] == gpu_delta.SENTINEL).all()
     one = accelerated.evaluate_two_switches(p[1], q[1], 3, int(E[1]), bad[1])
     assert np.array_equal(one, oracle.two_switches(p[1], q[1], 3, int(E[1]), bad[1].astype(np.int64)))
+
+
+@pytest.mark.parametrize("bad_bias", [0, 85])
+def test_tempering(bad_bias, oracle, cuda):
+    """Chains whose columns were set by hand: the walk of the oracle, and no error bit."""
+    import torch
+
+    n, L = 20, 8
+    p, q = state.seeded_population(n, L)
+    ch = tempering.TemperingChains(state.pq_to_columns(p, q), np.geomspace(0.1, 4.0, L), 7, ladder_size=L)
+    cols = state.pq_to_columns(3 * p, 3 * q)
+    E, bad = gpu.score_columns_gpu(cols, badness=True)
+    ch.cols[:, :2 * n] = torch.from_numpy(cols).cuda()
+    ch.badness_dev[:, :2 * n] = torch.from_numpy(bad).cuda()
+    ch.energy.copy_(torch.from_numpy(E))
+    ch.best_energy.copy_(ch.energy)
+    ch.best_cols.copy_(ch.cols)
+    g = lambda x: x.cpu().numpy()  # noqa: E731
+    take = lambda: {"cols": g(ch.cols).astype(np.int32), "bad": g(ch.badness_dev), "E": g(ch.energy),  # noqa: E731
+                    "bestE": g(ch.best_energy), "best_cols": g(ch.best_cols).astype(np.int32),
+                    "temp_of": g(ch.temp_of), "chain_at": g(ch.chain_at), "counter": g(ch.counter).astype(np.uint64),
+                    "accepted": g(ch.accepted_dev).astype(np.uint32), "ladder_n": g(ch.ladder_n),
+                    "ladder_round": g(ch.ladder_round).astype(np.uint32),
+                    "ladder_exch": g(ch.ladder_exchanges).astype(np.uint32)}
+    before = take()
+    ch.run(30, exchange_every=15, graph=False, bad_bias=bad_bias)
+    want = oracle.temper_run(before, ladder_size=L, acc=g(ch.acc_table).view(np.uint32),
+                             exch=g(ch.exch_table).view(np.uint32), seed=ch.seed, rounds=2, round_sweeps=15,
+                             bad_bias=bad_bias)
+    after = take()
+    for k in after:
+        assert np.array_equal(after[k].astype(np.int64), np.asarray(want[k]).astype(np.int64)), k
+    assert after["accepted"].sum() > 0 and int(ch.error_word.item()) == 0
