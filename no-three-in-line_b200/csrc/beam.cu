@@ -60,8 +60,10 @@ struct MutArgs {
 };
 
 // One thread per child, the reference's draws in the reference's order.  The
-// CTA's children live in shared memory in 16 bits (slot layout s = 2 * row +
-// layer) from the parent copy to one coalesced write of their rows.  When the
+// CTA's children live in shared memory (slot layout s = 2 * row + layer) from the
+// parent copy to one coalesced write of their rows: in 16 bits (short2) in a beam,
+// whose states lie on a grid, in 32 (int2) for n3_beam_mutate, which returns any
+// columns as they came.  When the
 // parents' badness prefix sums fit in shared memory (prefix_cap parents), the CTA
 // builds them once, a warp per parent, and the roulette draw becomes a binary
 // search: with no negative badness, the linear scan `t -= bad[u]` stops at the
@@ -76,7 +78,7 @@ struct MutArgs {
 // besides is the staging, which every CTA repeats: with as many threads as spread
 // the children over the SMs once (64 .. 256), 32,768 children of 64 parents at
 // n = 75 take 31 us, 71 us in CTAs of 64.
-constexpr int kMutThreads = 256;  // at most
+constexpr int kMutThreads = 256;  // at most; half of it in 32 bits
 constexpr size_t kMutPrefixMaxBytes = 96 * 1024;
 
 constexpr size_t kMutSmemMax = sizeof(int16_t) * kMutThreads * kMaxM + kMutPrefixMaxBytes;
@@ -94,7 +96,9 @@ struct Remainder {
   }
 };
 
+template <class Row>
 __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
+  using Cell = decltype(Row::x);
   chain_begin();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_parent[kMutThreads];
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
   const int child0 = blockIdx.x * threads, child = child0 + tid;
   const int nc = min(threads, A.population - child0);
   int32_t* prefix = reinterpret_cast<int32_t*>(smem);                       // [prefix_cap][m] inclusive prefix sums
-  short2* rows = reinterpret_cast<short2*>(prefix + (size_t)A.prefix_cap * m);  // [threads][n] both layers of a row
+  Row* rows = reinterpret_cast<Row*>(prefix + (size_t)A.prefix_cap * m);  // [threads][n] both layers of a row
   uint64_t rng = A.seed ^ (0x9e3779b97f4a7c15ULL * (uint64_t)(child + 1)) ^
                  (0xbf58476d1ce4e5b9ULL * (uint64_t)(A.generation + 1));
   int parent = child;
@@ -128,7 +132,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
 #pragma unroll
     for (int k = 0; k < (kMaxN + 31) / 32; ++k) {
       const int r = lane + 32 * k;
-      if (r < n) rows[c * n + r] = make_short2((short)src_p[r], (short)src_q[r]);
+      if (r < n) rows[c * n + r] = Row{(Cell)src_p[r], (Cell)src_q[r]};
     }
   }
   bool use_prefix = parent_count <= A.prefix_cap;  // uniform
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
     if (child < parent_count) {
       if (record) A.child_nmoves[child] = 0;
     } else {
-      int16_t* cs = reinterpret_cast<int16_t*>(rows + tid * n);
+      Cell* cs = reinterpret_cast<Cell*>(rows + tid * n);
       const int32_t* bad = A.pbad + (size_t)parent * m;
       const int32_t* pre = prefix + parent * m;
       int total = 0;
@@ -213,8 +217,8 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
           const int cu = cs[u], cv = cs[v];
           if (cu == cv) continue;
           if (cv == cs[u ^ 1] || cu == cs[v ^ 1]) continue;  // the other point of each row
-          cs[u] = (int16_t)cv;
-          cs[v] = (int16_t)cu;
+          cs[u] = (Cell)cv;
+          cs[v] = (Cell)cu;
           if (record && nmoves < A.moves_cap) A.child_moves[(size_t)child * A.moves_cap + nmoves] = u | (v << 8);
           ++nmoves;
           break;
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(kMutThreads) mutate_kernel(const MutArgs A) {
     int32_t* dst_p = A.cp + (size_t)(child0 + c) * n;
     int32_t* dst_q = A.cq + (size_t)(child0 + c) * n;
     for (int r = lane; r < n; r += 32) {
-      const short2 both = rows[c * n + r];
+      const Row both = rows[c * n + r];
       dst_p[r] = both.x;
       dst_q[r] = both.y;
     }
@@ -1063,16 +1067,19 @@ namespace n3host {
 
 // mutate_kernel over `population` children; the parents' prefix sums are staged
 // when at most `parents_bound` parents fit in kMutPrefixMaxBytes.
+template <class Row>
 static int launch_mutate(n3::beam::MutArgs A, int parents_bound, cudaStream_t st) {
   using namespace n3::beam;
+  constexpr int kMost = kMutThreads * (int)sizeof(short2) / (int)sizeof(Row);
   const int m = 2 * A.n;
   const int cap = (int)(kMutPrefixMaxBytes / (sizeof(int32_t) * (size_t)m));
   A.prefix_cap = parents_bound <= cap ? parents_bound : 0;
   int threads = 64;
-  while (threads < kMutThreads && (A.population + threads - 1) / threads > sm_count()) threads *= 2;
-  const size_t bytes = (size_t)m * (sizeof(int16_t) * (size_t)threads + sizeof(int32_t) * (size_t)A.prefix_cap);
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(mutate_kernel), kMutSmemMax));
-  return launch_chained("beam mutate_kernel", mutate_kernel, (A.population + threads - 1) / threads, threads, bytes, st, A);
+  while (threads < kMost && (A.population + threads - 1) / threads > sm_count()) threads *= 2;
+  const size_t bytes = (size_t)m * (sizeof(Row) / 2 * (size_t)threads + sizeof(int32_t) * (size_t)A.prefix_cap);
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(mutate_kernel<Row>), kMutSmemMax));
+  return launch_chained("beam mutate_kernel", mutate_kernel<Row>, (A.population + threads - 1) / threads, threads, bytes,
+                        st, A);
 }
 
 static int check_beam(const n3_beam* b) {
@@ -1149,7 +1156,7 @@ int n3_beam_mutate(const int32_t* parent_p, const int32_t* parent_q, const int32
   A.cq = child_q;
   A.child_parent = A.child_moves = A.child_nmoves = nullptr;
   A.moves_cap = 0;
-  return n3host::launch_mutate(A, parent_count, (cudaStream_t)stream);
+  return n3host::launch_mutate<int2>(A, parent_count, (cudaStream_t)stream);
 }
 
 int n3_py_random_seed(uint32_t* state, uint64_t seed, void* stream) {
@@ -1212,7 +1219,7 @@ int n3_beam_generation(const n3_beam* b, int generation, void* stream) {
   M.child_moves = b->child_moves;
   M.child_nmoves = b->child_nmoves;
   M.moves_cap = b->max_strength;
-  N3_TRY(n3host::launch_mutate(M, b->elite_size, st));
+  N3_TRY(n3host::launch_mutate<short2>(M, b->elite_size, st));
   N3_TRY(n3host::ensure_device_tables());
   N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::beam::child_delta_kernel), n3::beam::kDeltaSmem));
   n3::beam::DeltaArgs D;

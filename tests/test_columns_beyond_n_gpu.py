@@ -1,11 +1,11 @@
-"""States with columns at or beyond n (below the largest grid's 75): nothing in these calls needs the columns to
-lie in the state's own grid, and they count them as they are."""
+"""States with columns at or beyond n (below the largest grid's 75), and mutation of any columns at all: nothing
+in these calls needs the columns to lie in the state's own grid, and they count them as they are."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
-from no_three_in_line_b200 import accelerated, gpu, gpu_delta, state, tempering
+from no_three_in_line_b200 import _lib, accelerated, gpu, gpu_delta, state, tempering
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,24 @@ def test_tempering(bad_bias, oracle, cuda):
     for k in after:
         assert np.array_equal(after[k].astype(np.int64), np.asarray(want[k]).astype(np.int64)), k
     assert after["accepted"].sum() > 0 and int(ch.error_word.item()) == 0
+
+
+@pytest.mark.parametrize("parents", [3, 200])  # badness sums staged in shared memory, and not
+@pytest.mark.parametrize("shift", [0, 40000, -70000, 1 << 30])
+def test_mutation_returns_any_columns(parents, shift, oracle, cuda):
+    """Draws and swaps depend on which columns are equal, not on their values."""
+    import torch
+
+    n, population = 75, 700
+    p, q = state.seeded_population(n, parents)
+    bad = gpu.score_population_gpu(p, q, badness=True)[1]
+    args = dict(quality_count=max(1, parents // 4), population=population, active_strength=4, max_strength=9,
+                bad_bias=85, seed=11, generation=3)
+    want_p, want_q = oracle.beam_mutate(p + shift, q + shift, bad, **args)
+    dp, dq, db = (torch.from_numpy(np.ascontiguousarray(x, dtype=np.int32)).cuda() for x in (p + shift, q + shift, bad))
+    cp = torch.empty((population, n), dtype=torch.int32, device="cuda")
+    cq = torch.empty_like(cp)
+    _lib.call("n3_beam_mutate", _lib.ptr(dp), _lib.ptr(dq), _lib.ptr(db), parents, args["quality_count"], n, population,
+              args["active_strength"], args["max_strength"], args["bad_bias"], args["seed"], args["generation"],
+              _lib.ptr(cp), _lib.ptr(cq), _lib.stream_ptr())
+    assert np.array_equal(cp.cpu().numpy(), want_p) and np.array_equal(cq.cpu().numpy(), want_q)
