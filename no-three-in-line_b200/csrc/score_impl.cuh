@@ -276,6 +276,7 @@ __device__ __forceinline__ int tag_state(const int (&key)[kSlotsPerLane], int m,
         if (id[t] >= 0) win[t] = vtag[id[t]];
         lose |= (unsigned)(win[t] != lane + 32 * t) << t;
       }
+      __syncwarp();  // the next centre's tags come after every lane has read this one's
       if (__any_sync(0xffffffffu, lose != 0u)) {
         uint32_t before[kT];
 #pragma unroll

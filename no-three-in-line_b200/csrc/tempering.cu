@@ -208,6 +208,7 @@ __device__ __forceinline__ void running_sums(int* __restrict__ prefix, int m, in
     if (lane >= o) run += y;
   }
   run -= local;
+  __syncwarp();  // every lane is done with the sums before
 #pragma unroll
   for (int t = 0; t < kSlotsPerLane; ++t) {
     run += val[t];
