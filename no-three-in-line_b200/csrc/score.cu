@@ -35,6 +35,7 @@
 //       memory is busy 87 % of the cycles: a direction load (3.5 cycles for 32
 //       random 2-byte words), a tag store and a tag load (2.9 each) per 32 slots.
 #include <cstdio>
+#include <type_traits>
 
 #include "score_impl.cuh"
 
@@ -128,7 +129,11 @@ struct ColSource {
 constexpr int kDetWarps = 4;  // small CTAs: 4096 states spread evenly over 148 SMs
 
 // E by determinants: on packed floats when every column lies on the grid, else
-// on 32-bit integers (det_state), as the count has always taken any columns.
+// on 32-bit integers (det_state), as the count has always taken any columns.  On
+// small grids, with a warp per state, integers are ahead whatever the columns (their
+// set-up is shorter; 20,011 states, us, packed floats against integers: n = 10 20.8
+// and 19.5, n = 14 32.4 and 31.5, n = 20 56.0 and 56.7; with badness n = 20 81.2 and
+// 83.5, but 5000 of them 28.3 and 27.1).
 // PARTS = 1: a warp per state, kDetWarps states per CTA.  PARTS > 1, for fewer
 // states than warps that the GPU can hold: a CTA of PARTS warps per state,
 // which share its pivot rows.
@@ -141,15 +146,17 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = PARTS > 1 ? blockIdx.x : blockIdx.x * kDetWarps + warp;
   if (b >= B) return;
+  constexpr int kIntegersMaxN = PARTS > 1 ? 0 : BAD ? 20 : 16;
   float4* rows4 = rows_all[PARTS > 1 ? 0 : warp];
   int* bad = BAD ? bad_all[PARTS > 1 ? 0 : warp] : nullptr;
   const int first = PARTS > 1 ? threadIdx.x : lane, stride = PARTS > 1 ? PARTS * 32 : 32;
-  bool on_grid = true;
-  for (int r = first; r < n; r += stride) {
+  bool on_grid = n > kIntegersMaxN;
+  if (BAD)
+    for (int s = first; s < 2 * n; s += stride) bad[s] = 0;
+  for (int r = first; on_grid && r < n; r += stride) {
     const int c0 = src.col(b, n, 2 * r), c1 = src.col(b, n, 2 * r + 1);
     on_grid = on_grid && (unsigned)c0 < (unsigned)kMaxN && (unsigned)c1 < (unsigned)kMaxN;
     rows4[r] = make_float4((float)c0, (float)c0, (float)c1, (float)c1);
-    if (BAD) bad[2 * r] = bad[2 * r + 1] = 0;
   }
   if (PARTS > 1) {
     if (threadIdx.x == 0) total = 0;
@@ -180,10 +187,12 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
     for (int s = first; s < 2 * n; s += stride) badness[(size_t)b * 2 * n + s] = bad[s];
 }
 
-// The slope count (tag_state): up to kTagWarps warps share one compact direction
-// table, `parts` warps (a power of two) a state, which share its centres, so that
-// few states fill the SMs too (64 n = 75 states: 8.4 us; 51 us with a warp each);
-// with enough states for every warp, parts is 1.
+// The slope count (tag_state): the warps of a CTA share one compact direction table
+// and take consecutive states, a warp each; where fewer states than warps are left,
+// `parts` warps (a power of two) share a state's centres, so that few states fill
+// the SMs too (64 n = 75 states with badness: 8.9 us; 51 us with a warp each) and a batch just above
+// a round of all warps does not cost two (4300 n = 75 states with badness: 96 us,
+// 167 with the last 156 states on six CTAs, a warp each).
 //   kCount   E and, if wanted, badness of any states: one with a column off the
 //            grid or two equal points in a row, which has no line count, is
 //            counted by determinants (det_state), so the results are the
@@ -191,22 +200,38 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
 //   kSlope   the same, but such a state gets -1 (and the error bits, if wanted).
 //   kChecked E and the badness's sum compared with the determinant counts already
 //            in `scores` (written by det_kernel on the same stream).
+// NT, the slots a lane holds, bounds the unrolled work per centre and, with the ids of
+// the directions that a grid of 16 NT rows has, a warp's shared memory: 32 warps fit
+// up to n = 48 (4096 n = 14 states with badness: 8.6 us, 16.4 with NT = 5 and 28 warps).
 enum TagMode { kCount, kSlope, kChecked };
-constexpr int kTagWarps = 28;  // 28 x 148 = 4144 states at once; 32 would need 6.4 KB each beside the table
+// What a CTA does with its states: whole rounds of a warp each, a state shared by several
+// warps, or rounds and then the last states shared.  (A kernel that can do both takes 2
+// to 10 % longer where it needs only one.)
+enum TagPlan { kRounds, kShared, kRoundsThenShared };
 constexpr int kTagMaxParts = 16;     // warps that share a state
 constexpr int kTagMinThreads = 256;  // threads that copy the table when few states are scored
-__host__ __device__ constexpr size_t tag_smem(int warps) { return kCompactLutBytes + (size_t)warps * kTagWarpBytes; }
-static_assert(tag_smem(kTagWarps) <= 227 * 1024, "tag_kernel shared memory");
-static_assert(kDirCount >= (int)sizeof(int) * kMaxM, "a state's columns fit in a warp's tags");
+// Compact ids of the directions with dx < 16 NT (any dy), rounded up to 8: ids go by (dx, dy).
+__host__ __device__ constexpr int tag_ids(int nt) {
+  return nt == 1 ? 1400 : nt == 2 ? 2896 : nt == 3 ? 4352 : kDirCount;
+}
+__host__ __device__ constexpr int tag_warps(int nt) { return nt <= 3 ? 32 : 28; }  // 28 x 148 = 4144 states at once
+__host__ __device__ constexpr size_t tag_warp_bytes(int nt) { return tag_ids(nt) + sizeof(uint32_t) * 32 * nt; }
+__host__ __device__ constexpr size_t tag_smem(int nt, int warps) {
+  return kCompactLutBytes + (size_t)warps * tag_warp_bytes(nt);
+}
+static_assert(tag_smem(3, tag_warps(3)) <= 227 * 1024 && tag_smem(5, tag_warps(5)) <= 227 * 1024,
+              "tag_kernel shared memory");
+static_assert(tag_ids(1) >= (int)sizeof(int) * 32 && tag_ids(2) >= (int)sizeof(int) * 64, "columns fit in a warp's tags");
+static_assert(tag_ids(1) % 8 == 0 && tag_ids(2) % 8 == 0 && tag_ids(3) % 8 == 0 && tag_ids(5) % 8 == 0, "alignment");
 
 // State b's table keys for tag_state, its word[] cleared; returns the error bits of
 // columns outside [0, limit) and equal points in a row (the same in every lane).
-template <class Src>
-__device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int limit, int lane,
-                                             int (&key)[kSlotsPerLane], uint32_t* __restrict__ word) {
+template <class Src, int NT>
+__device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int limit, int lane, int (&key)[NT],
+                                             uint32_t* __restrict__ word) {
   uint32_t err = 0;
 #pragma unroll
-  for (int t = 0; t < kSlotsPerLane; ++t) {
+  for (int t = 0; t < NT; ++t) {
     const int s = lane + 32 * t;
     const bool in = s < 2 * n;
     const int c = in ? src.col(b, n, s) : 0;
@@ -220,50 +245,72 @@ __device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int l
   return __reduce_or_sync(0xffffffffu, err);
 }
 
-template <class Src, int MODE, bool BAD, bool SPLIT>
-__global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, int n, int W, int parts,
-                                                                 const uint16_t* __restrict__ g_lut,
-                                                                 int32_t* __restrict__ scores,
-                                                                 int32_t* __restrict__ badness,
-                                                                 int32_t* __restrict__ mismatch,
-                                                                 uint32_t* __restrict__ error_word) {
+// The states without a line count among first, first + step, ... below end, and
+// `extra` if it is not negative, by determinants.  Called once at a warp's end, so that
+// the code of these rare states takes no registers from tag_kernel's loops (inlined
+// there it cost 20,011 n = 17 states 47 us against 36).
+template <class Src, bool BAD>
+static __device__ __noinline__ void count_rare(Src src, int n, int lane, int first, int end, int step, int extra,
+                                               int* __restrict__ cs, int* __restrict__ bad,
+                                               int32_t* __restrict__ scores, int32_t* __restrict__ badness) {
+  for (int i = first;; i += step) {
+    const int b = i < end ? i : extra;
+    bool rare = false;
+    for (int r = lane; b >= 0 && r < n; r += 32) {
+      const int c0 = src.col(b, n, 2 * r), c1 = src.col(b, n, 2 * r + 1);
+      rare = rare || (unsigned)c0 >= (unsigned)kMaxN || (unsigned)c1 >= (unsigned)kMaxN || c0 == c1;
+    }
+    if (__any_sync(0xffffffffu, rare)) {
+      for (int s = lane; s < 2 * n; s += 32) {
+        cs[s] = src.col(b, n, s);
+        if (BAD) bad[s] = 0;
+      }
+      __syncwarp();
+      const int e = warp_sum(det_state<BAD>(cs, n, lane, bad));
+      if (lane == 0) scores[b] = e;
+      __syncwarp();
+      if (BAD)
+        for (int s = lane; s < 2 * n; s += 32) badness[(size_t)b * 2 * n + s] = bad[s];
+      __syncwarp();
+    }
+    if (i >= end) return;
+  }
+}
+
+template <class Src, int MODE, bool BAD, int NT, int PLAN>
+__global__ void __launch_bounds__(tag_warps(NT) * 32, 1) tag_kernel(Src src, int B, int n, int W,
+                                                                     const uint16_t* __restrict__ g_lut,
+                                                                     int32_t* __restrict__ scores,
+                                                                     int32_t* __restrict__ badness,
+                                                                     int32_t* __restrict__ mismatch,
+                                                                     uint32_t* __restrict__ error_word) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int total_all[kTagWarps];
+  __shared__ int total_all[tag_warps(NT)];
+  __shared__ volatile uint8_t rare[tag_warps(NT)];  // kCount: the warp met a state without a line count
   uint16_t* lut = reinterpret_cast<uint16_t*>(smem);
   compact_lut_copy(lut, g_lut);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp >= W) return;  // it only helped to copy the table
   const int m = 2 * n;
-  if (!SPLIT) parts = 1;
-  const int group = warp / parts, part = warp % parts;
-  uint8_t* tag = smem + kCompactLutBytes + (size_t)warp * kTagWarpBytes;
-  // the group's badness and count live with its first warp
-  uint32_t* word = reinterpret_cast<uint32_t*>(tag + kDirCount);
-  uint32_t* bad = reinterpret_cast<uint32_t*>(smem + kCompactLutBytes + (size_t)group * parts * kTagWarpBytes + kDirCount);
-  int* total = total_all + group;
-  auto group_sync = [&]() {  // at most 14 groups of more than one warp: barrier ids 1 .. 14
-    if (!SPLIT)
-      __syncwarp();
-    else
-      asm volatile("barrier.sync %0, %1;" ::"r"(1 + group), "r"(32 * parts) : "memory");
-  };
-  for (int b = blockIdx.x * (W / parts) + group; b < B; b += gridDim.x * (W / parts)) {
-    int key[kSlotsPerLane];
-    const uint32_t err = tag_load(src, b, n, MODE == kCount ? kMaxN : n, lane, key, word);
-    if (part == 0 && lane == 0) *total = 0;
-    group_sync();
+  uint8_t* tag = smem + kCompactLutBytes + (size_t)warp * tag_warp_bytes(NT);
+  uint32_t* word = reinterpret_cast<uint32_t*>(tag + tag_ids(NT));
+  if (MODE == kCount && lane == 0) rare[warp] = 0;
+
+  // State b by `parts` warps, this one `part` of them; the group's badness and count live with its first
+  // warp.  sync: the group's barrier.
+  const auto score = [&](auto split, int b, int group, int part, int parts, const auto& sync) {
+    constexpr bool SPLIT = decltype(split)::value;
+    uint32_t* bad = word - (size_t)part * (tag_warp_bytes(NT) / sizeof(uint32_t));
+    int* total = total_all + group;
+    int key[NT];
+    const uint32_t err = tag_load<Src, NT>(src, b, n, MODE == kCount ? kMaxN : n, lane, key, word);
+    if (SPLIT && part == 0 && lane == 0) *total = 0;
+    sync();
     if (err) {  // no line count exists
       if (part == 0) {
         if (MODE == kCount) {
-          int* cs = reinterpret_cast<int*>(tag);
-          for (int s = lane; s < m; s += 32) cs[s] = src.col(b, n, s);
-          __syncwarp();
-          const int e = warp_sum(det_state<BAD>(cs, n, lane, reinterpret_cast<int*>(bad)));
-          if (lane == 0) scores[b] = e;
-          __syncwarp();
-          if (BAD)
-            for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = (int)bad[s];
+          if (lane == 0) rare[warp] = 1;
         } else {
           if (lane == 0) {
             scores[b] = -1;
@@ -274,13 +321,13 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
             for (int s = lane; s < m; s += 32) badness[(size_t)b * m + s] = -1;
         }
       }
-      group_sync();
-      continue;
+      sync();
+      return;
     }
-    int e = tag_state<BAD, SPLIT>(key, m, lut, tag, lane, word, bad, part, parts);
+    int e = tag_state<BAD, SPLIT, NT>(key, m, lut, tag, lane, word, bad, part, parts);
     if (SPLIT) {
       if (lane == 0) atomicAdd(total, e);
-      group_sync();
+      sync();
       e = *total;
     } else {
       __syncwarp();
@@ -304,8 +351,31 @@ __global__ void __launch_bounds__(kTagWarps * 32, 1) tag_kernel(Src src, int B, 
         scores[b] = e;
       }
     }
-    group_sync();
+    sync();
+  };
+
+  const int b_begin = (int)((int64_t)B * blockIdx.x / gridDim.x);
+  const int b_end = (int)((int64_t)B * (blockIdx.x + 1) / gridDim.x);
+  int b = b_begin;
+  if (PLAN != kShared)
+    for (; PLAN == kRounds ? b + warp < b_end : 2 * (b_end - b) > W; b += W)
+      if (PLAN == kRounds || b + warp < b_end) score(std::false_type{}, b + warp, 0, 0, 1, [] { __syncwarp(); });
+  int shared = -1;  // the state that this warp led a group at
+  if (const int left = b_end - b; PLAN != kRounds && left > 0) {
+    int parts = 2;
+    while (parts < kTagMaxParts && 2 * parts * left <= W) parts *= 2;
+    const int group = warp / parts, part = warp % parts;
+    if (group < left) {
+      if (part == 0) shared = b + group;
+      // at most 16 groups: barrier ids 0 .. 15, the block's own is done with
+      score(std::true_type{}, b + group, group, part, parts,
+            [&] { asm volatile("barrier.sync %0, %1;" ::"r"(group), "r"(32 * parts) : "memory"); });
+    }
   }
+  __syncwarp();
+  if (MODE == kCount && rare[warp])
+    count_rare<Src, BAD>(src, n, lane, b_begin + warp, PLAN == kRounds ? b_end : b, W, shared, reinterpret_cast<int*>(tag),
+                         reinterpret_cast<int*>(word), scores, badness);
 }
 
 // Both counts of the checked score side by side: the determinants wait for the
@@ -470,23 +540,47 @@ static int check_common(int B, int n, const void* a, const void* out) {
   return N3_OK;
 }
 
+template <class Src, int MODE, bool BAD, int NT, int PLAN>
+static int launch_tag_plan(Src src, int B, int n, int W, int32_t* scores, int32_t* badness, int32_t* mismatch,
+                           uint32_t* error_word, cudaStream_t st) {
+  using namespace n3;
+  const auto kernel = tag_kernel<Src, MODE, BAD, NT, PLAN>;
+  N3_TRY(allow_smem(reinterpret_cast<const void*>(kernel), tag_smem(NT, tag_warps(NT))));
+  const int sms = sm_count(), threads = W * 32 > kTagMinThreads ? W * 32 : kTagMinThreads;
+  kernel<<<B < sms ? B : sms, threads, tag_smem(NT, W), st>>>(src, B, n, W, dir_lut_device_ptr(), scores, badness,
+                                                              mismatch, error_word);
+  return check_launch("tag_kernel");
+}
+
+template <class Src, int MODE, bool BAD, int NT>
+static int launch_tag_nt(Src src, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+                         uint32_t* error_word, cudaStream_t st) {
+  using namespace n3;
+  N3_TRY(ensure_device_tables());
+  const int sms = sm_count(), most = tag_warps(NT);
+  const int per = (B + sms - 1) / sms;  // states per SM
+  if (2 * per <= most) {
+    int parts = 2;
+    while (parts < kTagMaxParts && 2 * parts * per <= most) parts *= 2;
+    return launch_tag_plan<Src, MODE, BAD, NT, kShared>(src, B, n, per * parts, scores, badness, mismatch, error_word, st);
+  }
+  const int last = per % most;
+  if (per > most && last > 0 && 2 * last <= most)
+    return launch_tag_plan<Src, MODE, BAD, NT, kRoundsThenShared>(src, B, n, most, scores, badness, mismatch, error_word,
+                                                                  st);
+  return launch_tag_plan<Src, MODE, BAD, NT, kRounds>(src, B, n, per < most ? per : most, scores, badness, mismatch,
+                                                      error_word, st);
+}
+
 template <class Src, int MODE, bool BAD>
 static int launch_tag(Src src, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
                       uint32_t* error_word, cudaStream_t st) {
-  using namespace n3;
-  N3_TRY(ensure_device_tables());
-  const int sms = sm_count();
-  const int per = (B + sms - 1) / sms;  // states per SM
-  int parts = 1;
-  while (parts < kTagMaxParts && 2 * parts * per <= kTagWarps) parts *= 2;
-  const auto kernel = parts > 1 ? tag_kernel<Src, MODE, BAD, true> : tag_kernel<Src, MODE, BAD, false>;
-  N3_TRY(allow_smem(reinterpret_cast<const void*>(kernel), tag_smem(kTagWarps)));
-  const int groups = per * parts < kTagWarps ? per : kTagWarps / parts, W = groups * parts;
-  const int want = (B + groups - 1) / groups;
-  const int threads = W * 32 > kTagMinThreads ? W * 32 : kTagMinThreads;
-  kernel<<<want < sms ? want : sms, threads, tag_smem(W), st>>>(src, B, n, W, parts, dir_lut_device_ptr(), scores,
-                                                                badness, mismatch, error_word);
-  return check_launch("tag_kernel");
+  switch ((2 * n + 31) / 32) {
+    case 1: return launch_tag_nt<Src, MODE, BAD, 1>(src, B, n, scores, badness, mismatch, error_word, st);
+    case 2: return launch_tag_nt<Src, MODE, BAD, 2>(src, B, n, scores, badness, mismatch, error_word, st);
+    case 3: return launch_tag_nt<Src, MODE, BAD, 3>(src, B, n, scores, badness, mismatch, error_word, st);
+    default: return launch_tag_nt<Src, MODE, BAD, 5>(src, B, n, scores, badness, mismatch, error_word, st);
+  }
 }
 
 template <int MODE>
@@ -503,40 +597,66 @@ static int launch_det(Src src, int B, int n, int32_t* scores, int32_t* badness, 
   using namespace n3;
   const int sms = sm_count();
   // warps per state: 16 while two such CTAs fit every SM, 4 while eight do (64
-  // n = 75 states: 14 us against 79 us with one warp a state; 1024: 76 and 105)
+  // n = 75 states: 14 us against 79 us with one warp a state; 1024: 76 and 105), seven
+  // on the smallest grids (1184 n = 10 states: 4.5 us, 4.2 with one)
   if (B <= 2 * sms)
     det_kernel<Src, 16, BAD><<<B, 16 * 32, 0, st>>>(src, B, n, scores, badness);
-  else if (B <= 8 * sms)
+  else if (B <= (n <= 12 ? 7 : 8) * sms)
     det_kernel<Src, 4, BAD><<<B, 4 * 32, 0, st>>>(src, B, n, scores, badness);
   else
     det_kernel<Src, 1, BAD><<<(B + kDetWarps - 1) / kDetWarps, kDetWarps * 32, 0, st>>>(src, B, n, scores, badness);
   return check_launch("det_kernel");
 }
 
-// Up to these sizes the determinants are the faster count (us for 20,011
-// states, determinants against tags: E alone n = 24: 86 / 99, n = 28: 121 / 115;
-// with badness n = 20: 82 / 100, n = 24: 125 / 119): they grow with n^3, the
-// tags with n^2, but every centre costs the tags two round trips to shared
-// memory.  At 64 states the determinants stay ahead up to n = 60 by 1-2 us.
-constexpr int kDetMaxN = 26, kDetMaxNBad = 22;
+// Whether the determinants are the faster count: they grow with n^3, the tags with
+// n^2, but every centre costs the tags two round trips to shared memory, and every CTA
+// the copy of a table.  So on the smallest grids, for up to two states an SM (16 warps
+// share each) on those up to n = 28, and in between for little work.  us, determinants
+// against tags, E alone: 20,011 states n = 5 9.4 / 10.0, n = 10 20.8 / 16.2, n = 24 83 / 49;
+// n = 8, 5000 6.2 / 6.9 and 8300 8.0 / 8.0; n = 10, 4096 6.1 / 6.0; n = 12, 2100 5.3 / 5.6;
+// n = 20, 600 4.7 / 5.1 and 1184 7.7 / 6.0; n = 28, 296 4.3 / 4.7 and 297 5.8 / 4.7.  With
+// badness: 20,011 states n = 10 28 / 21, n = 20 81 / 53; n = 8, 4096 5.9 / 6.1; n = 10, 3000
+// 6.8 / 7.0; n = 12, 1036 4.5 / 4.9 and 1184 6.5 / 5.1; n = 17, 1000 6.2 / 6.5; n = 26,
+// 296 5.1 / 5.1.
+static bool determinants_faster(int B, int n, bool badness) {
+  if (n <= 5) return true;
+  if (B <= 2 * sm_count()) return n <= (badness ? 26 : 28);
+  if (n > (B <= 7 * sm_count() ? (badness ? 20 : 22) : (badness ? 10 : 12))) return false;
+  return (int64_t)B * n * n <= (badness ? 300000 : 400000);
+}
 
 template <class Src>
 static int launch_count(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
   if (B == 0) return N3_OK;
+  const bool det = determinants_faster(B, n, badness != nullptr);
   if (badness)
-    return n <= kDetMaxNBad ? launch_det<Src, true>(src, B, n, scores, badness, st)
-                         : launch_tag<Src, n3::kCount, true>(src, B, n, scores, badness, nullptr, nullptr, st);
-  return n <= kDetMaxN ? launch_det<Src, false>(src, B, n, scores, nullptr, st)
-                       : launch_tag<Src, n3::kCount, false>(src, B, n, scores, nullptr, nullptr, nullptr, st);
+    return det ? launch_det<Src, true>(src, B, n, scores, badness, st)
+               : launch_tag<Src, n3::kCount, true>(src, B, n, scores, badness, nullptr, nullptr, st);
+  return det ? launch_det<Src, false>(src, B, n, scores, nullptr, st)
+             : launch_tag<Src, n3::kCount, false>(src, B, n, scores, nullptr, nullptr, nullptr, st);
+}
+
+template <class Src, int MODE, int NT, int PLAN>
+static int prepare_tag_plan() {
+  using namespace n3;
+  const size_t smem = tag_smem(NT, tag_warps(NT));
+  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, true, NT, PLAN>), smem)));
+  return allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, NT, PLAN>), smem);
+}
+
+template <class Src, int MODE, int NT>
+static int prepare_tag_nt() {
+  N3_TRY((prepare_tag_plan<Src, MODE, NT, n3::kRounds>()));
+  N3_TRY((prepare_tag_plan<Src, MODE, NT, n3::kShared>()));
+  return prepare_tag_plan<Src, MODE, NT, n3::kRoundsThenShared>();
 }
 
 template <class Src, int MODE>
 static int prepare_tag() {
-  using namespace n3;
-  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, true, true>), tag_smem(kTagWarps))));
-  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, true, false>), tag_smem(kTagWarps))));
-  N3_TRY((allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, true>), tag_smem(kTagWarps))));
-  return allow_smem(reinterpret_cast<const void*>(tag_kernel<Src, MODE, false, false>), tag_smem(kTagWarps));
+  N3_TRY((prepare_tag_nt<Src, MODE, 1>()));
+  N3_TRY((prepare_tag_nt<Src, MODE, 2>()));
+  N3_TRY((prepare_tag_nt<Src, MODE, 3>()));
+  return prepare_tag_nt<Src, MODE, 5>();
 }
 
 // The two counts of the checked score in one kernel (checked_kernel) for many

@@ -235,6 +235,7 @@ __host__ __device__ inline uint32_t checked_error(int det, int slope, bool has_b
 // byte of their winner's word: a direction of c slots has c - 1 losers, which
 // find 0, 1, ... there and add 1 + 2 + ... = C(c, 2) triples.
 //
+// NT: the slots a lane may hold, at least ceil(m / 32).
 // key: this lane's slots' table keys row * kLutW + column, negative beyond m.
 // lut: the compact direction table in shared memory, whose entry of the
 // difference d = key(k) - key(a) > 0 is lut[d + kMaxN - 1].  tag: this warp's
@@ -246,11 +247,11 @@ constexpr size_t kTagWarpBytes = kDirCount + sizeof(uint32_t) * kMaxM;  // the t
 // two up to 32), so that `parts` warps can share a state.  Each then counts its
 // losers in words of its own, and the badness of all goes to `bad`, the first
 // warp's (only that warp touches a top byte there).
-template <bool BAD, bool SPLIT = false>
-__device__ __forceinline__ int tag_state(const int (&key)[kSlotsPerLane], int m, const uint16_t* __restrict__ lut,
+template <bool BAD, bool SPLIT = false, int NT = kSlotsPerLane>
+__device__ __forceinline__ int tag_state(const int (&key)[NT], int m, const uint16_t* __restrict__ lut,
                                          uint8_t* __restrict__ tag, int lane, uint32_t* word, uint32_t* bad,
                                          int part = 0, int parts = 1) {
-  constexpr int kT = kSlotsPerLane;
+  constexpr int kT = NT;
   constexpr uint32_t kOne = 1u << 24;
   volatile uint8_t* vtag = tag;
   int total = 0;  // this lane's triples
