@@ -24,6 +24,8 @@
 // A second, independent kernel evaluates the reference formulation literally
 // (every pair (i<j) outside {u,v} tested against u, u', v, v' with int32 cross
 // products, plus every k against (u,v) and (u',v')); tests compare the two.
+#include <type_traits>
+
 #include "cover.cuh"
 #include "dirs.cuh"
 #include "n3_common.cuh"
@@ -289,10 +291,17 @@ __global__ void __launch_bounds__(kDeltaWarps * 32, 1) swap_delta_kernel(const M
 //       so a walk per lane took 8 us more); the last anchors of a run share
 //       their partners among the warps left (4 us)
 //   fewer               a warp per partner, both new centres' histograms side by
-//       side (pair_move.cuh), whatever the columns hold
+//       side (pair_move.cuh), whatever the columns hold; each warp holds the state
+//       itself, so that short runs follow each other without a barrier, and the next
+//       run's first partners go to the warps that the last one left idle (512 n = 20
+//       states with a slot each: 14.0 us, 17.7 with the state shared by the CTA, 14.8 with
+//       a CTA of eight warps per anchor)
 // 64 n = 75 states, every slot: 70 us, 834 us with two histograms per partner one
 // after the other; 1024 states with a slot each, partners of its layer: 48 and 60 us.
 constexpr int kPartnerWarps = 24;
+// Anchors of one state from which its cover table is built (512 states, us: n = 75, 5 anchors each by
+// pairs 177, 7 by pairs 245, 8 by the table 142; n = 40 74, 100, 57; n = 20 38, 50, 30; n = 10 18, 23, 19;
+// n = 4 13, 15, 17: from five on the table would do as well on larger grids).
 constexpr int kRunCover = 8;
 constexpr int kPartnerRegion = ((kMaxN * kMaxN + 1) / 2 + 3) / 4 * 4;  // words of the cover table
 
@@ -312,9 +321,10 @@ static_assert(sizeof(PartnerSmem) <= 227 * 1024, "partner_scores_kernel shared m
 
 // One partner's score by 8-bit histograms over A, one centre at a time: for equal
 // columns and where a 4-bit counter may have wrapped.
-__device__ __noinline__ int partner_by_histograms(const PartnerSmem& S, uint32_t* __restrict__ hist, int m, int u,
-                                                  int v, int cur, int bad_uv, int lane) {
-  const int ru = u >> 1, rv = v >> 1, cu = S.cs[u], cv = S.cs[v];
+__device__ __noinline__ int partner_by_histograms(const uint16_t* __restrict__ lut4, const uint8_t* __restrict__ cs,
+                                                  uint32_t* __restrict__ hist, int m, int u, int v, int cur,
+                                                  int bad_uv, int lane) {
+  const int ru = u >> 1, rv = v >> 1, cu = cs[u], cv = cs[v];
   int part = 0, j_new = 0;
   for (int c = 0; c < 2; ++c) {
     const int rx = c ? rv : ru, centre = c ? rv * kLutW + cu : ru * kLutW + cv;
@@ -324,16 +334,16 @@ __device__ __noinline__ int partner_by_histograms(const PartnerSmem& S, uint32_t
       const int k = lane + 32 * t;
       ids[t] = -1;
       if (k < m && k != u && k != v && (k >> 1) != rx) {
-        const int ck = S.cs[k];
-        ids[t] = (int)(dir4(S.dir4, (k >> 1) * kLutW + ck, centre) >> 2);
+        const int ck = cs[k];
+        ids[t] = (int)(dir4(lut4, (k >> 1) * kLutW + ck, centre) >> 2);
         part += hist_add(hist, ids[t]);
         if (c == 0) part += ((rv - ru) * (ck - cu) == (cv - cu) * ((k >> 1) - ru)) << 16;  // joint
       } else if (c == 0 && k < m && k != u && k != v) {  // u's row partner
-        part += ((rv - ru) * (S.cs[k] - cu) == (cv - cu) * ((k >> 1) - ru)) << 16;
+        part += ((rv - ru) * (cs[k] - cu) == (cv - cu) * ((k >> 1) - ru)) << 16;
       }
     }
     __syncwarp();
-    if (c == 0) j_new = hist_get(hist, (int)(dir4(S.dir4, rv * kLutW + cu, centre) >> 2));
+    if (c == 0) j_new = hist_get(hist, (int)(dir4(lut4, rv * kLutW + cu, centre) >> 2));
     __syncwarp();
     hist_release(hist, ids);
     __syncwarp();
@@ -342,12 +352,19 @@ __device__ __noinline__ int partner_by_histograms(const PartnerSmem& S, uint32_t
   return cur - (bad_uv - (sum >> 16)) + (sum & 0xFFFF) + j_new;
 }
 
-// A run's partners by a warp each.
+// A state's column as the partner scores hold it: the histograms take columns beyond n as well.
+__device__ __forceinline__ uint8_t partner_column(int c) { return (uint8_t)min(max(c, 0), kMaxN - 1); }
+
+// The partners of the anchors [a0, a1) of one state (`cols`, m columns) by a warp each.  cs: the
+// warp's 152 bytes; turn: the warp that the next partner is for; await: the block's barrier comes
+// first (the same in every warp), for the tables to be in place and the space of cs to be free.
 template <bool SAME_LAYER, int NT>
-__device__ __forceinline__ void partners_by_pairs(const PartnerSmem& S, uint32_t* __restrict__ hist, int n,
+__device__ __forceinline__ void partners_by_pairs(const uint16_t* __restrict__ lut4, uint8_t* __restrict__ cs,
+                                                  uint32_t* __restrict__ hist, int n,
+                                                  const int16_t* __restrict__ cols,
                                                   const int32_t* __restrict__ anchors, int a0, int a1,
                                                   const int32_t* __restrict__ bad, int cur, int warp, int lane,
-                                                  int32_t* __restrict__ out) {
+                                                  int& turn, bool& await, int32_t* __restrict__ out) {
   const int m = 2 * n, width = SAME_LAYER ? n : m;
   WarpState W;
   W.m = m;
@@ -355,23 +372,37 @@ __device__ __forceinline__ void partners_by_pairs(const PartnerSmem& S, uint32_t
   W.cs = nullptr;
   W.bs = nullptr;
 #pragma unroll
-  for (int t = 0; t < kSlotsPerLane; ++t)
-    W.key2[t] = W.slot(t) < m ? 2 * ((W.slot(t) >> 1) * kLutW + S.cs[W.slot(t)]) : 0;
+  for (int t = 0; t < kSlotsPerLane; ++t) {
+    const int s = W.slot(t);
+    W.key2[t] = 0;
+    if (t < NT && s < m) W.key2[t] = 2 * ((s >> 1) * kLutW + partner_column(cols[s]));
+  }
+  if (await)
+    __syncthreads();
+  else
+    __syncwarp();  // done with the state before
+  await = false;
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+    if (W.slot(t) < m) cs[W.slot(t)] = (uint8_t)(W.key2[t] / 2 - (W.slot(t) >> 1) * kLutW);
+  __syncwarp();
   for (int a = a0; a < a1; ++a) {
     const int u = anchors[2 * a + 1];
     const bool in_range = u >= 0 && u < m;
-    for (int w = warp; w < width; w += kPartnerWarps) {
+    int w = warp - turn;
+    if (w < 0) w += kPartnerWarps;
+    for (; w < width; w += kPartnerWarps) {
       int score = N3_SENTINEL;
       if (in_range) {  // uniform
         const int v = SAME_LAYER ? 2 * w + (u & 1) : w;
-        const int ru = u >> 1, rv = v >> 1, cu = S.cs[u], cv = S.cs[v];
-        if (rv != ru && cv != S.cs[u ^ 1] && cu != S.cs[v ^ 1]) {  // uniform in the warp
+        const int ru = u >> 1, rv = v >> 1, cu = cs[u], cv = cs[v];
+        if (rv != ru && cv != cs[u ^ 1] && cu != cs[v ^ 1]) {  // uniform in the warp
           const int bad_uv = bad[u] + bad[v];
           bool redo = cu == cv;
           if (!redo) {
             Directions x, y;
             uint32_t line_new;
-            const PairCount p = count_pair<DenseNumbering, NT>(W, S.dir4, hist, ru, rv, cu, cv, x, y, line_new);
+            const PairCount p = count_pair<DenseNumbering, NT>(W, lut4, hist, ru, rv, cu, cv, x, y, line_new);
             __syncwarp();
             clear_centre<NT>(x);
             clear_centre<NT>(y);
@@ -379,11 +410,12 @@ __device__ __forceinline__ void partners_by_pairs(const PartnerSmem& S, uint32_t
             score = cur - (bad_uv - p.joint) + p.ta + p.tb + p.j_new;
             redo = p.wide;
           }
-          if (redo) score = partner_by_histograms(S, hist, m, u, v, cur, bad_uv, lane);
+          if (redo) score = partner_by_histograms(lut4, cs, hist, m, u, v, cur, bad_uv, lane);
         }
       }
       if (lane == 0) out[(size_t)a * width + w] = score;
     }
+    turn = (turn + width) % kPartnerWarps;
   }
 }
 
@@ -401,6 +433,11 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
   for (int a = tid; a <= kMaxN; a += blockDim.x) S.recip[a] = a ? (65536u + (uint32_t)a - 1u) / (uint32_t)a : 0u;
   uint32_t* hist = S.hist[warp];
   for (int i = lane; i < 2 * DenseNumbering::kWords; i += 32) hist[i] = 0u;
+  // the warp's own state, in the cover table's space
+  uint8_t* const mine = reinterpret_cast<uint8_t*>(S.T) + 152 * warp;
+  static_assert(152 * kPartnerWarps <= sizeof(S.T), "the warps' states");
+  int turn = 0;
+  bool await = true;
   const int a_end = min(A, (int)(blockIdx.x + 1) * per_cta);
   for (int a0 = blockIdx.x * per_cta; a0 < a_end;) {
     // the run of anchors of one state (the same in every warp)
@@ -413,7 +450,6 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
       a1 += more < 0 ? 32 : more;
       if (more >= 0) break;
     }
-    __syncthreads();  // the previous run is done with the state
     if (b < 0 || b >= B) {  // uniform
       for (int i = tid; i < (a1 - a0) * width; i += blockDim.x) out[(size_t)a0 * width + i] = N3_SENTINEL;
       a0 = a1;
@@ -421,28 +457,28 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
     }
     const int cur = current[b];
     const int32_t* bad = badness + (size_t)b * m;
+    const int16_t* state = cols + (size_t)b * m;
     bool cover = a1 - a0 >= kRunCover;
     if (cover) {
+      __syncthreads();  // the warps are done with the table, or with their own states
       for (int i = tid; i < kMaxN; i += blockDim.x) S.columns[i] = 0;
       for (int i = tid; i < (kMaxN * kMaxN + 31) / 32; i += blockDim.x) S.bits[i] = 0u;
       for (int i = tid; i < kPartnerRegion; i += blockDim.x) S.T[i] = 0u;
       __syncthreads();
-    }
-    bool regular = true;  // two points in every column, in cells of their own
-    for (int s = tid; s < m; s += blockDim.x) {
-      const int c = cols[(size_t)b * m + s];
-      const bool on_grid = c >= 0 && c < n;
-      regular = regular && on_grid;
-      S.cs[s] = (uint8_t)min(max(c, 0), kMaxN - 1);  // the histograms take columns beyond n as well
-      if (cover && on_grid) {
-        atomicAdd(&S.columns[c], 1);
-        const int cell = (s >> 1) * n + c;
-        const uint32_t bit = 1u << (cell & 31);
-        if (atomicOr(&S.bits[cell >> 5], bit) & bit) regular = false;
+      bool regular = true;  // two points in every column, in cells of their own
+      for (int s = tid; s < m; s += blockDim.x) {
+        const int c = state[s];
+        const bool on_grid = c >= 0 && c < n;
+        regular = regular && on_grid;
+        S.cs[s] = partner_column(c);
+        if (on_grid) {
+          atomicAdd(&S.columns[c], 1);
+          const int cell = (s >> 1) * n + c;
+          const uint32_t bit = 1u << (cell & 31);
+          if (atomicOr(&S.bits[cell >> 5], bit) & bit) regular = false;
+        }
       }
-    }
-    __syncthreads();
-    if (cover) {
+      __syncthreads();
       for (int c = tid; c < n; c += blockDim.x) regular = regular && S.columns[c] == 2;
       cover = __syncthreads_and(regular);
     }
@@ -488,13 +524,18 @@ __global__ void __launch_bounds__(kPartnerWarps * 32, 1) partner_scores_kernel(
         hist_release(hist, ids);
         __syncwarp();
       }
+      await = true;
     } else {
+      const auto pairs = [&](auto nt) {
+        partners_by_pairs<SAME_LAYER, decltype(nt)::value>(S.dir4, mine, hist, n, state, anchors, a0, a1, bad, cur, warp,
+                                                           lane, turn, await, out);
+      };
       switch ((m + 31) >> 5) {
-        case 5: partners_by_pairs<SAME_LAYER, 5>(S, hist, n, anchors, a0, a1, bad, cur, warp, lane, out); break;
-        case 4: partners_by_pairs<SAME_LAYER, 4>(S, hist, n, anchors, a0, a1, bad, cur, warp, lane, out); break;
-        case 3: partners_by_pairs<SAME_LAYER, 3>(S, hist, n, anchors, a0, a1, bad, cur, warp, lane, out); break;
-        case 2: partners_by_pairs<SAME_LAYER, 2>(S, hist, n, anchors, a0, a1, bad, cur, warp, lane, out); break;
-        default: partners_by_pairs<SAME_LAYER, 1>(S, hist, n, anchors, a0, a1, bad, cur, warp, lane, out); break;
+        case 5: pairs(std::integral_constant<int, 5>{}); break;
+        case 4: pairs(std::integral_constant<int, 4>{}); break;
+        case 3: pairs(std::integral_constant<int, 3>{}); break;
+        case 2: pairs(std::integral_constant<int, 2>{}); break;
+        default: pairs(std::integral_constant<int, 1>{}); break;
       }
     }
     a0 = a1;
