@@ -169,7 +169,6 @@ struct ScanArgs {
   int n, anchor;
   int64_t base;          // E of the state
   int combos;            // C(n - 1, 3)
-  bool small;            // scan_any_kernel takes every state
   const uint16_t* lut;    // scan_any_kernel's table
   const uint16_t* prim4;  // scan_kernel's
   const uint16_t* dir4;
@@ -214,6 +213,93 @@ __device__ __forceinline__ bool regular_state(const ScanArgs& A, int* __restrict
   return __syncthreads_and(regular);
 }
 
+// The nine candidates of slot set gw by a warp, from 4 + 12 histograms.
+__device__ __forceinline__ void scan_slot_set(const ScanArgs& A, const int* __restrict__ cs, int gw, int lane,
+                                              const uint16_t* __restrict__ lutf, uint32_t* __restrict__ hist,
+                                              int (*jt)[12], int* tn) {
+  const int n = A.n, m = 2 * n;
+  const int combo = gw >> 3, layers = gw & 7;
+  const int arow = A.anchor >> 1;
+  int r[3];
+  unrank3(combo, n - 1, r[0], r[1], r[2]);
+  int T[4];
+  T[0] = A.anchor;
+  for (int i = 0; i < 3; ++i) {
+    const int row = r[i] < arow ? r[i] : r[i] + 1;  // i-th row other than the anchor's
+    T[i + 1] = 2 * row + ((layers >> (2 - i)) & 1);
+  }
+  int rowT[4], colT[4], partner[4];
+  for (int i = 0; i < 4; ++i) {
+    rowT[i] = T[i] >> 1;
+    colT[i] = cs[T[i]];
+    partner[i] = cs[T[i] ^ 1];
+  }
+  const uint32_t skip = skip_mask(lane, T, 4);
+  int key[kT];
+  lane_keys(cs, m, lane, key);
+  const int before = side_sum(key, m, rowT, colT, 4, skip, lutf, hist, lane);
+  // the 12 candidate positions: target i with the column of source j != i (index 3 i + (j > i ? j - 1 : j))
+  for (int a = 0; a < 12; ++a) {
+    const int i = a / 3, jj = a % 3, j = jj >= i ? jj + 1 : jj;
+    const int rx = rowT[i], cx = colT[j];
+    int ids[kT];
+    const int part = hist_build_excl(key, m, rx, cx, skip, lutf, hist, lane, ids);
+    __syncwarp();
+    if (lane < 12) {
+      const int b = lane, ib = b / 3, jb = b % 3 >= ib ? b % 3 + 1 : b % 3;
+      jt[a][b] = ib != i ? hist_get(hist, dir_id_full(lutf, rowT[ib] - rx, colT[jb] - cx)) : 0;
+    }
+    __syncwarp();
+    hist_release(hist, ids);
+    const int t = warp_sum(part);
+    if (lane == 0) tn[a] = t;
+    __syncwarp();
+  }
+  // the moves: sigma[i] = source of target i
+  if (lane < 9) {
+    int sigma[4];
+    unsigned int idx;
+    if (lane < 6) {  // four-cycle with ordering number `lane` of (T1, T2, T3)
+      const int perm[6][3] = {{1, 2, 3}, {1, 3, 2}, {2, 1, 3}, {2, 3, 1}, {3, 1, 2}, {3, 2, 1}};
+      const int o0 = perm[lane][0], o1 = perm[lane][1], o2 = perm[lane][2];
+      sigma[0] = o0;
+      sigma[o0] = o1;
+      sigma[o1] = o2;
+      sigma[o2] = 0;
+      idx = (unsigned)((combo * 8 + layers) * 6 + lane);
+    } else {  // double switch pairing lane - 6: (a, anchor, c, b), (b, c, anchor, a), (c, b, a, anchor)
+      const int pairs[3][4] = {{1, 0, 3, 2}, {2, 3, 0, 1}, {3, 2, 1, 0}};
+      for (int i = 0; i < 4; ++i) sigma[i] = pairs[lane - 6][i];
+      idx = (unsigned)((combo * 8 + layers) * 3 + (lane - 6));
+    }
+    bool legal = true;
+    int after = 0, pos[4], nr[4], nc[4];
+    for (int i = 0; i < 4; ++i) {
+      const int j = sigma[i];
+      legal = legal && colT[j] != partner[i];
+      pos[i] = 3 * i + (j > i ? j - 1 : j);
+      nr[i] = rowT[i];
+      nc[i] = colT[j];
+      after += tn[pos[i]];
+    }
+    for (int i = 0; i < 4; ++i)
+      for (int k = i + 1; k < 4; ++k) after += jt[pos[i]][pos[k]];
+    for (int i = 0; i < 4; ++i)
+      for (int j = i + 1; j < 4; ++j)
+        for (int k = j + 1; k < 4; ++k) after += collinear(nr[i], nc[i], nr[j], nc[j], nr[k], nc[k]);
+    if (legal) {
+      const int64_t score = A.base + after - before;
+      const unsigned long long key = ((unsigned long long)score << 32) | idx;
+      const int which = lane < 6 ? 0 : 1;
+      atomicMin(A.best + which, key);
+      atomicAdd(A.legal + which, 1ull);
+    }
+  }
+}
+
+// SMALL: every state, a warp per slot set (n = 5: 14.4 us, 17.1 with the loop and the test of
+// the state); else irregular ones only, in loops.
+template <bool SMALL>
 __global__ void __launch_bounds__(kWarps * 32) scan_any_kernel(const ScanArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* lutf = reinterpret_cast<uint16_t*>(smem);
@@ -223,94 +309,21 @@ __global__ void __launch_bounds__(kWarps * 32) scan_any_kernel(const ScanArgs A)
   __shared__ int tn_all[kWarps][12];      // t_A of each candidate position
   __shared__ int columns[kMaxN];
   const int n = A.n, m = 2 * n;
-  if (!A.small && regular_state(A, columns)) return;
+  if (!SMALL && regular_state(A, columns)) return;
   full_lut_copy(lutf, A.lut);
   for (int i = threadIdx.x; i < kWarps * kDirWords; i += blockDim.x) hist_all[i] = 0u;
   for (int s = threadIdx.x; s < m; s += blockDim.x) cs[s] = (s & 1) ? A.q[s >> 1] : A.p[s >> 1];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t* hist = hist_all + warp * kDirWords;
-  int (*jt)[12] = jt_all[warp];
-  int* tn = tn_all[warp];
-  for (int gw = blockIdx.x * kWarps + warp; gw < A.combos * 8; gw += gridDim.x * kWarps) {
-    const int combo = gw >> 3, layers = gw & 7;
-    const int arow = A.anchor >> 1;
-    int r[3];
-    unrank3(combo, n - 1, r[0], r[1], r[2]);
-    int T[4];
-    T[0] = A.anchor;
-    for (int i = 0; i < 3; ++i) {
-      const int row = r[i] < arow ? r[i] : r[i] + 1;  // i-th row other than the anchor's
-      T[i + 1] = 2 * row + ((layers >> (2 - i)) & 1);
-    }
-    int rowT[4], colT[4], partner[4];
-    for (int i = 0; i < 4; ++i) {
-      rowT[i] = T[i] >> 1;
-      colT[i] = cs[T[i]];
-      partner[i] = cs[T[i] ^ 1];
-    }
-    const uint32_t skip = skip_mask(lane, T, 4);
-    int key[kT];
-    lane_keys(cs, m, lane, key);
-    const int before = side_sum(key, m, rowT, colT, 4, skip, lutf, hist, lane);
-    // the 12 candidate positions: target i with the column of source j != i (index 3 i + (j > i ? j - 1 : j))
-    for (int a = 0; a < 12; ++a) {
-      const int i = a / 3, jj = a % 3, j = jj >= i ? jj + 1 : jj;
-      const int rx = rowT[i], cx = colT[j];
-      int ids[kT];
-      const int part = hist_build_excl(key, m, rx, cx, skip, lutf, hist, lane, ids);
-      __syncwarp();
-      if (lane < 12) {
-        const int b = lane, ib = b / 3, jb = b % 3 >= ib ? b % 3 + 1 : b % 3;
-        jt[a][b] = ib != i ? hist_get(hist, dir_id_full(lutf, rowT[ib] - rx, colT[jb] - cx)) : 0;
-      }
-      __syncwarp();
-      hist_release(hist, ids);
-      const int t = warp_sum(part);
-      if (lane == 0) tn[a] = t;
+  const int first = blockIdx.x * kWarps + warp;
+  if (SMALL) {
+    if (first < A.combos * 8) scan_slot_set(A, cs, first, lane, lutf, hist, jt_all[warp], tn_all[warp]);
+  } else {
+    for (int gw = first; gw < A.combos * 8; gw += gridDim.x * kWarps) {
+      scan_slot_set(A, cs, gw, lane, lutf, hist, jt_all[warp], tn_all[warp]);
       __syncwarp();
     }
-    // the moves: sigma[i] = source of target i
-    if (lane < 9) {
-      int sigma[4];
-      unsigned int idx;
-      if (lane < 6) {  // four-cycle with ordering number `lane` of (T1, T2, T3)
-        const int perm[6][3] = {{1, 2, 3}, {1, 3, 2}, {2, 1, 3}, {2, 3, 1}, {3, 1, 2}, {3, 2, 1}};
-        const int o0 = perm[lane][0], o1 = perm[lane][1], o2 = perm[lane][2];
-        sigma[0] = o0;
-        sigma[o0] = o1;
-        sigma[o1] = o2;
-        sigma[o2] = 0;
-        idx = (unsigned)((combo * 8 + layers) * 6 + lane);
-      } else {  // double switch pairing lane - 6: (a, anchor, c, b), (b, c, anchor, a), (c, b, a, anchor)
-        const int pairs[3][4] = {{1, 0, 3, 2}, {2, 3, 0, 1}, {3, 2, 1, 0}};
-        for (int i = 0; i < 4; ++i) sigma[i] = pairs[lane - 6][i];
-        idx = (unsigned)((combo * 8 + layers) * 3 + (lane - 6));
-      }
-      bool legal = true;
-      int after = 0, pos[4], nr[4], nc[4];
-      for (int i = 0; i < 4; ++i) {
-        const int j = sigma[i];
-        legal = legal && colT[j] != partner[i];
-        pos[i] = 3 * i + (j > i ? j - 1 : j);
-        nr[i] = rowT[i];
-        nc[i] = colT[j];
-        after += tn[pos[i]];
-      }
-      for (int i = 0; i < 4; ++i)
-        for (int k = i + 1; k < 4; ++k) after += jt[pos[i]][pos[k]];
-      for (int i = 0; i < 4; ++i)
-        for (int j = i + 1; j < 4; ++j)
-          for (int k = j + 1; k < 4; ++k) after += collinear(nr[i], nc[i], nr[j], nc[j], nr[k], nc[k]);
-      if (legal) {
-        const int64_t score = A.base + after - before;
-        const unsigned long long key = ((unsigned long long)score << 32) | idx;
-        const int which = lane < 6 ? 0 : 1;
-        atomicMin(A.best + which, key);
-        atomicAdd(A.legal + which, 1ull);
-      }
-    }
-    __syncwarp();
   }
 }
 
@@ -633,7 +646,9 @@ int n3_neighborhood_scan(const int32_t* p, const int32_t* q, int n, int anchor, 
   if (anchor < 0 || anchor >= 2 * n) return n3host::set_error(N3_ERR_RANGE, "anchor index outside point slots");
   if (!p || !q || !best || !legal) return n3host::set_error(N3_ERR_ARG, "neighbourhood scan: null buffer");
   N3_TRY(n3host::ensure_device_tables());
-  N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::multi::scan_any_kernel), n3::multi::kSmem));
+  const bool small = n < n3::multi::kScanSmallN;
+  const auto scan_any = small ? n3::multi::scan_any_kernel<true> : n3::multi::scan_any_kernel<false>;
+  N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(scan_any), n3::multi::kSmem));
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemsetAsync(best, 0xFF, 2 * sizeof(unsigned long long), st) != cudaSuccess ||
       cudaMemsetAsync(legal, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess)
@@ -648,9 +663,8 @@ int n3_neighborhood_scan(const int32_t* p, const int32_t* q, int n, int anchor, 
   A.lut = n3host::dir_lut_full_device_ptr();
   A.best = best;
   A.legal = legal;
-  A.small = n < n3::multi::kScanSmallN;
   int grid = (A.combos * 8 + n3::multi::kWarps - 1) / n3::multi::kWarps;
-  if (!A.small) {
+  if (!small) {
     A.prim4 = n3host::prim4_lut_device_ptr();
     A.dir4 = n3host::dir4_lut_device_ptr();
     N3_TRY(n3host::allow_smem(reinterpret_cast<const void*>(n3::multi::scan_kernel), sizeof(n3::multi::ScanSmem)));
@@ -660,7 +674,7 @@ int n3_neighborhood_scan(const int32_t* p, const int32_t* q, int n, int anchor, 
     N3_TRY(n3host::check_launch("scan_kernel"));
     if (grid > 2 * sms) grid = 2 * sms;
   }
-  n3::multi::scan_any_kernel<<<grid, n3::multi::kWarps * 32, n3::multi::kSmem, st>>>(A);
+  scan_any<<<grid, n3::multi::kWarps * 32, n3::multi::kSmem, st>>>(A);
   return n3host::check_launch("scan_any_kernel");
 }
 
