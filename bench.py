@@ -43,9 +43,6 @@ TESTS_PER_STATE = math.comb(2 * N, 3)  # 551,300
 # the determinant kernel tests every triple except those holding two points of
 # one row (never collinear with a third point in another row): 75 rows x 148
 KERNEL_TESTS_PER_STATE = TESTS_PER_STATE - N * (2 * N - 2)  # 540,200
-# per test: one product on the FMA pipe (2 multiplies + 2 multiply-adds serve
-# 4 tests) and one compare on the ALU pipe
-OPS_PER_TEST = 2
 L2_FLUSH_BYTES = 256 << 20             # > 126 MB L2
 WORKLOAD = "n=75 population scoring, 4096 states, determinant + slope cross-check + badness"
 # dram__bytes_read.sum + dram__bytes_write.sum of one checked_kernel launch over the
@@ -848,8 +845,8 @@ def run_b200(args):
     det_ms = [a.elapsed_time(b) for a, b in det_ms[2:]]
     det_launch_s = statistics.mean(det_ms) / 1e3
 
-    # integer-pipe ceilings: each pipe alone (multiply-add chains, logic-op
-    # chains), and the scorer's own expression on registers
+    # the determinants' own expression on registers, their ceiling, and for
+    # context the integer pipes alone (multiply-add chains, logic-op chains)
     scratch = torch.zeros(2, dtype=torch.int64, device=dev)
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
 
@@ -879,9 +876,7 @@ def run_b200(args):
         tests_per_s = value * TESTS_PER_STATE
         # the determinants alone: 4096 states x 540,200 tested triples per launch
         kernel_tests = B * KERNEL_TESTS_PER_STATE / det_launch_s
-        pipe_tests = min(pipe_rate["imad"], pipe_rate["alu"])  # one op of each pipe per test
-        achieved = kernel_tests * OPS_PER_TEST / 1e9
-        peak = pipe_tests * OPS_PER_TEST / 1e9
+        achieved, peak = kernel_tests / 1e9, ceiling_tests / 1e9
         peaks, peak_kind = measured_peaks()
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -896,22 +891,21 @@ def run_b200(args):
                     "d2h_bytes_per_step": int(h_scores.numel() * 4 + h_flags.numel() * 4),
                     "copies": "pinned host buffers; H2D of step k+1 and read-back of step k on a second stream beside the compute"},
             "gpu_launches": args.steps * (2 if args.mode == "checked" and B < 8 * sms else 1),
-            "roofline": {"bound": "int32 pipes (FMA pipe for products, ALU pipe for compares)",
-                         "kernel": "n3::checked_kernel<true> (the step's one launch: determinants on the multiply-add "
-                                   "pipe beside the slope count on shared memory), timed alone; the operations "
-                                   "counted are the determinants'",
+            "roofline": {"bound": "determinant tests on packed floats (multiply-add pipe and register reads)",
+                         "kernel": "n3::checked_kernel<true> (the step's one launch: determinants on 20 of a CTA's 32 "
+                                   "warps beside the slope count, which shared memory bounds, on the others), timed "
+                                   "alone; what is counted are the determinants' tests",
                          "kernel_launch_us": det_launch_s * 1e6,
                          "kernel_tests_per_s": kernel_tests,
-                         "achieved": achieved, "peak": peak, "unit": "Gop/s", "frac": achieved / peak,
-                         "peak_source": "measured on this GPU: n3_calibrate_int_pipe, multiply-add chains "
-                                        f"{pipe_rate['imad'] / 1e12:.2f} Top/s and logic-op chains "
-                                        f"{pipe_rate['alu'] / 1e12:.2f} Top/s; 2 ops per tested triple (one "
-                                        "product share on the FMA pipe, one compare on the ALU pipe), "
+                         "achieved": achieved, "peak": peak, "unit": "Gtest/s", "frac": achieved / peak,
+                         "peak_source": "measured on this GPU: n3_calibrate_det_ceiling, the determinants' test "
+                                        "expression (per four tests two packed multiply-adds, a packed multiply and "
+                                        "add, two compares, two counts) on registers, every warp of the GPU on it; "
                                         f"{KERNEL_TESTS_PER_STATE} tested triples per state",
-                         "expression_ceiling": {"tests_per_s": ceiling_tests,
-                                                "frac": kernel_tests / ceiling_tests,
-                                                "source": "n3_calibrate_det_ceiling: the scorer's test "
-                                                          "expression with per-test counting, on registers"},
+                         "integer_pipes_context": {"multiply_add_per_s": pipe_rate["imad"],
+                                                   "logic_op_per_s": pipe_rate["alu"],
+                                                   "source": "n3_calibrate_int_pipe; the determinants of these states "
+                                                             "do not run on integers"},
                          "traffic": CHECKED_TRAFFIC_BYTES,
                          "hbm_context": {"bytes_per_step": int(cols_host.nbytes + B * 4 + B * 2 * N * 4),
                                          "hbm_gbs_peak": peaks.get("hbm_gbs"), "peak_kind": peak_kind}},

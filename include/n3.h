@@ -526,17 +526,17 @@ int n3_graph_destroy(void* graph_exec);
  * Measurement helper (no reference counterpart).
  * ------------------------------------------------------------------------- */
 
-/* Runs the scorer's determinant test expression on register operands only
- * (no memory traffic): blocks x 256 threads x iters x 16 triple tests.  Its
- * event-timed rate is the integer-pipe ceiling that bench.py reports the
- * scorer's rate against.  scratch2: device uint64[2]. */
+/* Runs the scorer's determinant test expression (packed floats) on register
+ * operands only (no memory traffic): blocks x 256 threads x iters x 16 triple
+ * tests.  Its event-timed rate is the ceiling that bench.py reports the
+ * determinants' rate against.  scratch2: device uint64[2]. */
 int n3_calibrate_det_ceiling(int blocks, int iters, unsigned long long* scratch2, void* stream);
 
 /* Throughput of one integer pipe on its own: blocks x 256 threads x iters x 8
- * dependent-chain operations, kind 0 an integer multiply-add (the FMA pipe,
- * which the scorer's products use), kind 1 a three-input logic operation (the
- * ALU pipe, which its compares use).  Event-timed, these are the pipe ceilings
- * bench.py states the scorer's roofline against.  scratch2: device uint64[2]. */
+ * dependent-chain operations, kind 0 an integer multiply-add (the FMA pipe),
+ * kind 1 a three-input logic operation (the ALU pipe): the pipes of the
+ * determinants on integers.  bench.py reports them beside its roofline.
+ * scratch2: device uint64[2]. */
 int n3_calibrate_int_pipe(int kind, int blocks, int iters, unsigned long long* scratch2, void* stream);
 
 /* Random 4-byte gathers from `table` (int32 [entries], sized to stay in L2):

@@ -1,51 +1,57 @@
 // Instruction-throughput ceiling of the determinant test.
 //
-// The population scorer's inner step (score.cu, det_pivot_row) performs, per
-// four triple tests, two integer multiplies, two multiply-adds and four
-// compares.  det_ceiling_kernel runs the same expression on register-resident
-// operands with no shared-memory traffic, counting every hit, on every SM: a
-// ceiling of that expression.  int_pipe_kernel measures the two integer pipes
-// the expression uses on their own (no integer peak is published for B200).
-#include "n3_common.cuh"
+// The population scorer's inner step (score_impl.cuh, det_pivot_row_f) performs, per
+// four triple tests, two packed multiply-adds, a packed multiply and a packed add,
+// two compares and two counts.  det_ceiling_kernel runs the same expression on
+// register-resident operands with no shared-memory traffic, counting every hit, on
+// every SM: a ceiling of that expression.  int_pipe_kernel measures the two integer
+// pipes on their own, which the determinants on integers use (off-grid and small
+// states; no integer peak is published for B200).
+#include "score_impl.cuh"
 
 namespace n3 {
 
 template <int R>
 __global__ void __launch_bounds__(256) det_ceiling_kernel(int iters, int seed, unsigned long long* out) {
-  int ax[R], bx0[R], bx1[R], k0[R], k1[R];
+  uint64_t ax[R], nb[R], nt[R];
   const int t = threadIdx.x + seed;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    ax[r] = (t + 3 * r) % 37 - 18;
-    bx0[r] = (t * 7 + r) % 41 - 20;
-    bx1[r] = (t * 5 + 2 * r) % 43 - 21;
-    k0[r] = ax[r] * (t % 29);
-    k1[r] = ax[r] * (t % 31);
+    const float a = (float)((t + 3 * r) % 37 - 18);
+    const float b0 = (float)((t * 7 + r) % 41 - 20), b1 = (float)((t * 5 + 2 * r) % 43 - 21);
+    ax[r] = pack2(a, a);
+    nb[r] = pack2(-b0, -b1);
+    nt[r] = pack2(30.f * b0 - a * (float)(t % 29), 30.f * b1 - a * (float)(t % 31));
   }
-  int cnt = 0;
-  int cx = t & 63, cyv = (t >> 3) & 63, ay = -30;
-#pragma unroll 2
-  for (int it = 0; it < iters; ++it) {
+  int cnt = 0, cnt1 = 0;
+  // two rows' columns, taken in turn
+  const float c = (float)(t & 63), d = (float)((t >> 3) & 63);
+  const uint64_t cy[2][2] = {{pack2(c, c), pack2(d, d)}, {pack2(c + 13.f, c + 13.f), pack2(d + 29.f, d + 29.f)}};
+#pragma unroll 1
+  for (int it = 0; it < iters; it += 2) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int P0 = ax[r] * cx, P1 = ax[r] * cyv;
-      const int T0 = ay * bx0[r] + k0[r], T1 = ay * bx1[r] + k1[r];
-      cnt += ((P0 == T0) + (P1 == T0)) + ((P0 == T1) + (P1 == T1));
+    for (int row = 0; row < 2; ++row) {
+      if (it + row >= iters) break;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint64_t p = mul2(fma2(ax[r], cy[row][0], nt[r]), fma2(ax[r], cy[row][1], nt[r]));
+        float p0, p1;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
+        count_zero(cnt, p0);
+        count_zero(cnt1, p1);
+        nt[r] = add2(nt[r], nb[r]);
+      }
     }
-    // next "row": the scorer loads two columns and bumps the row offset
-    cx = (cx + 13) & 63;
-    cyv = (cyv + 29) & 63;
-    ay += 1;
   }
-  if (cnt == 0x7fffffff) out[0] = cnt;  // keeps the loop live
+  if (cnt + cnt1 == 0x7fffffff) out[0] = cnt;  // keeps the loop live
   if (threadIdx.x == 0 && blockIdx.x == 0) out[1] = (unsigned long long)iters;
 }
 
 // Pipe ceilings independent of the scorer's expression.  Each thread runs 8
 // independent loop-carried chains of one instruction kind on runtime values
 // (so nothing folds): an integer multiply-add a = a * b + c (the FMA pipe's
-// integer work, as the scorer's products) or a three-input logic op
-// a = (a & b) | (a ^ c) (the ALU pipe, as the scorer's compares).  Ops per
+// integer work, as the products on integers) or a three-input logic op
+// a = (a & b) | (a ^ c) (the ALU pipe, as the compares).  Ops per
 // launch = blocks * 256 * iters * 8.
 template <int KIND>
 __global__ void __launch_bounds__(256) int_pipe_kernel(int iters, int seed, unsigned long long* out) {
