@@ -904,9 +904,9 @@ __device__ __forceinline__ void tc_tile(const GemmArgs& G, int n0, int m0, int s
     for (int j = 0; j < 32; ++j) blk[lane * 33 + j] = v[j];
     __syncwarp();
     const int nn = n0 + c0 + lane, row0 = m0 + 32 * quarter, rows = min(32, G.M - row0);
+    float sum = 0.f;
     if (nn < G.N && rows > 0) {
       const float bias = EPI == 1 || EPI == 3 ? G.bias[nn] : 0.f;
-      float sum = 0.f;
 #pragma unroll 8
       for (int rr = 0; rr < rows; ++rr) {
         const float x = blk[rr * 33 + lane];
@@ -928,7 +928,14 @@ __device__ __forceinline__ void tc_tile(const GemmArgs& G, int n0, int m0, int s
           sum += dz;
         }
       }
-      if (EPI == 2) atomicAdd(G.sums + nn, sum);
+    }
+    if (EPI == 2) {  // the tile's column sums in a fixed order (head_kernel says why)
+      blk[lane] = sum;
+      __syncthreads();
+      if (quarter == 0 && nn < G.N) {
+        for (int q = 1; q < 4; ++q) sum += blk[q * (32 * 33) + lane];
+        atomicAdd(G.sums + nn, sum);
+      }
     }
   } else if (tid == 0 && error_word) {
     atomicOr(error_word, kErrTimeout);
@@ -963,13 +970,21 @@ __global__ void __launch_bounds__(kTcThreads) tc_back_kernel(const GemmArgs Z, c
 // sums stay in registers to the end, so each block adds once per column.  (One
 // addition to the loss per row cost 12 us for 4096 rows, a pass per column
 // sum 12 to 20 us.)
-constexpr int kHeadWarps = 8;
+//
+// A batch of up to kRepeatableBatch rows gives the same bits every time: no gradient
+// is then added up from more than two parts (here two blocks, in tc_tile two row
+// tiles and no K split), and two additions to zero give the same in either order.
+// For that such a batch takes two blocks of 32 warps (a step of 256 rows: 54.7 us, 51.0 with
+// 32 blocks of 8, 128 with a launch per sum).
+constexpr int kRepeatableBatch = 256;
+template <int kHeadWarps>
 __global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const float* Z2, const float* P, const float* y,
                                                                float* __restrict__ d, float* __restrict__ dZ2,
                                                                float* __restrict__ grads, float* __restrict__ loss) {
   chain_begin();
   constexpr int kC = kH / 32;
-  __shared__ float s_w3[kHeadWarps][kH], s_b2[kHeadWarps][kH], s_loss[kHeadWarps], s_b3[kHeadWarps];
+  extern __shared__ float s_parts[];  // [2][kHeadWarps][kH]: the warps' shares of w3's and b2's gradients
+  __shared__ float s_loss[kHeadWarps], s_b3[kHeadWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float w3[kC], g_w3[kC], g_b2[kC], loss_sum = 0.f, b3_sum = 0.f;
 #pragma unroll
@@ -978,6 +993,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const floa
     g_w3[j] = g_b2[j] = 0.f;
   }
   const float b3 = P[oB3];
+#pragma unroll 2
   for (int b = blockIdx.x * kHeadWarps + warp; b < B; b += gridDim.x * kHeadWarps) {
     float z[kC], acc = 0.f;
 #pragma unroll
@@ -1002,23 +1018,20 @@ __global__ void __launch_bounds__(kHeadWarps * 32) head_kernel(int B, const floa
   }
 #pragma unroll
   for (int j = 0; j < kC; ++j) {
-    s_w3[warp][lane + 32 * j] = g_w3[j];
-    s_b2[warp][lane + 32 * j] = g_b2[j];
+    s_parts[warp * kH + lane + 32 * j] = g_w3[j];
+    s_parts[(kHeadWarps + warp) * kH + lane + 32 * j] = g_b2[j];
   }
   if (lane == 0) {
     s_loss[warp] = loss_sum;
     s_b3[warp] = b3_sum;
   }
   __syncthreads();
-  for (int n = threadIdx.x; n < kH; n += blockDim.x) {
-    float a = 0.f, c = 0.f;
+  for (int i = threadIdx.x; i < 2 * kH; i += blockDim.x) {
+    const int which = i / kH, n = i % kH;
+    float a = 0.f;
 #pragma unroll
-    for (int w = 0; w < kHeadWarps; ++w) {
-      a += s_w3[w][n];
-      c += s_b2[w][n];
-    }
-    atomicAdd(grads + oW3 + n, a);
-    atomicAdd(grads + oB2 + n, c);
+    for (int w = 0; w < kHeadWarps; ++w) a += s_parts[(which * kHeadWarps + w) * kH + n];
+    atomicAdd(grads + (which ? oB2 : oW3) + n, a);
   }
   if (threadIdx.x == 0) {
     float a = 0.f, c = 0.f;
@@ -1135,9 +1148,16 @@ static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t s
   N3_TRY(launch_chained("mlp layer 1", tc_gemm_kernel<1>, dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st, l1, ew));
   const GemmArgs l2 = {B, kH, kH, H1, kH, 1, P + oW2, 1, kH, H2, kH, P + oB2, Z2, nullptr};
   N3_TRY(launch_chained("mlp layer 2", tc_gemm_kernel<1>, dim3(kH / kTcN, row_tiles, 1), kTcThreads, kTcSmem, st, l2, ew));
-  const int head_blocks = (B + kHeadWarps - 1) / kHeadWarps;
-  N3_TRY(launch_chained("mlp head_kernel", head_kernel, head_blocks < sm_count() ? head_blocks : sm_count(),
-                        kHeadWarps * 32, 0, st, B, Z2, P, y, d, dZ2, grads, loss));
+  const auto head_smem = [](int warps) { return sizeof(float) * 2 * kH * (size_t)warps; };
+  if (B <= kRepeatableBatch) {
+    N3_TRY(allow_smem(reinterpret_cast<const void*>(head_kernel<32>), head_smem(32)));
+    N3_TRY(launch_chained("mlp head_kernel", head_kernel<32>, B <= kRepeatableBatch / 2 ? 1 : 2, 32 * 32, head_smem(32),
+                          st, B, Z2, P, y, d, dZ2, grads, loss));
+  } else {
+    const int head_blocks = (B + 7) / 8;
+    N3_TRY(launch_chained("mlp head_kernel", head_kernel<8>, head_blocks < sm_count() ? head_blocks : sm_count(), 8 * 32,
+                          head_smem(8), st, B, Z2, P, y, d, dZ2, grads, loss));
+  }
   // dZ1 = (dZ2 W2) * (Z1 > 0)            (B(k, n) = W2[k*256 + n]), and b1's gradient
   const GemmArgs z1 = {B, kH, kH, dZ2, kH, 1, P + oW2, kH, 1, dZ1, kH, nullptr, Z1, grads + oB1};
   // gW2[n][k] = sum_b dZ2[b][n] H1[b][k]
