@@ -9,8 +9,11 @@ src/no_three_75/hardware.py:48-80).  Here the choices are measured:
   together: every pair the ladder admits (at most 16 warps per CTA; cpb a
   divisor of L with at most 8 CTAs per cluster, or a multiple of L) is timed on
   a copy of the chains and the fastest kept.  One warp works on a chain at
-  every width, so the width only bounds cpb; fewer chains per CTA leave each
-  warp more of its SM when there are too few chains to fill the GPU.
+  every width, so the width only bounds cpb, and widths with the same cpb are
+  the same launch: among pairs within 1 % of the fastest (those differ by noise,
+  0.02 % measured) the narrowest width is kept, which bounds cpb least.  Fewer
+  chains per CTA leave each warp more of its SM when there are too few chains to
+  fill the GPU.
 * per-size sweeps per launch: in one mixed-size launch every CTA runs its own
   ladders' rounds, and the launch ends with its slowest CTA.  The tuner times
   each size alone, then gives each size a number of sweeps proportional to its
@@ -52,7 +55,7 @@ class TuneResult:
 
 
 def _valid_cpb(L: int, ladders: int, threads_per_chain: int = 32) -> list[int]:
-    """Chains per CTA that the launch admits for this ladder and team width."""
+    """Chains per CTA that the launch admits for this ladder and width (which only bounds them)."""
     cap = 16 // (threads_per_chain // 32)
     out = []
     for cpb in range(1, cap + 1):
@@ -113,8 +116,7 @@ def autotune(ch: TemperingChains, *, exchange_every: int = 10, probe_sweeps: int
     if len(sizes) > 1:
         ladder_sweeps = [size_sweeps[int(n)] for n in ch.ladder_n_host]
     # 3. threads per chain and chains per CTA
-    candidates = {}
-    best = None
+    candidates, timed = {}, []
     for tpc, cpb in _shapes(L, len(ch.ladder_n_host)):
         if ladder_sweeps is not None and cpb > L:
             ls = np.asarray(ladder_sweeps).reshape(-1, cpb // L)
@@ -126,9 +128,11 @@ def autotune(ch: TemperingChains, *, exchange_every: int = 10, probe_sweeps: int
             base * 2 * sizes[0] * ch.cols.shape[0]
         key = f"{tpc}x{cpb}"
         candidates[key] = props / secs
-        if best is None or candidates[key] > candidates[best[0]]:
-            best = (key, tpc, cpb, secs)
-    key, tpc, cpb, secs = best
+        timed.append((key, tpc, cpb, secs))
+    fastest = max(candidates.values())
+    # the pairs go by width, so this is the narrowest of those as fast (fastest first within it)
+    near = [shape for shape in timed if candidates[shape[0]] >= 0.99 * fastest]
+    key, tpc, cpb, secs = min(near, key=lambda shape: (shape[1], -candidates[shape[0]]))
     # 4. per-size deltas/s of the chosen layout and the sweeps per launch
     per_size = {n: size_sweeps[n] * 2 * n * L * len(ladders_of[n]) / secs for n in sizes} if ladder_sweeps else \
         {sizes[0]: candidates[key]}

@@ -313,11 +313,11 @@ class TemperingChains:
             self._removed_exact = False
 
     def default_chains_per_block(self, threads_per_chain: int = 32) -> int:
-        """Chains per CTA for teams of ``threads_per_chain`` threads (at most 16
-        warps per CTA, so cap = 16 / warps per chain): whole ladders per CTA
-        when L <= cap (as many as fit and divide the ladder count), else the
-        largest divisor of L up to cap whose cluster (L / cpb CTAs) has at most
-        8 CTAs."""
+        """Chains per CTA under the bound that ``threads_per_chain`` sets (cap =
+        16 / (threads_per_chain / 32); one warp works on a chain at every width):
+        whole ladders per CTA when L <= cap (as many as fit and divide the ladder
+        count), else the largest divisor of L up to cap whose cluster (L / cpb
+        CTAs) has at most 8 CTAs."""
         if threads_per_chain not in (32, 64, 128, 256):
             raise ValueError("threads_per_chain must be 32, 64, 128 or 256")
         cap = 16 // (threads_per_chain // 32)
@@ -332,8 +332,8 @@ class TemperingChains:
                          f"({threads_per_chain} threads per chain)")
 
     def _shape_cpb(self, threads_per_chain: int) -> int:
-        """The set's chains_per_block when it was chosen for this team width,
-        else the default."""
+        """The set's chains_per_block when it was chosen for this width, else the
+        default."""
         if self.chains_per_block and threads_per_chain == self.threads_per_chain:
             return int(self.chains_per_block)
         return self.default_chains_per_block(threads_per_chain)
