@@ -139,7 +139,14 @@ __device__ void exchange_ladder(int* tmp_chain, int* tmp_temp, const int* e, int
 // cover table 15 per proposal, 36,000 per accepted move and 300,000 to build.  100
 // sweeps of 2048 chains, ladders of 64 from 0.05 to 5.0: 16.8 ms with the line at
 // 0.008, 16.5 ms at 0.039, 24.8 ms at 0.078 (38.3 ms with one 8-bit histogram at a
-// time, a team barrier after each, and no cover table).
+// time, a team barrier after each, and no cover table).  40 sweeps on other grids, ms with
+// no table, the line at 0.02, 0.039 and 0.078, and one 8-bit histogram at a time:
+//   2048 chains 0.05 .. 5.0   n = 8  0.49 0.52 0.57 0.70 0.94   n = 20 1.75 1.49 1.58 2.18 2.93
+//                             n = 40 3.68 3.10 3.06 4.58 6.72   n = 75 8.6  6.4  6.4  11.1 15.3
+//   512 chains 0.3 .. 1.2     n = 8  0.39 0.48 0.60 0.68 0.68   n = 20 1.31 1.17 1.52 1.88 2.07
+//                             n = 40 2.67 2.24 2.85 4.13 4.47   n = 75 6.3  4.6  5.1  9.4  9.9
+// So the line suits wide ladders from n = 16 on; for small grids, and for ladders that
+// sit in the middle of it, 0.02 would do better.
 constexpr uint32_t kCoverAccept = 0x0A000000u;  // 0.039
 constexpr int kCoverMinProposals = 512;         // proposals left in the launch that pay for building the table
 
