@@ -541,45 +541,46 @@ static int check_common(int B, int n, const void* a, const void* out) {
 }
 
 template <class Src, int MODE, bool BAD, int NT, int PLAN>
-static int launch_tag_plan(Src src, int B, int n, int W, int32_t* scores, int32_t* badness, int32_t* mismatch,
+static int launch_tag_plan(Src src, int sms, int B, int n, int W, int32_t* scores, int32_t* badness, int32_t* mismatch,
                            uint32_t* error_word, cudaStream_t st) {
   using namespace n3;
   const auto kernel = tag_kernel<Src, MODE, BAD, NT, PLAN>;
   N3_TRY(allow_smem(reinterpret_cast<const void*>(kernel), tag_smem(NT, tag_warps(NT))));
-  const int sms = sm_count(), threads = W * 32 > kTagMinThreads ? W * 32 : kTagMinThreads;
+  const int threads = W * 32 > kTagMinThreads ? W * 32 : kTagMinThreads;
   kernel<<<B < sms ? B : sms, threads, tag_smem(NT, W), st>>>(src, B, n, W, dir_lut_device_ptr(), scores, badness,
                                                               mismatch, error_word);
   return check_launch("tag_kernel");
 }
 
 template <class Src, int MODE, bool BAD, int NT>
-static int launch_tag_nt(Src src, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+static int launch_tag_nt(Src src, int sms, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
                          uint32_t* error_word, cudaStream_t st) {
   using namespace n3;
   N3_TRY(ensure_device_tables());
-  const int sms = sm_count(), most = tag_warps(NT);
+  const int most = tag_warps(NT);
   const int per = (B + sms - 1) / sms;  // states per SM
   if (2 * per <= most) {
     int parts = 2;
     while (parts < kTagMaxParts && 2 * parts * per <= most) parts *= 2;
-    return launch_tag_plan<Src, MODE, BAD, NT, kShared>(src, B, n, per * parts, scores, badness, mismatch, error_word, st);
+    return launch_tag_plan<Src, MODE, BAD, NT, kShared>(src, sms, B, n, per * parts, scores, badness, mismatch,
+                                                        error_word, st);
   }
   const int last = per % most;
   if (per > most && last > 0 && 2 * last <= most)
-    return launch_tag_plan<Src, MODE, BAD, NT, kRoundsThenShared>(src, B, n, most, scores, badness, mismatch, error_word,
-                                                                  st);
-  return launch_tag_plan<Src, MODE, BAD, NT, kRounds>(src, B, n, per < most ? per : most, scores, badness, mismatch,
+    return launch_tag_plan<Src, MODE, BAD, NT, kRoundsThenShared>(src, sms, B, n, most, scores, badness, mismatch,
+                                                                  error_word, st);
+  return launch_tag_plan<Src, MODE, BAD, NT, kRounds>(src, sms, B, n, per < most ? per : most, scores, badness, mismatch,
                                                       error_word, st);
 }
 
 template <class Src, int MODE, bool BAD>
-static int launch_tag(Src src, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
+static int launch_tag(Src src, int sms, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
                       uint32_t* error_word, cudaStream_t st) {
   switch ((2 * n + 31) / 32) {
-    case 1: return launch_tag_nt<Src, MODE, BAD, 1>(src, B, n, scores, badness, mismatch, error_word, st);
-    case 2: return launch_tag_nt<Src, MODE, BAD, 2>(src, B, n, scores, badness, mismatch, error_word, st);
-    case 3: return launch_tag_nt<Src, MODE, BAD, 3>(src, B, n, scores, badness, mismatch, error_word, st);
-    default: return launch_tag_nt<Src, MODE, BAD, 5>(src, B, n, scores, badness, mismatch, error_word, st);
+    case 1: return launch_tag_nt<Src, MODE, BAD, 1>(src, sms, B, n, scores, badness, mismatch, error_word, st);
+    case 2: return launch_tag_nt<Src, MODE, BAD, 2>(src, sms, B, n, scores, badness, mismatch, error_word, st);
+    case 3: return launch_tag_nt<Src, MODE, BAD, 3>(src, sms, B, n, scores, badness, mismatch, error_word, st);
+    default: return launch_tag_nt<Src, MODE, BAD, 5>(src, sms, B, n, scores, badness, mismatch, error_word, st);
   }
 }
 
@@ -588,14 +589,14 @@ static int launch_slope(const int16_t* cols, int B, int n, int32_t* scores, int3
                         uint32_t* error_word, cudaStream_t st) {
   if (B == 0) return N3_OK;
   const n3::ColSource src{cols};
-  return badness ? launch_tag<n3::ColSource, MODE, true>(src, B, n, scores, badness, mismatch, error_word, st)
-                 : launch_tag<n3::ColSource, MODE, false>(src, B, n, scores, nullptr, mismatch, error_word, st);
+  const int sms = sm_count();
+  return badness ? launch_tag<n3::ColSource, MODE, true>(src, sms, B, n, scores, badness, mismatch, error_word, st)
+                 : launch_tag<n3::ColSource, MODE, false>(src, sms, B, n, scores, nullptr, mismatch, error_word, st);
 }
 
 template <class Src, bool BAD>
-static int launch_det(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
+static int launch_det(Src src, int sms, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
   using namespace n3;
-  const int sms = sm_count();
   // warps per state: 16 while two such CTAs fit every SM, 4 while eight do (64
   // n = 75 states: 14 us against 79 us with one warp a state; 1024: 76 and 105), seven
   // on the smallest grids (1184 n = 10 states: 4.5 us, 4.2 with one)
@@ -611,29 +612,33 @@ static int launch_det(Src src, int B, int n, int32_t* scores, int32_t* badness, 
 // Whether the determinants are the faster count: they grow with n^3, the tags with
 // n^2, but every centre costs the tags two round trips to shared memory, and every CTA
 // the copy of a table.  So on the smallest grids, for up to two states an SM (16 warps
-// share each) on those up to n = 28, and in between for little work.  us, determinants
+// share each) on those up to n = 28, and in between for little work, where they may take
+// a microsecond more: the tags' tables cost the host 0.6, and it is the slower of the
+// two for such calls (413 n = 22 states with badness 16.5 us a call, 17.1).  us, determinants
 // against tags, E alone: 20,011 states n = 5 9.4 / 10.0, n = 10 20.8 / 16.2, n = 24 83 / 49;
 // n = 8, 5000 6.2 / 6.9 and 8300 8.0 / 8.0; n = 10, 4096 6.1 / 6.0; n = 12, 2100 5.3 / 5.6;
 // n = 20, 600 4.7 / 5.1 and 1184 7.7 / 6.0; n = 28, 296 4.3 / 4.7 and 297 5.8 / 4.7.  With
 // badness: 20,011 states n = 10 28 / 21, n = 20 81 / 53; n = 8, 4096 5.9 / 6.1; n = 10, 3000
-// 6.8 / 7.0; n = 12, 1036 4.5 / 4.9 and 1184 6.5 / 5.1; n = 17, 1000 6.2 / 6.5; n = 26,
-// 296 5.1 / 5.1.
-static bool determinants_faster(int B, int n, bool badness) {
+// 6.8 / 7.0; n = 12, 1036 4.5 / 4.9 and 1184 6.5 / 5.1; n = 20, 1036 7.4 / 6.8; n = 22, 600
+// 6.9 / 6.5 and 1036 8.6 / 7.2; n = 26, 296 5.1 / 5.1.
+static bool determinants_faster(int sms, int B, int n, bool badness) {
   if (n <= 5) return true;
-  if (B <= 2 * sm_count()) return n <= (badness ? 26 : 28);
-  if (n > (B <= 7 * sm_count() ? (badness ? 20 : 22) : (badness ? 10 : 12))) return false;
-  return (int64_t)B * n * n <= (badness ? 300000 : 400000);
+  if (B <= 2 * sms) return n <= (badness ? 26 : 28);
+  const int64_t work = (int64_t)B * n * n;
+  if (B <= 7 * sms) return n <= (badness ? 22 : 24) && work <= (badness ? 400000 : 500000);
+  return n <= (badness ? 10 : 12) && work <= (badness ? 300000 : 400000);
 }
 
 template <class Src>
 static int launch_count(Src src, int B, int n, int32_t* scores, int32_t* badness, cudaStream_t st) {
   if (B == 0) return N3_OK;
-  const bool det = determinants_faster(B, n, badness != nullptr);
+  const int sms = sm_count();
+  const bool det = determinants_faster(sms, B, n, badness != nullptr);
   if (badness)
-    return det ? launch_det<Src, true>(src, B, n, scores, badness, st)
-               : launch_tag<Src, n3::kCount, true>(src, B, n, scores, badness, nullptr, nullptr, st);
-  return det ? launch_det<Src, false>(src, B, n, scores, nullptr, st)
-             : launch_tag<Src, n3::kCount, false>(src, B, n, scores, nullptr, nullptr, nullptr, st);
+    return det ? launch_det<Src, true>(src, sms, B, n, scores, badness, st)
+               : launch_tag<Src, n3::kCount, true>(src, sms, B, n, scores, badness, nullptr, nullptr, st);
+  return det ? launch_det<Src, false>(src, sms, B, n, scores, nullptr, st)
+             : launch_tag<Src, n3::kCount, false>(src, sms, B, n, scores, nullptr, nullptr, nullptr, st);
 }
 
 template <class Src, int MODE, int NT, int PLAN>
@@ -713,8 +718,9 @@ int n3_score_determinants(const int16_t* cols, int B, int n, int32_t* scores, in
   N3_TRY(n3host::check_common(B, n, cols, scores));
   if (B == 0) return N3_OK;
   const n3::ColSource src{cols};
-  return badness ? n3host::launch_det<n3::ColSource, true>(src, B, n, scores, badness, (cudaStream_t)stream)
-                 : n3host::launch_det<n3::ColSource, false>(src, B, n, scores, nullptr, (cudaStream_t)stream);
+  const int sms = n3host::sm_count();
+  return badness ? n3host::launch_det<n3::ColSource, true>(src, sms, B, n, scores, badness, (cudaStream_t)stream)
+                 : n3host::launch_det<n3::ColSource, false>(src, sms, B, n, scores, nullptr, (cudaStream_t)stream);
 }
 
 int n3_score_slope(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, void* stream) {
@@ -736,7 +742,7 @@ int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t
   // Two launches on one stream: the determinant count at full occupancy, then
   // the independent slope count, which validates each state, compares, and
   // gives the badness if it is wanted.
-  N3_TRY((n3host::launch_det<n3::ColSource, false>(n3::ColSource{cols}, B, n, scores, nullptr,
+  N3_TRY((n3host::launch_det<n3::ColSource, false>(n3::ColSource{cols}, n3host::sm_count(), B, n, scores, nullptr,
                                                    (cudaStream_t)stream)));
   return n3host::launch_slope<n3::kChecked>(cols, B, n, scores, badness, mismatch, error_word, (cudaStream_t)stream);
 }
