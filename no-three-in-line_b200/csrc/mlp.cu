@@ -715,27 +715,36 @@ __global__ void __launch_bounds__(kGatherRows * 32) gather_kernel(
     float* __restrict__ grads, float* __restrict__ loss) {
   chain_begin();
   const int lane = threadIdx.x & 31, b = blockIdx.x * kGatherRows + (threadIdx.x >> 5);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) grads[i] = 0.f;
   if (blockIdx.x == 0 && threadIdx.x < 2) loss[threadIdx.x] = 0.f;
-  if (b >= B) return;
+  const auto clear = [&]() {  // after the row's loads are on their way
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) grads[i] = 0.f;
+  };
+  if (b >= B) {
+    clear();
+    return;
+  }
   const uint64_t steps = counters[0], t = counters[1];
   const uint64_t recorded = steps * (uint64_t)n_chains;
   const uint64_t filled = recorded < (uint64_t)capacity ? (recorded ? recorded : 1) : (uint64_t)capacity;
   const U4 r = philox4x32_10(U4{(uint32_t)t, (uint32_t)(t >> 32), (uint32_t)b, 0x7A000000u}, k0, k1);
   const int64_t s = (int64_t)((((uint64_t)r.x << 32) | r.y) % filled);
-  if (lane == 0) y[b] = (float)rb_dE[s] / kTargetScale;
+  const int dE = rb_dE[s];
+  float v[kIn / 32];
 #pragma unroll
   for (int j = 0; j < kIn / 32; ++j) {
     const int k = lane + 32 * j;
-    float v = 0.f;
+    v[j] = 0.f;
     if (k < kCandFeat) {
       const uint16_t h = rb_feat[s * kCandFeat + k];
-      v = __uint_as_float((uint32_t)h << 16);
+      v[j] = __uint_as_float((uint32_t)h << 16);
     } else if (k < kCandFeat + kChainFeat) {
-      v = (float)rb_bad[s * kChainFeat + (k - kCandFeat)] * (1.0f / 16.0f);
+      v[j] = (float)rb_bad[s * kChainFeat + (k - kCandFeat)] * (1.0f / 16.0f);
     }
-    X[(size_t)b * kIn + k] = v;
   }
+  clear();
+  if (lane == 0) y[b] = (float)dE / kTargetScale;
+#pragma unroll
+  for (int j = 0; j < kIn / 32; ++j) X[(size_t)b * kIn + lane + 32 * j] = v[j];
 }
 
 // GEMMs on the tensor cores (tcgen05, kind::f16): C (M x N, fp32) =
@@ -1115,9 +1124,9 @@ namespace n3host {
 // Adam with the tensor-core weight images.  `scratch` holds the batch
 // activations (n3_mlp_scratch_floats(batch) floats), `grads` the gradient
 // (kParams floats); both entry points below call this body.  Seven launches, each
-// waiting for the one before, bound it: a batch of 4096 takes 60 us chained, 70 us
-// launched plainly, and took 154 us in 17 launches with passes of their own for the
-// sums, the counter and the images.
+// waiting for the one before, bound it: a batch of 4096 takes 57.5 us (10 us more when
+// launched plainly; 154 us in 17 launches with passes of their own for the sums, the
+// counter and the images).
 static int train_step(const n3_mlp* M, int n_chains, int B, float lr, uint64_t seed, float* scratch, float* grads,
                       float* adam_m, float* adam_v, cudaStream_t st) {
   using namespace n3::mlp;
