@@ -225,7 +225,8 @@ static_assert(tag_ids(1) >= (int)sizeof(int) * 32 && tag_ids(2) >= (int)sizeof(i
 static_assert(tag_ids(1) % 8 == 0 && tag_ids(2) % 8 == 0 && tag_ids(3) % 8 == 0 && tag_ids(5) % 8 == 0, "alignment");
 
 // State b's table keys for tag_state, its word[] cleared; returns the error bits of
-// columns outside [0, limit) and equal points in a row (the same in every lane).
+// columns outside [0, limit) and equal points in a row (the same in every lane), which
+// are told after such columns have been moved to the edge, as they always were.
 template <class Src, int NT>
 __device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int limit, int lane, int (&key)[NT],
                                              uint32_t* __restrict__ word) {
@@ -235,10 +236,11 @@ __device__ __forceinline__ uint32_t tag_load(const Src& src, int b, int n, int l
     const int s = lane + 32 * t;
     const bool in = s < 2 * n;
     const int c = in ? src.col(b, n, s) : 0;
+    const int inside = min(max(c, 0), limit - 1);
     // the two points of a row are neighbouring lanes
-    const int c2 = __shfl_xor_sync(0xffffffffu, c, 1);
-    if (in && (c < 0 || c >= limit)) err |= kErrColumnRange;
-    if (in && c == c2) err |= kErrDuplicate;
+    const int other = __shfl_xor_sync(0xffffffffu, inside, 1);
+    if (in && inside != c) err |= kErrColumnRange;
+    if (in && inside == other) err |= kErrDuplicate;
     key[t] = in ? (s >> 1) * kLutW + c : -1;
     if (in) word[s] = 0u;
   }
