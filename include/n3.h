@@ -57,7 +57,7 @@ int n3_init_device(void);
  * ------------------------------------------------------------------------- */
 
 /* Exact collinear-triple count of B states given as P/Q.  Counted by cross
- * products on small grids and by gcd-reduced directions on larger ones (a state
+ * products for small grids and few states and by gcd-reduced directions else (a state
  * with a column off the 75 x 75 grid or two equal points in a row, which has no
  * direction count, by cross products at every size): the same integers.
  * Replaces the reference kernel score_population (src/no_three_75/gpu.py:13-42,

@@ -190,9 +190,9 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
 // The slope count (tag_state): the warps of a CTA share one compact direction table
 // and take consecutive states, a warp each; where fewer states than warps are left,
 // `parts` warps (a power of two) share a state's centres, so that few states fill
-// the SMs too (64 n = 75 states with badness: 8.9 us; 51 us with a warp each) and a batch just above
-// a round of all warps does not cost two (4300 n = 75 states with badness: 96 us,
-// 167 with the last 156 states on six CTAs, a warp each).
+// the SMs too (64 n = 75 states with badness: 8.9 us; 51 us with a warp each) and a
+// batch just above a round of all warps does not cost two (4300 n = 75 states with
+// badness: 96 us, 167 with the last 156 states on six CTAs, a warp each).
 //   kCount   E and, if wanted, badness of any states: one with a column off the
 //            grid or two equal points in a row, which has no line count, is
 //            counted by determinants (det_state), so the results are the
@@ -202,7 +202,8 @@ __global__ void __launch_bounds__((PARTS > 1 ? PARTS : kDetWarps) * 32)
 //            in `scores` (written by det_kernel on the same stream).
 // NT, the slots a lane holds, bounds the unrolled work per centre and, with the ids of
 // the directions that a grid of 16 NT rows has, a warp's shared memory: 32 warps fit
-// up to n = 48 (4096 n = 14 states with badness: 8.6 us, 16.4 with NT = 5 and 28 warps).
+// up to n = 48 (4096 n = 14 states with badness: 8.6 us, 16.4 with NT = 5 and 28
+// warps).
 enum TagMode { kCount, kSlope, kChecked };
 // What a CTA does with its states: whole rounds of a warp each, a state shared by several
 // warps, or rounds and then the last states shared.  (A kernel that can do both takes 2
