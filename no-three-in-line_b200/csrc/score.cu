@@ -669,13 +669,21 @@ static int prepare_tag() {
 
 // The two counts of the checked score in one kernel (checked_kernel) for many
 // states of larger grids.  us with badness, two kernels against one: 4096 states
-// n = 75: 373 / 352, 61: 242 / 226, 47: 146 / 136, 38: 105 / 101, 32: 82 / 82; 20,011
-// states: 1687 / 1628, 1077 / 1030, 632 / 611, 441 / 458, 337 / 364; 4300 states, which
-// leave the determinants a last wave of few blocks: 491 / 372, 328 / 240, 205 / 166.
-// n = 75, 1200 states: 181 / 124; 900: 109 / 118 (fewer states get more warps each in
-// the two kernels).  Warps for the tags: 12 from n = 56 on, 14 below (n = 50: 14
-// take 150 us for 4096 states, 12 take 173; n = 75: 352 both).
-constexpr int kCheckedMinN = 44, kCheckedMinPerSm = 8;
+// n = 75 364 / 346, 60 224 / 212, 49 148 / 140; 20,011 states 1668 / 1630, 1020 / 988,
+// 663 / 655; 4300 states, which leave the determinants a last wave of few blocks,
+// 414 / 365, 258 / 226, 173 / 165; 1300 states, which four warps each no longer take,
+// 171 / 119, 109 / 77, 73 / 58; n = 75, 900 states 109 / 118 (fewer states get more warps
+// each in the two kernels).  Up to n = 48 the tags alone have 32 warps of less work:
+// one kernel only where the determinants have many states for four warps and few for
+// one (n = 48: 1184 states 43 / 54, 1300 65 / 56, 2000 79 / 71, 4096 130 / 133, 4300
+// 144 / 160, 20,011 582 / 625; n = 44: 37 / 49, 56 / 51, 68 / 61, 110 / 115, 122 / 144, 495 / 544).
+// Warps for the tags: 12 from n = 56 on, 14 below (n = 50: 14 take 150 us for 4096
+// states, 12 take 173; n = 75: 352 both).
+static bool checked_in_one(int B, int n) {
+  if (n < 44) return false;
+  const int sms = sm_count();
+  return n > 48 ? B >= 8 * sms : B > 8 * sms && B <= 20 * sms;
+}
 constexpr int kCheckedTagWarps = 12, kCheckedTagWarpsSmall = 14, kCheckedSmallN = 56;
 
 static int launch_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t* badness, int32_t* mismatch,
@@ -740,7 +748,7 @@ int n3_score_checked(const int16_t* cols, int B, int n, int32_t* scores, int32_t
   N3_TRY(n3host::check_common(B, n, cols, scores));
   if (B > 0 && mismatch == nullptr) return n3host::set_error(N3_ERR_ARG, "null mismatch counter");
   if (B == 0) return N3_OK;
-  if (n >= n3host::kCheckedMinN && B >= n3host::kCheckedMinPerSm * n3host::sm_count())
+  if (n3host::checked_in_one(B, n))
     return n3host::launch_checked(cols, B, n, scores, badness, mismatch, error_word, (cudaStream_t)stream);
   // Two launches on one stream: the determinant count at full occupancy, then
   // the independent slope count, which validates each state, compares, and
